@@ -154,6 +154,12 @@ struct gb_bfs {
 };
 
 namespace gb {
+// Levels a trace of the last run would hold: the persistent and batched
+// kernels record the first kTraceLevels.
+constexpr uint32_t kTraceLevels = 1u << 16;
+inline size_t recordedLevels(int variant, uint32_t levels) {
+    return variant == GB_BFS_PERSISTENT || variant == GB_BFS_BATCH ? (levels < kTraceLevels ? levels : kTraceLevels) : levels;
+}
 uint32_t checkTg(uint32_t tg);
 void validateOptions(const gb_bfs_options& o);
 }  // namespace gb

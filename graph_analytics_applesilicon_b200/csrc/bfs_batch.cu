@@ -26,7 +26,7 @@ namespace {
 
 constexpr unsigned long long kHubShift = 40;
 constexpr unsigned long long kHubMask = (1ull << kHubShift) - 1;
-constexpr uint32_t kTraceCap = 1u << 16;
+constexpr uint32_t kTraceCap = kTraceLevels;
 #ifndef GB_BATCH_BU_SERIAL
 #define GB_BATCH_BU_SERIAL 64
 #endif

@@ -277,7 +277,8 @@ int gb_bfs_run(gb_bfs* h, int variant, uint32_t source, uint32_t* out_host, cons
         if (opt) o = *opt;
         validateOptions(o);
         std::vector<gb_level> tr;
-        std::vector<gb_level>* tp = (trace || nlev) ? &tr : nullptr;
+        // the level count alone needs no records: every form leaves it in lastLevels
+        std::vector<gb_level>* tp = trace ? &tr : nullptr;
         switch (variant) {
             case GB_BFS_VERTEX: h->runVertex(source, o, tp); break;
             case GB_BFS_NAIVE: h->runNaive(source, o, tp); break;
@@ -288,7 +289,7 @@ int gb_bfs_run(gb_bfs* h, int variant, uint32_t source, uint32_t* out_host, cons
             default: throw Error(GB_ERR_ARG, "unknown BFS variant " + std::to_string(variant));
         }
         if (out_host) copyDepthsToHost(h, h->dist.get(), h->n, out_host, h->lastLevels);
-        if (nlev) *nlev = tr.size();
+        if (nlev) *nlev = trace ? tr.size() : recordedLevels(variant, h->lastLevels);
         if (trace) {
             std::memcpy(trace, tr.data(), std::min(cap, tr.size()) * sizeof(gb_level));
             if (tr.size() > cap) throw Error(GB_ERR_CAPACITY, "trace capacity too small");

@@ -56,9 +56,9 @@ int gb_bfs_run_batch(gb_bfs* h, const uint32_t* sources, int k, uint32_t* out_ho
         GB_REQUIRE(h && sources, "null argument");
         gb_bfs_options o = optsOrDefault(opt);
         std::vector<gb_level> tr;
-        h->runBatch(sources, k, o, (trace || nlev) ? &tr : nullptr);
+        h->runBatch(sources, k, o, trace ? &tr : nullptr);
         if (out_host) copyDepthsToHost(h, h->bDist.get(), (uint64_t)k * h->n, out_host, h->lastLevels);
-        if (nlev) *nlev = tr.size();
+        if (nlev) *nlev = trace ? tr.size() : recordedLevels(GB_BFS_BATCH, h->lastLevels);
         if (trace) {
             std::memcpy(trace, tr.data(), std::min(cap, tr.size()) * sizeof(gb_level));
             if (tr.size() > cap) throw Error(GB_ERR_CAPACITY, "trace capacity too small");
