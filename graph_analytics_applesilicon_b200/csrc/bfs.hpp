@@ -30,6 +30,14 @@ struct GbPCounters {
     unsigned long long pad[2];
 };
 
+// What one source's cluster reports (bfs_cluster.cu).
+struct GbClusterStat {
+    uint32_t levels, status;  // status 0: done
+    unsigned long long ns;    // device time of the traversal
+};
+constexpr uint32_t kClusterOverflow = 1;  // a frontier outgrew the queues
+constexpr uint32_t kClusterTimeout = 2;   // a bounded wait gave up
+
 struct gb_bfs;
 namespace gb {
 // Copies count depths from device d to host out (uint32, unreached ~0), packed
@@ -96,6 +104,15 @@ struct gb_bfs {
     gb::DevBuf<uint2> bDefer;            // bottom-up: lists whose rest a whole block scans
     int bGrid = 0, bBlock = 0, bMax = 0;
 
+    // bounded-degree graphs: a cluster per source (bfs_cluster.cu)
+    uint32_t maxDegree = 0xFFFFFFFFu;  // of the graph, set when the handle's CSR is checked
+    bool cOff = false;                 // a frontier of this graph outgrew the queues
+    bool cNbrReady = false;            // neighbour table built (dropped when the lists are re-sorted)
+    gb::DevBuf<uint4> cNbr;
+    gb::DevBuf<uint32_t> cSrc;
+    gb::DevBuf<GbClusterStat> cStat;
+    gb::HostPinned<GbClusterStat> cStatHost;
+
     // learned selector parameters (single-source, batched)
     gb::DevBuf<float> selParams[2];
     bool selLoaded[2] = {false, false};
@@ -138,6 +155,12 @@ struct gb_bfs {
                            const gb_bfs_options& o, float* ms, uint32_t* levels);
     void runBatchMany(const uint32_t* src, uint32_t count, uint32_t* out, uint64_t stride,
                       const gb_bfs_options& o, float* ms, uint32_t* levels);
+    bool clusterFits(uint32_t k, const gb_bfs_options& o) const;
+    bool runCluster(const uint32_t* src, uint32_t k, uint32_t* out);
+    bool runClusterMany(const uint32_t* src, uint32_t count, uint32_t* out, uint64_t stride, float* ms,
+                        uint32_t* levels);
+    // Rows 0..k-1 of bDist to the host (row j at out + j * stride).
+    void returnRows(uint32_t k, uint32_t* out, uint64_t stride);
     // Profiling (selector training data).
     size_t profileLevels(uint32_t src, const gb_bfs_options& o, int repeats, float* feats, float* times,
                          size_t cap);

@@ -216,7 +216,7 @@ int gb_bfs_create(const uint32_t* row_ptr, const uint32_t* col_idx, uint64_t n, 
         h->dist.ensure(n + 4);
         GB_CUDA(cudaMemcpyAsync(h->rowPtr.get(), row_ptr, (n + 1) * 4, cudaMemcpyHostToDevice, h->stream.s));
         if (m) GB_CUDA(cudaMemcpyAsync(h->colIdx.get(), col_idx, m * 4, cudaMemcpyHostToDevice, h->stream.s));
-        checkDeviceCsr(h->rowPtr.get(), h->colIdx.get(), n, m, h->stream.s);  // ids below n before any traversal
+        checkDeviceCsr(h->rowPtr.get(), h->colIdx.get(), n, m, h->stream.s, &h->maxDegree);  // ids below n before any traversal
         h->stats.ensure(1);
         h->hstats.ensure(1);
         h->hstage.ensure(16);
@@ -255,6 +255,7 @@ int gb_bfs_hub_first(gb_bfs* h) {
         GB_REQUIRE(h, "null handle");
         hubFirstAdjacency(h->rowPtr.get(), h->colIdx.get(), h->n, h->m, h->stream.s);
         h->hubFirst = true;
+        h->cNbrReady = false;  // its long lists point into the re-sorted adjacency
     });
 }
 

@@ -150,12 +150,18 @@ __global__ void edgeKeysKernel(const uint32_t* eu, const uint32_t* ev, uint64_t 
 
 // Input checks on the device (every id that reaches the key kernels must be
 // below n): bad |= 1 row_ptr decreases, 2 column >= n, 4 edge endpoint >= n,
-// 8 perm value >= n or repeated (seen: ceil(n/32) zeroed words).
+// 8 perm value >= n or repeated (seen: ceil(n/32) zeroed words).  bad[1]
+// becomes the longest list's length.
 __global__ void checkCsrKernel(const uint32_t* rp, const uint32_t* ci, uint64_t n, uint64_t m, unsigned* bad) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    unsigned f = 0;
-    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride)
-        if (rp[v] > rp[v + 1]) f |= 1u;
+    unsigned f = 0, longest = 0;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+        const uint32_t b = rp[v], e = rp[v + 1];
+        if (b > e) f |= 1u;
+        else longest = max(longest, e - b);
+    }
+    longest = __reduce_max_sync(0xFFFFFFFFu, longest);
+    if ((threadIdx.x & 31) == 0 && longest) atomicMax(bad + 1, longest);
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += stride)
         if (ci[i] >= n) f |= 2u;
     if (f) atomicOr(bad, f);
@@ -342,15 +348,18 @@ void connectedComponents(const uint32_t* rp, const uint32_t* ci, uint64_t n, uin
 
 namespace {
 
-// Reads the device check word; throws if any check failed.
-void requireChecks(DevBuf<unsigned>& bad, cudaStream_t st) {
-    unsigned h = 0;
-    GB_CUDA(cudaMemcpyAsync(&h, bad.get(), 4, cudaMemcpyDeviceToHost, st));
+// Reads the device check words; throws if any check failed.  Returns the
+// second word (checkCsrKernel's longest list; 0 after the other checks).
+uint32_t requireChecks(DevBuf<unsigned>& bad, cudaStream_t st) {
+    unsigned w[2];
+    GB_CUDA(cudaMemcpyAsync(w, bad.get(), 8, cudaMemcpyDeviceToHost, st));
     GB_CUDA(cudaStreamSynchronize(st));
+    const unsigned h = w[0];
     if (h & 1u) throw Error(GB_ERR_ARG, "graph prep: row_ptr must not decrease");
     if (h & 2u) throw Error(GB_ERR_ARG, "graph prep: column id >= n");
     if (h & 4u) throw Error(GB_ERR_ARG, "gb_csr_from_edges_gpu: edge endpoint >= n");
     if (h & 8u) throw Error(GB_ERR_ARG, "gb_csr_permute_gpu: perm is not a permutation of [0, n)");
+    return w[1];
 }
 
 // Uploads a host CSR.
@@ -363,13 +372,15 @@ void uploadCsr(const gb_csr* g, DevBuf<uint32_t>& rp, DevBuf<uint32_t>& ci, cuda
 
 }  // namespace
 
-void checkDeviceCsr(const uint32_t* rp, const uint32_t* ci, uint64_t n, uint64_t m, cudaStream_t st) {
+void checkDeviceCsr(const uint32_t* rp, const uint32_t* ci, uint64_t n, uint64_t m, cudaStream_t st,
+                    uint32_t* maxDegree) {
     DevBuf<unsigned> bad;
-    bad.ensure(1);
-    GB_CUDA(cudaMemsetAsync(bad.get(), 0, 4, st));
+    bad.ensure(2);
+    GB_CUDA(cudaMemsetAsync(bad.get(), 0, 8, st));
     checkCsrKernel<<<prepGrid(std::max(n, m), 256), 256, 0, st>>>(rp, ci, n, m, bad.get());
     GB_LAUNCH_CHECK();
-    requireChecks(bad, st);
+    const uint32_t longest = requireChecks(bad, st);
+    if (maxDegree) *maxDegree = longest;
 }
 
 void uploadCheckedCsr(const gb_csr* g, DevBuf<uint32_t>& rp, DevBuf<uint32_t>& ci, cudaStream_t st) {
@@ -378,8 +389,8 @@ void uploadCheckedCsr(const gb_csr* g, DevBuf<uint32_t>& rp, DevBuf<uint32_t>& c
     GB_REQUIRE(g->m < (1ull << 32), "graph prep: m must fit in uint32");
     GB_REQUIRE(g->row_ptr[0] == 0 && g->row_ptr[g->n] == g->m, "graph prep: row_ptr must run from 0 to m");
     DevBuf<unsigned> bad;
-    bad.ensure(1);
-    GB_CUDA(cudaMemsetAsync(bad.get(), 0, 4, st));
+    bad.ensure(2);
+    GB_CUDA(cudaMemsetAsync(bad.get(), 0, 8, st));
     uploadCsr(g, rp, ci, st);
     checkCsrKernel<<<prepGrid(std::max(g->n, g->m), 256), 256, 0, st>>>(rp.get(), ci.get(), g->n, g->m, bad.get());
     GB_LAUNCH_CHECK();
@@ -402,8 +413,8 @@ void csrOp(const gb_csr* g, int mode, const uint32_t* permHost, bool unique, boo
     ScanScratch sc;
     DevBuf<uint32_t> rp, ci, perm, seen;
     DevBuf<unsigned> bad;
-    bad.ensure(1);
-    GB_CUDA(cudaMemsetAsync(bad.get(), 0, 4, st.s));
+    bad.ensure(2);
+    GB_CUDA(cudaMemsetAsync(bad.get(), 0, 8, st.s));
     uploadCsr(g, rp, ci, st.s);
     checkCsrKernel<<<prepGrid(std::max(g->n, g->m), 256), 256, 0, st.s>>>(rp.get(), ci.get(), g->n, g->m, bad.get());
     GB_LAUNCH_CHECK();
@@ -445,10 +456,10 @@ int gb_csr_from_edges_gpu(uint64_t n, const uint32_t* eu, const uint32_t* ev, ui
         ScanScratch sc;
         DevBuf<uint32_t> du, dv;
         DevBuf<unsigned> bad;
-        bad.ensure(1);
+        bad.ensure(2);
         du.ensure(ne + 1);
         dv.ensure(ne + 1);
-        GB_CUDA(cudaMemsetAsync(bad.get(), 0, 4, st.s));
+        GB_CUDA(cudaMemsetAsync(bad.get(), 0, 8, st.s));
         if (ne) {
             GB_CUDA(cudaMemcpyAsync(du.get(), eu, ne * 4, cudaMemcpyHostToDevice, st.s));
             GB_CUDA(cudaMemcpyAsync(dv.get(), ev, ne * 4, cudaMemcpyHostToDevice, st.s));

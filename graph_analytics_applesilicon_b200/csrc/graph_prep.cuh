@@ -26,8 +26,9 @@ void keysToCsr(DevBuf<unsigned long long>& keys, uint64_t N, uint64_t n, int b, 
 // non-decreasing, every column below n); throws GB_ERR_ARG otherwise.
 void uploadCheckedCsr(const gb_csr* g, DevBuf<uint32_t>& rp, DevBuf<uint32_t>& ci, cudaStream_t st);
 // Checks a device CSR (row_ptr non-decreasing, every column below n); throws
-// GB_ERR_ARG otherwise.
-void checkDeviceCsr(const uint32_t* rp, const uint32_t* ci, uint64_t n, uint64_t m, cudaStream_t st);
+// GB_ERR_ARG otherwise.  maxDegree (optional) receives the longest list.
+void checkDeviceCsr(const uint32_t* rp, const uint32_t* ci, uint64_t n, uint64_t m, cudaStream_t st,
+                    uint32_t* maxDegree = nullptr);
 // Connected components of a symmetric device CSR: parent[v] = the smallest
 // vertex of v's component.
 void connectedComponents(const uint32_t* rp, const uint32_t* ci, uint64_t n, uint32_t* parent, cudaStream_t st);

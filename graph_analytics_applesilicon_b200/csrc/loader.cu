@@ -267,7 +267,7 @@ int gb_bfs_create_from_file(const char* path, gb_bfs** out, uint64_t* n_out, uin
             }
             GB_CUDA(cudaStreamSynchronize(st));
         }
-        checkDeviceCsr(h->rowPtr.get(), h->colIdx.get(), b.n, b.m, st);
+        checkDeviceCsr(h->rowPtr.get(), h->colIdx.get(), b.n, b.m, st, &h->maxDegree);
         h->stats.ensure(1);
         h->hstats.ensure(1);
         h->hstage.ensure(16);
