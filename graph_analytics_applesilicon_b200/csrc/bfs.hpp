@@ -97,7 +97,7 @@ struct gb_bfs {
     std::unique_ptr<gb::Stream> pStream[gb::kMaxInFlight - 1];  // created on first use
 
     // batched (64 sources)
-    gb::DevBuf<unsigned long long> bSeen, bFront[2], bNext;
+    gb::DevBuf<unsigned long long> bSeen, bFront[2], bNext, bPlane;
     gb::DevBuf<uint32_t> bActive[2], bCand, bHubV[2];
     gb::DevBuf<unsigned long long> bHubOff[2];
     gb::DevBuf<uint32_t> bDist;          // k * n results
