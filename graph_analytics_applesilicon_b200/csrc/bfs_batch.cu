@@ -31,25 +31,16 @@ namespace {
 constexpr unsigned long long kHubShift = 40;
 constexpr unsigned long long kHubMask = (1ull << kHubShift) - 1;
 constexpr uint32_t kTraceCap = kTraceLevels;
-#ifndef GB_BATCH_BU_SERIAL
-#define GB_BATCH_BU_SERIAL 64
-#endif
-#ifndef GB_BATCH_BU_COOP
-#define GB_BATCH_BU_COOP 64
-#endif
-#ifndef GB_BATCH_BU_BLOCK
-#define GB_BATCH_BU_BLOCK 256
-#endif
-// bottom-up list scans: serial per thread for the first kBatchBuSerial entries,
-// then a rest of kBatchBuCoop entries or more by the warp, kBatchBuBlock or
-// more by the block
-constexpr uint32_t kBatchBuSerial = GB_BATCH_BU_SERIAL;
-constexpr uint32_t kBatchBuCoop = GB_BATCH_BU_COOP;
-constexpr uint32_t kBatchBuBlock = GB_BATCH_BU_BLOCK;
-#ifndef GB_BATCH_BU_UNROLL
-#define GB_BATCH_BU_UNROLL 8
-#endif
-constexpr int kBuUnroll = GB_BATCH_BU_UNROLL;  // entries per thread per cooperative step
+// Bottom-up list scans: serial per thread for the first kBatchBuSerial entries,
+// then a rest of kBatchBuCoop entries or more by the warp; from kBatchBuDefer on
+// the rest is listed and taken by any warp of the grid, from kBatchBuBlock on by
+// any block.  64 sources, R-MAT 22 / Chung-Lu 3.07M: 2.16 / 1.79 ms as here;
+// 32, 32, 128: 2.27 / 1.81; 16, 32, 64: 2.29 / 2.01; blocks from 16384: 2.24 / 1.78.
+constexpr uint32_t kBatchBuSerial = 64;
+constexpr uint32_t kBatchBuCoop = 64;
+constexpr uint32_t kBatchBuDefer = 256;
+constexpr uint32_t kBatchBuBlock = 4096;
+constexpr int kBuUnroll = 8;  // entries per thread per cooperative step (4: 2.18 / 1.77 ms)
 
 // Depths below 2^kPlanes are held in bit planes.  8 planes (64 bytes per vertex,
 // a quarter of 64 depth rows) cover every traversal of a graph without a long
@@ -72,7 +63,7 @@ struct BCounters {
     unsigned long long fullEdges;  // degree sum of vertices that became fully seen
     unsigned long long fullCount;
     unsigned long long examined;
-    unsigned dcnt;                 // bottom-up: lists whose rest is deferred to a whole block
+    unsigned dcnt[2];              // bottom-up: deferred rests, for a warp / for a block
 };
 
 struct BArgs {
@@ -90,7 +81,7 @@ struct BArgs {
     uint32_t* cq;
     unsigned long long* plane;  // [kPlanes][n]
     uint32_t planeDepth;        // depths below this are held in planes (1: none)
-    uint2* dq;  // bottom-up: (vertex, resume position) of the deferred rests
+    uint2* dq;  // bottom-up: (vertex, resume position) of the deferred rests, a warp's from the front, a block's from the back
     uint32_t* dist;
     const uint32_t* sources;
     BCounters* ctr;
@@ -136,7 +127,7 @@ struct BSmem {
     uint32_t base;
     int ok;
     unsigned bor[2];  // bottom-up deferred rests: OR of the frontier masks found (lo, hi)
-    uint32_t dn;      // ... and their count
+    uint32_t dn[2];   // ... and their counts
 };
 
 // Grid barrier after which every thread of the block sees counters *c in
@@ -474,8 +465,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batchBfsKernel(BArgs a) {
                 // are loaded at once with their 4 masks.  What is left of a
                 // list then goes to the whole warp (kBatchBuCoop or more
                 // entries left: the warp takes such lists one after another,
-                // 32 kBuUnroll entries per step) or, from kBatchBuBlock entries
-                // left, to a whole block after this loop; shorter rests finish
+                // 32 kBuUnroll entries per step) or, from kBatchBuDefer entries
+                // left, to a list for after this loop; shorter rests finish
                 // serially.  One long list scanned by one thread would hold its
                 // warp and the level; the loop has no block barrier, so the
                 // warps of a block do not wait for one another.
@@ -492,7 +483,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batchBfsKernel(BArgs a) {
                 };
                 if (need) scanTo(st + min(d, kBatchBuSerial));
                 const uint32_t rest = (need && (got & need) != need) ? e - i : 0u;
-                const bool huge = rest >= kBatchBuBlock;
+                const bool huge = rest >= kBatchBuDefer;
                 const bool coop = !huge && rest >= kBatchBuCoop;
                 if (rest && !huge && !coop) scanTo(e);
                 const unsigned long long want = need & ~got;  // still missing after the serial part
@@ -518,12 +509,17 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batchBfsKernel(BArgs a) {
                         i += min(off, hd);
                     }
                 }
-                // rests of kBatchBuBlock or more entries: deferred to the phase
+                // rests of kBatchBuDefer or more entries: deferred to the phase
                 // below (the masks found so far wait in nx, zero in bottom-up levels)
                 if (huge) a.nx[v] = got;
                 if (__any_sync(kFull, huge)) {
-                    const uint32_t p = warpAppend(huge, &cur->dcnt);
-                    if (huge) a.dq[p] = make_uint2((uint32_t)v, i);
+                    const bool forBlock = huge && rest >= kBatchBuBlock;
+                    const uint32_t p = warpAppend(huge && !forBlock, &cur->dcnt[0]);
+                    if (huge && !forBlock) a.dq[p] = make_uint2((uint32_t)v, i);
+                    if (__any_sync(kFull, forBlock)) {
+                        const uint32_t q = warpAppend(forBlock, &cur->dcnt[1]);
+                        if (forBlock) a.dq[a.n - 1 - q] = make_uint2((uint32_t)v, i);
+                    }
                 }
                 if (v < a.n && !huge) {
                     if (need) {
@@ -542,19 +538,47 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batchBfsKernel(BArgs a) {
                 }
                 warpAppendActive(a, b != 0, (uint32_t)v, st, d, nq, cur);
             }
-            // the deferred rests, one at a time per block, taken by ticket over
-            // the whole grid (kBuUnroll NT entries per step, the block's OR of
-            // masks in shared memory, stopping once every missing source is found)
+            // the deferred rests, taken by ticket over the whole grid: the long
+            // ones by blocks (kBuUnroll NT entries per step, the block's OR of
+            // masks in shared memory), then the others by warps, which need no
+            // block barrier; both stop once every missing source is found.
+            // R-MAT 22's second level defers 35,443 rests: 570 us with a block
+            // each (64 sources: 2.66 ms in all, 2.16 with a warp each).
             if (!batchBarrier<NT>(a, sm, cur)) return;
-            if (tid == 0) sm.dn = ldv32(&cur->dcnt);
+            if (tid < 2) sm.dn[tid] = ldv32(&cur->dcnt[tid]);
             __syncthreads();
-            const uint32_t D = sm.dn;
+            // the result b of vertex v's finished scan (one thread)
+            auto finish = [&](uint32_t v, uint32_t st, uint32_t d, unsigned long long old, unsigned long long b) {
+                a.nx[v] = 0;
+                a.fr[nq][v] = b;
+                if (!b) return;
+                foldBits(a, v, old, b, d, acc);
+                if (inPlanes) {
+                    setPlanes(a, v, b, depth);
+                } else {
+                    for (unsigned long long bb = b; bb; bb &= bb - 1)
+                        a.dist[(uint64_t)(__ffsll((long long)bb) - 1) * a.n + v] = depth;
+                }
+                if (d >= a.hubMin) {
+                    const unsigned long long hp = atomicAdd(&cur->hubPack, (1ull << kHubShift) | d);
+                    const uint32_t hi = (uint32_t)(hp >> kHubShift);
+                    a.hv[nq][hi] = v;
+                    a.hs[nq][hi] = st;
+                    a.ho[nq][hi] = hp & kHubMask;
+                } else {
+                    const uint32_t p = atomicAdd(&cur->acnt, 1u);
+                    a.qv[nq][p] = v;
+                    a.qs[nq][p] = st;
+                    a.qd[nq][p] = d;
+                }
+            };
+            const uint32_t D = sm.dn[1], DW = sm.dn[0];
             for (bool first = true;; first = false) {
                 if (tid == 0) sm.item = first ? blockIdx.x : gridDim.x + atomicAdd(&cur->work[0], 1u);
                 __syncthreads();
                 const uint32_t item = sm.item;
                 if (item >= D) break;  // block-uniform
-                const uint2 ent = a.dq[item];
+                const uint2 ent = a.dq[a.n - 1 - item];
                 const uint32_t v = ent.x, st = a.row_ptr[v], e = a.row_ptr[v + 1];
                 const unsigned long long old = a.seen[v], need = a.all & ~old, got0 = a.nx[v];
                 const unsigned long long hn = need & ~got0;
@@ -585,34 +609,38 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batchBfsKernel(BArgs a) {
                     __syncthreads();
                 }
                 if (tid == 0) {
-                    const unsigned long long b = (got0 | g2) & need;
-                    const uint32_t d = e - st;
                     acc.exam += (ent.y - st) + min(off, hd);
-                    a.nx[v] = 0;
-                    a.fr[nq][v] = b;
-                    if (b) {
-                        foldBits(a, v, old, b, d, acc);
-                        if (inPlanes) {
-                            setPlanes(a, v, b, depth);
-                        } else {
-                            for (unsigned long long bb = b; bb; bb &= bb - 1)
-                                a.dist[(uint64_t)(__ffsll((long long)bb) - 1) * a.n + v] = depth;
-                        }
-                        if (d >= a.hubMin) {
-                            const unsigned long long hp = atomicAdd(&cur->hubPack, (1ull << kHubShift) | d);
-                            const uint32_t hi = (uint32_t)(hp >> kHubShift);
-                            a.hv[nq][hi] = v;
-                            a.hs[nq][hi] = st;
-                            a.ho[nq][hi] = hp & kHubMask;
-                        } else {
-                            const uint32_t p = atomicAdd(&cur->acnt, 1u);
-                            a.qv[nq][p] = v;
-                            a.qs[nq][p] = st;
-                            a.qd[nq][p] = d;
-                        }
-                    }
+                    finish(v, st, e - st, old, (got0 | g2) & need);
                 }
                 __syncthreads();  // sm.bor and sm.item are reused by the next list
+            }
+            const uint32_t gwarp = (uint32_t)(gtid >> 5), gwarps = (uint32_t)(gthreads >> 5);
+            for (uint32_t item = gwarp; item < DW;) {  // warp-uniform
+                uint32_t ticket = 0;
+                if (laneId() == 0) ticket = atomicAdd(&cur->work[1], 1u);  // the next item, on its way during this one
+                const uint2 ent = a.dq[item];
+                const uint32_t v = ent.x, st = a.row_ptr[v], e = a.row_ptr[v + 1];
+                const unsigned long long old = a.seen[v], need = a.all & ~old, got0 = a.nx[v];
+                const unsigned long long hn = need & ~got0;
+                const uint32_t hd = e - ent.y;
+                unsigned long long g2 = 0;
+                uint32_t off = 0;
+                while (off < hd) {
+                    unsigned long long g = 0;
+#pragma unroll
+                    for (int q = 0; q < kBuUnroll; ++q) {
+                        const uint32_t j = off + laneId() + 32u * q;
+                        if (j < hd) g |= fc[a.col_idx[ent.y + j]];
+                    }
+                    g2 |= warpOr64(g);
+                    off += 32u * kBuUnroll;
+                    if ((g2 & hn) == hn) break;
+                }
+                if (laneId() == 0) {
+                    acc.exam += (ent.y - st) + min(off, hd);
+                    finish(v, st, e - st, old, (got0 | g2) & need);
+                }
+                item = gwarps + __shfl_sync(kFull, ticket, 0);
             }
         } else {
             // phase A: clear the previous level's frontier entries of fr[nq]
