@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_copy.hpp"
 #include "prims.cuh"
 #include "selector.cuh"
 
@@ -41,13 +42,27 @@ constexpr uint32_t kClusterTimeout = 2;   // a bounded wait gave up
 struct gb_bfs;
 namespace gb {
 // Copies count depths from device d to host out (uint32, unreached ~0), packed
-// to 1 or 2 bytes per depth over PCIe when `levels` allows (depth_out.cu).
+// to 4 bits, 1 or 2 bytes per depth over PCIe when `levels` allows (depth_out.cu).
 void copyDepthsToHost(gb_bfs* h, const uint32_t* d, uint64_t count, uint32_t* out, uint32_t levels);
+// The same in two stages on the handle's stream: beginDepths enqueues the
+// packing (for at most `levels` levels, which may be a guess) and the copies;
+// waitDepths returns once the work enqueued before them is done; endDepths
+// widens into out, packing again if the guess was too low for the real level
+// count.
+struct DepthReturn {
+    const uint32_t* d = nullptr;
+    uint64_t count = 0;
+    int fmt = -1;
+};
+void beginDepths(gb_bfs* h, const uint32_t* d, uint64_t count, uint32_t levels, DepthReturn& r);
+void waitDepths(gb_bfs* h, const DepthReturn& r);
+void endDepths(gb_bfs* h, const DepthReturn& r, uint32_t levels, uint32_t* out);
 // The same packing as stages of a pipeline: packFormat picks the width for a
 // traversal of `levels` levels (0: 4 bits, 1: 1 byte, 2: 2 bytes per depth;
 // -1: send uint32), enqueuePack packs on `st` (sets *overflow when a depth does
-// not fit), widenPacked turns the copied bytes back into uint32 on the host.
-int packFormat(uint64_t count, uint32_t levels);
+// not fit; dev has room for 16 bytes more), widenPacked turns the copied bytes
+// back into uint32 on the host.
+int packFormat(uint32_t levels);
 uint64_t packedBytes(int fmt, uint64_t count);
 void enqueuePack(int fmt, const uint32_t* d, uint64_t count, uint8_t* dev, unsigned* overflow, cudaStream_t st);
 void widenPacked(int fmt, const uint8_t* in, uint64_t count, uint32_t* out);
@@ -81,6 +96,7 @@ struct gb_bfs {
     bool pIsoReady = false;
     gb::DevBuf<GbPCounters> pctr;        // [3]
     gb::DevBuf<unsigned> pctl;           // [0] barrier, [1] error, [2] levels, [3] flags
+    gb::HostPinned<unsigned> pctlHost;
     gb::DevBuf<gb_level> ptrace;
     gb::DevBuf<double> pstate;           // level state for resumable (profiling) runs
     int pGrid = 0, pBlock = 0, pMax = 0, pWant = 0;
@@ -123,6 +139,7 @@ struct gb_bfs {
     gb::DevBuf<unsigned> packFlag;
     gb::HostPinned<unsigned> packFlagHost;
     std::vector<cudaEvent_t> packEv;
+    gb::StagedCopy staged;
 
     // several sources per call (runPersistentMany): depth buffers besides
     // dist, per-slot packed copies, per-source control words and events
@@ -149,7 +166,8 @@ struct gb_bfs {
     void runBinned(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr);
     void runEdge(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr);
     void runDirOpt(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr);
-    void runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr);
+    // out: also return the depths there (host memory), the copy queued behind the traversal
+    void runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr, uint32_t* out = nullptr);
     void runBatch(const uint32_t* src, int k, const gb_bfs_options& o, std::vector<gb_level>* tr);
     void runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* out, uint64_t stride,
                            const gb_bfs_options& o, float* ms, uint32_t* levels);

@@ -888,12 +888,10 @@ void gb_bfs::returnRows(uint32_t k, uint32_t* out, uint64_t stride) {
         mSlotEv.push_back(e);
     }
     cudaStream_t cs = copyStream.s;
-    const int fmt = packFormat(n, lastLevels);
+    const int fmt = packFormat(lastLevels);
     if (fmt < 0) {
         for (uint32_t j = 0; j < k; ++j)
-            GB_CUDA(cudaMemcpyAsync(out + (uint64_t)j * stride, bDist.get() + (uint64_t)j * n, n * 4,
-                                    cudaMemcpyDeviceToHost, stream.s));
-        GB_CUDA(cudaStreamSynchronize(stream.s));
+            staged.run(bDist.get() + (uint64_t)j * n, n * 4, out + (uint64_t)j * stride, stream.s);
         return;
     }
     auto enqueue = [&](uint32_t j) {
@@ -918,8 +916,7 @@ void gb_bfs::returnRows(uint32_t k, uint32_t* out, uint64_t stride) {
         if (mFlagHost.p[j] == 0) {
             widenPacked(fmt, mPackHost[b].p, n, dst);
         } else {  // a depth did not fit the width: the row is still intact on the device
-            GB_CUDA(cudaMemcpyAsync(dst, bDist.get() + (uint64_t)j * n, n * 4, cudaMemcpyDeviceToHost, cs));
-            GB_CUDA(cudaStreamSynchronize(cs));
+            staged.run(bDist.get() + (uint64_t)j * n, n * 4, dst, cs);
         }
         if (queued < k) enqueue(queued++);
     }

@@ -857,7 +857,7 @@ void gb_bfs::ensurePersistent(const gb_bfs_options& o) {
     pGrid = pWant > 0 ? std::min(pWant, pMax) : pMax;
 }
 
-void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr) {
+void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr, uint32_t* out) {
     validateOptions(o);
     if (o.selector == GB_SELECT_LEARNED && !selLoaded[0])
         throw Error(GB_ERR_STATE, "learned selector requested but no parameters are loaded");
@@ -865,7 +865,10 @@ void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb
     // vertex (1,914 of 1,953 on the 1400 x 1400 grid); the cluster form is that
     // strategy for narrow frontiers.  The rule keeps the grid-wide form it is
     // compared in, and so does a traced run, whose records are that form's.
-    if (!tr && o.selector == GB_SELECT_LEARNED && clusterFits(1, o) && runCluster(&src, 1, dist.get())) return;
+    if (!tr && o.selector == GB_SELECT_LEARNED && clusterFits(1, o) && runCluster(&src, 1, dist.get())) {
+        if (out) copyDepthsToHost(this, dist.get(), n, out, lastLevels);
+        return;
+    }
     ensurePersistent(o);
     PArgs a = makeArgs(*this, o, src);
     GB_CUDA(cudaMemsetAsync(pctl.get(), 0, 4 * sizeof(unsigned), stream.s));
@@ -873,12 +876,22 @@ void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb
     GB_CUDA(cudaMemsetAsync(dist.get(), 0xFF, n * 4, stream.s));  // every depth infinity (0xFFFFFFFF)
     launchFor(*this, a);
     GB_CUDA(cudaEventRecord(ev.b, stream.s));
-    unsigned ctl[4];
-    GB_CUDA(cudaMemcpyAsync(ctl, pctl.get(), sizeof ctl, cudaMemcpyDeviceToHost, stream.s));
-    GB_CUDA(cudaStreamSynchronize(stream.s));
+    pctlHost.ensure(4);
+    const unsigned* ctl = pctlHost.p;
+    GB_CUDA(cudaMemcpyAsync(pctlHost.p, pctl.get(), 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream.s));
+    // the depths follow on the stream, packed for as many levels as the last
+    // run had (else for one byte), so one wait covers traversal and copy
+    DepthReturn ret;
+    if (out) beginDepths(this, dist.get(), n, lastLevels ? lastLevels : 254, ret);
+    if (out) waitDepths(this, ret);
+    else GB_CUDA(cudaStreamSynchronize(stream.s));
     lastGpuMs = ev.ms();
     lastLevels = ctl[2];
-    if (ctl[1]) throw Error(GB_ERR_TIMEOUT, "persistent BFS: grid barrier wait exceeded its spin limit");
+    if (ctl[1]) {
+        GB_CUDA(cudaStreamSynchronize(stream.s));
+        throw Error(GB_ERR_TIMEOUT, "persistent BFS: grid barrier wait exceeded its spin limit");
+    }
+    if (out) endDepths(this, ret, lastLevels, out);
     if (tr) {
         const uint32_t k = std::min<uint32_t>(ctl[2], kTraceCap);
         std::vector<gb_level> t(k);
@@ -985,7 +998,7 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
             GB_CUDA(cudaEventRecord(released, st));
             return;
         }
-        fmt[i] = packFormat(n, anySeen ? maxSeen : lastLevels ? lastLevels : 254);
+        fmt[i] = packFormat(anySeen ? maxSeen : lastLevels ? lastLevels : 254);
         if (fmt[i] >= 0) {
             GB_CUDA(cudaMemsetAsync(mFlag.get() + b, 0, sizeof(unsigned), st));
             enqueuePack(fmt[i], bufs[b], n, mPackDev[b].get(), mFlag.get() + b, st);
@@ -1034,8 +1047,7 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
             if (fmt[i] >= 0 && mFlagHost.p[i] == 0) {
                 widenPacked(fmt[i], mPackHost[b].p, n, dst);
             } else {  // too many levels for the predicted width: the buffer is still intact
-                GB_CUDA(cudaMemcpyAsync(dst, bufs[b], n * 4, cudaMemcpyDeviceToHost, cs));
-                GB_CUDA(cudaStreamSynchronize(cs));
+                staged.run(bufs[b], n * 4, dst, cs);
             }
         }
         joinStreams();

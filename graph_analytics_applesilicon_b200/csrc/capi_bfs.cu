@@ -286,10 +286,10 @@ int gb_bfs_run(gb_bfs* h, int variant, uint32_t source, uint32_t* out_host, cons
             case GB_BFS_BINNED: h->runBinned(source, o, tp); break;
             case GB_BFS_EDGE: h->runEdge(source, o, tp); break;
             case GB_BFS_DO: h->runDirOpt(source, o, tp); break;
-            case GB_BFS_PERSISTENT: h->runPersistent(source, o, tp); break;
+            case GB_BFS_PERSISTENT: h->runPersistent(source, o, tp, out_host); break;
             default: throw Error(GB_ERR_ARG, "unknown BFS variant " + std::to_string(variant));
         }
-        if (out_host) copyDepthsToHost(h, h->dist.get(), h->n, out_host, h->lastLevels);
+        if (out_host && variant != GB_BFS_PERSISTENT) copyDepthsToHost(h, h->dist.get(), h->n, out_host, h->lastLevels);
         if (nlev) *nlev = trace ? tr.size() : recordedLevels(variant, h->lastLevels);
         if (trace) {
             std::memcpy(trace, tr.data(), std::min(cap, tr.size()) * sizeof(gb_level));

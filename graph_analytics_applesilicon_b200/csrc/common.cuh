@@ -65,21 +65,34 @@ struct DevBuf {
     }
 };
 
+// Pinned host memory from the process's pool (host_pool.cpp): page-locking costs
+// about a millisecond a call and several per megabyte.  Safe from any thread.
+void* pinnedAcquire(size_t bytes, size_t* got);
+void pinnedRelease(void* p, size_t got);
+
 // Pinned host allocation.
 template <class T>
 struct HostPinned {
     T* p = nullptr;
     size_t n = 0;
-    ~HostPinned() {
-        if (p) cudaFreeHost(p);
+    HostPinned() = default;
+    HostPinned(const HostPinned&) = delete;
+    HostPinned& operator=(const HostPinned&) = delete;
+    ~HostPinned() { release(); }
+    void release() {
+        if (p) pinnedRelease(p, bytes_);
+        p = nullptr;
+        n = 0;
     }
     void ensure(size_t count) {
         if (count <= n && p) return;
-        if (p) cudaFreeHost(p);
-        p = nullptr;
-        GB_CUDA(cudaMallocHost(&p, (count ? count : 1) * sizeof(T)));
-        n = count;
+        release();
+        p = static_cast<T*>(pinnedAcquire((count ? count : 1) * sizeof(T), &bytes_));
+        n = bytes_ / sizeof(T);
     }
+
+private:
+    size_t bytes_ = 0;
 };
 
 struct Stream {

@@ -1,145 +1,132 @@
-// depth_out.cu -- returning BFS depths to host memory.  A depth array is
-// 4 bytes per vertex, but a traversal of L levels only needs depths below L:
-// when L < 15 (255, 65535) the depths travel over PCIe as 4 bits (1 byte,
-// 2 bytes) per vertex, sentinel all ones for unreached, in chunks whose host-side widening to
-// uint32 (OpenMP threads) overlaps the copy of the next chunk.  The pack
-// kernel also checks every depth against the width, so a wrong level count
-// can only cost a plain copy, never a wrong result.
+// depth_out.cu -- returning results to host memory.
+//
+// A depth array is 4 bytes per vertex, but a traversal of L levels only needs
+// depths below L: when L < 15 (255, 65535) the depths travel over PCIe as 4
+// bits (1 byte, 2 bytes) per vertex, sentinel all ones for unreached, in chunks
+// whose host-side widening to uint32 (SSE2, OpenMP threads) overlaps the copy
+// of the next chunk.  The pack kernel also checks every depth against the
+// width, so a wrong level count can only cost a plain copy, never a wrong
+// result; a caller may therefore enqueue the packing behind a traversal whose
+// level count it does not know yet (beginDepths) and widen after one wait.
+#include <emmintrin.h>
 #include <omp.h>
 
 #include <algorithm>
 #include <cstring>
 
 #include "bfs.hpp"
+#include "host_copy.hpp"
 
 namespace gb {
 namespace {
 
-constexpr uint64_t kPackMin = 1u << 18;   // smaller arrays go as one plain copy
-constexpr uint64_t kPackChunk = 1u << 20;  // vertices per pipelined chunk
+constexpr uint64_t kPackChunk = 1u << 20;    // vertices per pipelined chunk (a multiple of 32)
+constexpr uint64_t kOneThread = 1u << 16;    // up to this many depths one thread widens: an OpenMP region costs more
 
-template <typename T>
-__global__ void packDepthsKernel(const uint32_t* d, uint64_t count, T* out, unsigned* overflow) {
-    const uint32_t sentinel = (uint32_t)(T)~0u;
+int hostThreads(int most) { return std::max(1, std::min(most, omp_get_max_threads())); }
+
+// Eight depths per thread and step: two 16-byte loads (where d is aligned to
+// them; a batch's rows need not be), one store of 4, 8 or 16 bytes.  FMT 0: two
+// depths per byte, low nibble first; 1: a byte; 2: two bytes.  The last group
+// is filled up with the sentinel (out has room for it).
+template <int FMT>
+__global__ void packDepthsKernel(const uint32_t* d, uint64_t count, uint8_t* out, unsigned* overflow) {
+    constexpr uint32_t kBits = FMT == 0 ? 4 : FMT == 1 ? 8 : 16, kSentinel = (1u << kBits) - 1u;
+    const bool aligned = (reinterpret_cast<uintptr_t>(d) & 15) == 0;
     bool bad = false;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = d[i];
-        bad |= v != 0xFFFFFFFFu && v >= sentinel;
-        out[i] = v == 0xFFFFFFFFu ? (T)sentinel : (T)v;
+    const uint64_t groups = (count + 7) / 8;
+    for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t v[8];
+        if (aligned && 8 * g + 8 <= count) {
+            const uint4 a = reinterpret_cast<const uint4*>(d)[2 * g], b = reinterpret_cast<const uint4*>(d)[2 * g + 1];
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = 8 * g + i < count ? d[8 * g + i] : kInf;
+        }
+        uint32_t w[FMT == 0 ? 1 : FMT == 1 ? 2 : 4] = {};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            bad |= v[i] != kInf && v[i] >= kSentinel;
+            w[i * kBits / 32] |= (v[i] & kSentinel) << (i * kBits % 32);  // infinity ends as the sentinel
+        }
+        if (FMT == 0) reinterpret_cast<uint32_t*>(out)[g] = w[0];
+        else if (FMT == 1) reinterpret_cast<uint2*>(out)[g] = make_uint2(w[0], w[1]);
+        else reinterpret_cast<uint4*>(out)[g] = make_uint4(w[0], w[1], w[2], w[3]);
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(overflow, 1u);
 }
 
-// Two depths per byte (low nibble first), 0xF for unreached; depths must be < 15.
-__global__ void packDepths4Kernel(const uint32_t* d, uint64_t count, uint8_t* out, unsigned* overflow) {
-    bool bad = false;
-    const uint64_t pairs = (count + 1) / 2;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t v0 = d[2 * i], v1 = 2 * i + 1 < count ? d[2 * i + 1] : 0xFFFFFFFFu;
-        bad |= (v0 != 0xFFFFFFFFu && v0 >= 15u) || (v1 != 0xFFFFFFFFu && v1 >= 15u);
-        const uint32_t a = v0 == 0xFFFFFFFFu ? 15u : (v0 & 15u), b = v1 == 0xFFFFFFFFu ? 15u : (v1 & 15u);
-        out[i] = (uint8_t)(a | (b << 4));
+inline uint32_t widenOne(int fmt, const uint8_t* in, uint64_t i) {
+    if (fmt == 0) {
+        const uint32_t v = (in[i / 2] >> (4 * (i & 1))) & 15u;
+        return v == 15u ? kInf : v;
     }
-    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(overflow, 1u);
+    if (fmt == 1) return in[i] == 0xFFu ? kInf : in[i];
+    const uint32_t v = reinterpret_cast<const uint16_t*>(in)[i];
+    return v == 0xFFFFu ? kInf : v;
 }
 
-void widen4(const uint8_t* in, uint32_t* out, uint64_t count) {  // count even, or the array's tail
-    const int threads = std::max(1, std::min(16, omp_get_max_threads()));
-    const int64_t pairs = (int64_t)(count / 2);
-#pragma omp parallel for num_threads(threads) schedule(static) if (count >= (1u << 16))
-    for (int64_t i = 0; i < pairs; ++i) {
-        const uint32_t b = in[i], lo = b & 15u, hi = b >> 4;
-        out[2 * i] = lo == 15u ? 0xFFFFFFFFu : lo;
-        out[2 * i + 1] = hi == 15u ? 0xFFFFFFFFu : hi;
-    }
-    if (count & 1) {
-        const uint32_t lo = in[pairs] & 15u;
-        out[count - 1] = lo == 15u ? 0xFFFFFFFFu : lo;
-    }
+inline void store4(uint32_t* o, __m128i x) { _mm_storeu_si128(reinterpret_cast<__m128i*>(o), x); }
+
+// Sixteen bytes b (sentinel 0xFF) to sixteen uint32 (sentinel all ones): the
+// sentinel's compare mask is the high part in both unpacking steps.
+inline void widen16(__m128i b, uint32_t* o) {
+    const __m128i m = _mm_cmpeq_epi8(b, _mm_set1_epi8(-1));
+    const __m128i lo = _mm_unpacklo_epi8(b, m), hi = _mm_unpackhi_epi8(b, m);
+    const __m128i ml = _mm_unpacklo_epi8(m, m), mh = _mm_unpackhi_epi8(m, m);
+    store4(o, _mm_unpacklo_epi16(lo, ml));
+    store4(o + 4, _mm_unpackhi_epi16(lo, ml));
+    store4(o + 8, _mm_unpacklo_epi16(hi, mh));
+    store4(o + 12, _mm_unpackhi_epi16(hi, mh));
 }
 
-template <typename T>
-void widen(const T* in, uint32_t* out, uint64_t count) {
-    const uint32_t sentinel = (uint32_t)(T)~0u;
-    const int threads = std::max(1, std::min(16, omp_get_max_threads()));
-#pragma omp parallel for num_threads(threads) schedule(static) if (count >= (1u << 16))
-    for (int64_t i = 0; i < (int64_t)count; ++i) {
-        const uint32_t v = in[i];
-        out[i] = v == sentinel ? 0xFFFFFFFFu : v;
+// Depths [lo, hi) of a packed array; lo is a multiple of 32.  Plain stores: with
+// stores that bypass the cache the 16.8 MB of R-MAT 22 take 358 us a call, so 307.
+void widenRange(int fmt, const uint8_t* in, uint64_t lo, uint64_t hi, uint32_t* out) {
+    uint64_t i = lo;
+    if (fmt == 0) {
+        const __m128i low = _mm_set1_epi8(15);
+        for (; i + 32 <= hi; i += 32) {
+            const __m128i x = _mm_loadu_si128(reinterpret_cast<const __m128i*>(in + i / 2));
+            const __m128i a = _mm_and_si128(x, low), b = _mm_and_si128(_mm_srli_epi16(x, 4), low);
+            const __m128i y0 = _mm_unpacklo_epi8(a, b), y1 = _mm_unpackhi_epi8(a, b);
+            widen16(_mm_or_si128(y0, _mm_cmpeq_epi8(y0, low)), out + i);
+            widen16(_mm_or_si128(y1, _mm_cmpeq_epi8(y1, low)), out + i + 16);
+        }
+    } else if (fmt == 1) {
+        for (; i + 16 <= hi; i += 16)
+            widen16(_mm_loadu_si128(reinterpret_cast<const __m128i*>(in + i)), out + i);
+    } else {
+        const __m128i ones = _mm_set1_epi16(-1);
+        for (; i + 8 <= hi; i += 8) {
+            const __m128i x = _mm_loadu_si128(reinterpret_cast<const __m128i*>(in + 2 * i));
+            const __m128i m = _mm_cmpeq_epi16(x, ones);
+            store4(out + i, _mm_unpacklo_epi16(x, m));
+            store4(out + i + 4, _mm_unpackhi_epi16(x, m));
+        }
     }
-}
-
-template <typename T>
-bool packedCopy(gb_bfs* h, const uint32_t* d, uint64_t count, uint32_t* out) {
-    cudaStream_t st = h->stream.s;
-    h->packDev.ensure(count * sizeof(T));
-    h->packHost.ensure(count * sizeof(T));
-    h->packFlag.ensure(1);
-    h->packFlagHost.ensure(1);
-    GB_CUDA(cudaMemsetAsync(h->packFlag.get(), 0, 4, st));
-    T* dp = reinterpret_cast<T*>(h->packDev.get());
-    T* hp = reinterpret_cast<T*>(h->packHost.p);
-    packDepthsKernel<T><<<deviceSmCount() * 8, 256, 0, st>>>(d, count, dp, h->packFlag.get());
-    GB_LAUNCH_CHECK();
-    const uint64_t chunks = (count + kPackChunk - 1) / kPackChunk;
-    while (h->packEv.size() < chunks) {
-        cudaEvent_t e;
-        GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        h->packEv.push_back(e);
-    }
-    for (uint64_t c = 0; c < chunks; ++c) {
-        const uint64_t lo = c * kPackChunk, len = std::min(kPackChunk, count - lo);
-        GB_CUDA(cudaMemcpyAsync(hp + lo, dp + lo, len * sizeof(T), cudaMemcpyDeviceToHost, st));
-        if (c + 1 == chunks)
-            GB_CUDA(cudaMemcpyAsync(h->packFlagHost.p, h->packFlag.get(), 4, cudaMemcpyDeviceToHost, st));
-        GB_CUDA(cudaEventRecord(h->packEv[c], st));
-    }
-    for (uint64_t c = 0; c < chunks; ++c) {
-        const uint64_t lo = c * kPackChunk, len = std::min(kPackChunk, count - lo);
-        GB_CUDA(cudaEventSynchronize(h->packEv[c]));
-        widen(hp + lo, out + lo, len);
-    }
-    return *h->packFlagHost.p == 0;
-}
-
-bool packedCopy4(gb_bfs* h, const uint32_t* d, uint64_t count, uint32_t* out) {
-    cudaStream_t st = h->stream.s;
-    const uint64_t bytes = (count + 1) / 2;
-    h->packDev.ensure(bytes);
-    h->packHost.ensure(bytes);
-    h->packFlag.ensure(1);
-    h->packFlagHost.ensure(1);
-    GB_CUDA(cudaMemsetAsync(h->packFlag.get(), 0, 4, st));
-    uint8_t* dp = h->packDev.get();
-    uint8_t* hp = h->packHost.p;
-    packDepths4Kernel<<<deviceSmCount() * 8, 256, 0, st>>>(d, count, dp, h->packFlag.get());
-    GB_LAUNCH_CHECK();
-    const uint64_t chunks = (count + kPackChunk - 1) / kPackChunk;  // kPackChunk is even
-    while (h->packEv.size() < chunks) {
-        cudaEvent_t e;
-        GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        h->packEv.push_back(e);
-    }
-    for (uint64_t c = 0; c < chunks; ++c) {
-        const uint64_t lo = c * kPackChunk, len = std::min(kPackChunk, count - lo);
-        GB_CUDA(cudaMemcpyAsync(hp + lo / 2, dp + lo / 2, (len + 1) / 2, cudaMemcpyDeviceToHost, st));
-        if (c + 1 == chunks)
-            GB_CUDA(cudaMemcpyAsync(h->packFlagHost.p, h->packFlag.get(), 4, cudaMemcpyDeviceToHost, st));
-        GB_CUDA(cudaEventRecord(h->packEv[c], st));
-    }
-    for (uint64_t c = 0; c < chunks; ++c) {
-        const uint64_t lo = c * kPackChunk, len = std::min(kPackChunk, count - lo);
-        GB_CUDA(cudaEventSynchronize(h->packEv[c]));
-        widen4(hp + lo / 2, out + lo, len);
-    }
-    return *h->packFlagHost.p == 0;
+    for (; i < hi; ++i) out[i] = widenOne(fmt, in, i);
 }
 
 }  // namespace
 
-int packFormat(uint64_t count, uint32_t levels) {
-    if (count < kPackMin) return -1;
+void widenPacked(int fmt, const uint8_t* in, uint64_t count, uint32_t* out) {
+    if (count <= kOneThread) {
+        widenRange(fmt, in, 0, count, out);
+        return;
+    }
+    const int threads = hostThreads(16);
+    const uint64_t step = ((count + threads - 1) / threads + 31) / 32 * 32;
+#pragma omp parallel for num_threads(threads) schedule(static)
+    for (int t = 0; t < threads; ++t) {
+        const uint64_t lo = std::min(count, (uint64_t)t * step), hi = std::min(count, lo + step);
+        if (lo < hi) widenRange(fmt, in, lo, hi, out);
+    }
+}
+
+int packFormat(uint32_t levels) {
     if (levels < 15) return 0;
     if (levels < 255) return 1;
     if (levels < 65535) return 2;
@@ -151,29 +138,101 @@ uint64_t packedBytes(int fmt, uint64_t count) {
 }
 
 void enqueuePack(int fmt, const uint32_t* d, uint64_t count, uint8_t* dev, unsigned* overflow, cudaStream_t st) {
-    const int grid = deviceSmCount() * 8;
-    if (fmt == 0) packDepths4Kernel<<<grid, 256, 0, st>>>(d, count, dev, overflow);
-    else if (fmt == 1) packDepthsKernel<uint8_t><<<grid, 256, 0, st>>>(d, count, dev, overflow);
-    else packDepthsKernel<uint16_t><<<grid, 256, 0, st>>>(d, count, reinterpret_cast<uint16_t*>(dev), overflow);
+    const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((count / 8 + 255) / 256, (uint64_t)deviceSmCount() * 8));
+    if (fmt == 0) packDepthsKernel<0><<<grid, 256, 0, st>>>(d, count, dev, overflow);
+    else if (fmt == 1) packDepthsKernel<1><<<grid, 256, 0, st>>>(d, count, dev, overflow);
+    else packDepthsKernel<2><<<grid, 256, 0, st>>>(d, count, dev, overflow);
     GB_LAUNCH_CHECK();
 }
 
-void widenPacked(int fmt, const uint8_t* in, uint64_t count, uint32_t* out) {
-    if (fmt == 0) widen4(in, out, count);
-    else if (fmt == 1) widen(in, out, count);
-    else widen(reinterpret_cast<const uint16_t*>(in), out, count);
+void beginDepths(gb_bfs* h, const uint32_t* d, uint64_t count, uint32_t levels, DepthReturn& r) {
+    cudaStream_t st = h->stream.s;
+    r.d = d;
+    r.count = count;
+    r.fmt = packFormat(levels);
+    if (r.fmt < 0) return;
+    const uint64_t bytes = packedBytes(r.fmt, count);
+    h->packDev.ensure(bytes + 16);
+    h->packHost.ensure(bytes);
+    if (!h->packFlag.get()) {  // zero but after an overflow, which endDepths clears again
+        h->packFlag.ensure(1);
+        GB_CUDA(cudaMemsetAsync(h->packFlag.get(), 0, 4, st));
+    }
+    h->packFlagHost.ensure(1);
+    enqueuePack(r.fmt, d, count, h->packDev.get(), h->packFlag.get(), st);
+    GB_CUDA(cudaMemcpyAsync(h->packFlagHost.p, h->packFlag.get(), 4, cudaMemcpyDeviceToHost, st));
+    const uint64_t chunks = (count + kPackChunk - 1) / kPackChunk;
+    while (h->packEv.size() < chunks) {
+        cudaEvent_t e;
+        GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        h->packEv.push_back(e);
+    }
+    for (uint64_t c = 0; c < chunks; ++c) {
+        const uint64_t lo = packedBytes(r.fmt, c * kPackChunk), hi = packedBytes(r.fmt, std::min(count, (c + 1) * kPackChunk));
+        GB_CUDA(cudaMemcpyAsync(h->packHost.p + lo, h->packDev.get() + lo, hi - lo, cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaEventRecord(h->packEv[c], st));
+    }
+}
+
+void waitDepths(gb_bfs* h, const DepthReturn& r) {
+    if (r.fmt < 0) GB_CUDA(cudaStreamSynchronize(h->stream.s));
+    else GB_CUDA(cudaEventSynchronize(h->packEv[0]));
+}
+
+void endDepths(gb_bfs* h, const DepthReturn& r, uint32_t levels, uint32_t* out) {
+    if (r.fmt >= 0) {
+        const uint64_t chunks = (r.count + kPackChunk - 1) / kPackChunk;
+        for (uint64_t c = 0; c < chunks; ++c) {
+            GB_CUDA(cudaEventSynchronize(h->packEv[c]));
+            if (*h->packFlagHost.p) break;  // copied ahead of the chunks
+            const uint64_t lo = c * kPackChunk, len = std::min(kPackChunk, r.count - lo);
+            widenPacked(r.fmt, h->packHost.p + packedBytes(r.fmt, lo), len, out + lo);
+        }
+        if (*h->packFlagHost.p == 0) return;
+        GB_CUDA(cudaStreamSynchronize(h->stream.s));
+        GB_CUDA(cudaMemsetAsync(h->packFlag.get(), 0, 4, h->stream.s));
+        // the guessed width was too narrow: once more with the level count, which fits
+        if (packFormat(levels) > r.fmt) {
+            DepthReturn again;
+            beginDepths(h, r.d, r.count, levels, again);
+            endDepths(h, again, levels, out);
+            return;
+        }
+    }
+    h->staged.run(r.d, r.count * 4, out, h->stream.s);
 }
 
 void copyDepthsToHost(gb_bfs* h, const uint32_t* d, uint64_t count, uint32_t* out, uint32_t levels) {
-    bool done = false;
-    if (count >= kPackMin) {
-        if (levels < 15) done = packedCopy4(h, d, count, out);
-        else if (levels < 255) done = packedCopy<uint8_t>(h, d, count, out);
-        else if (levels < 65535) done = packedCopy<uint16_t>(h, d, count, out);
-    }
-    if (!done) {
-        GB_CUDA(cudaMemcpyAsync(out, d, count * 4, cudaMemcpyDeviceToHost, h->stream.s));
-        GB_CUDA(cudaStreamSynchronize(h->stream.s));
+    DepthReturn r;
+    beginDepths(h, d, count, levels, r);
+    endDepths(h, r, levels, out);
+}
+
+void StagedCopy::run(const void* dev, size_t bytes, void* out, cudaStream_t st) {
+    const size_t chunks = (bytes + kChunk - 1) / kChunk;
+    ring_.ensure(std::min(bytes, kSlots * kChunk));
+    for (cudaEvent_t& e : ev_)
+        if (!e) GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    const uint8_t* src = static_cast<const uint8_t*>(dev);
+    uint8_t* dst = static_cast<uint8_t*>(out);
+    auto length = [&](size_t c) { return std::min(kChunk, bytes - c * kChunk); };
+    auto enqueue = [&](size_t c) {
+        GB_CUDA(cudaMemcpyAsync(ring_.p + c % kSlots * kChunk, src + c * kChunk, length(c), cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaEventRecord(ev_[c % kSlots], st));
+    };
+    for (size_t c = 0; c < std::min<size_t>(chunks, kSlots); ++c) enqueue(c);
+    const int threads = hostThreads(4);
+    for (size_t c = 0; c < chunks; ++c) {
+        GB_CUDA(cudaEventSynchronize(ev_[c % kSlots]));
+        const uint8_t* from = ring_.p + c % kSlots * kChunk;
+        uint8_t* to = dst + c * kChunk;
+        const size_t len = length(c);
+        constexpr size_t kPiece = 1 << 16;
+        const int pieces = (int)((len + kPiece - 1) / kPiece);
+#pragma omp parallel for num_threads(threads) schedule(static) if (pieces > 3)
+        for (int p = 0; p < pieces; ++p)
+            std::memcpy(to + p * kPiece, from + p * kPiece, std::min(kPiece, len - p * kPiece));
+        if (c + kSlots < chunks) enqueue(c + kSlots);
     }
 }
 

@@ -830,6 +830,12 @@ __global__ void __launch_bounds__(kBlkThreads, 1) prBlockedKernel(PrArgs a, BlkA
     finishBlock<0>(a, acc);
 }
 
+// out[v] = in[map[v]].
+__global__ void unpermuteKernel(const float* __restrict__ in, const uint32_t* __restrict__ map, uint32_t n, float* out) {
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
+        out[v] = in[map[v]];
+}
+
 // Double-precision Jacobi pull (warp per vertex): the GPU oracle against
 // which FP32 runs are measured at sizes where the CPU reference is slow.
 __global__ void prPullF64Kernel(PrArgs a) {
@@ -1158,6 +1164,7 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
     GB_CUDA(cudaStreamSynchronize(stream.s));
     res.gpu_ms = ev.ms();
     if (hc.error) throw Error(GB_ERR_TIMEOUT, "PageRank: a device wait for a staging copy exceeded its limit");
+    lastCur = hc.cur;
     res.iters = hc.iters;
     res.floor_stop = hc.floorStop;
     if (tolMode) {
@@ -1170,23 +1177,18 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
 void gb_pr::ranks(float* out) {
     if (lastVariant < 0) throw Error(GB_ERR_STATE, "ranks() before run()");
     if (lastVariant == GB_PR_PULL_F64) throw Error(GB_ERR_STATE, "last run was FP64: use the double ranks");
-    GbPrControl hc{};
-    GB_CUDA(cudaMemcpy(&hc, ctl.get(), sizeof hc, cudaMemcpyDeviceToHost));
-    const std::vector<uint32_t>* map = lastVariant == GB_PR_PULL_ADAPTIVE ? &permA : gsLastRun ? &gsNewId : nullptr;
-    if (!map) {
-        GB_CUDA(cudaMemcpy(out, r[hc.cur].get(), n * 4, cudaMemcpyDeviceToHost));
-        return;
+    const float* from = r[lastCur].get();
+    const uint32_t* map = lastVariant == GB_PR_PULL_ADAPTIVE ? permADev.get() : gsLastRun ? gsNewIdDev.get() : nullptr;
+    if (map) {  // relabeled layout: back to the caller's ids
+        // into the contributions' buffer, which every run writes afresh
+        unpermuteKernel<<<gridFor(n, 256), 256, 0, stream.s>>>(from, map, (uint32_t)n, contrib[0].get());
+        GB_LAUNCH_CHECK();
+        from = contrib[0].get();
     }
-    std::vector<float> tmp(n);  // relabeled layout: back to the caller's ids
-    GB_CUDA(cudaMemcpy(tmp.data(), r[hc.cur].get(), n * 4, cudaMemcpyDeviceToHost));
-    const uint32_t* m = map->data();
-#pragma omp parallel for schedule(static)
-    for (int64_t v = 0; v < (int64_t)n; ++v) out[v] = tmp[m[v]];
+    staged.run(from, n * 4, out, stream.s);
 }
 
 void gb_pr::ranks64(double* out) {
     if (lastVariant != GB_PR_PULL_F64) throw Error(GB_ERR_STATE, "no FP64 run to read");
-    GbPrControl hc{};
-    GB_CUDA(cudaMemcpy(&hc, ctl.get(), sizeof hc, cudaMemcpyDeviceToHost));
-    GB_CUDA(cudaMemcpy(out, r64[hc.cur].get(), n * 8, cudaMemcpyDeviceToHost));
+    staged.run(r64[lastCur].get(), n * 8, out, stream.s);
 }

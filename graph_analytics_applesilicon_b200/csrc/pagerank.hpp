@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_copy.hpp"
 
 constexpr uint32_t kGsHubMin = 4096;  // natural-order GS: split vertices with this many in-edges
 constexpr uint32_t kGsNatSlices = 8;    // natural-order GS: the main list runs as this many ordered launches
@@ -74,6 +75,7 @@ struct gb_pr {
     gb::DevBuf<unsigned> hubDone;    // per hub: chunks finished (reset by the last)
     gb::DevBuf<float> hubPart;       // per chunk: Kahan sum, compensation
     std::vector<uint32_t> permA;     // old id -> new id
+    gb::DevBuf<uint32_t> permADev;
     uint32_t nHubs = 0, nChunks = 0;
     uint32_t binLo[8] = {0}, binHi[8] = {0}, binG[8] = {0};  // group-size ranges (G = 1..32)
     int nBins = 0;
@@ -103,8 +105,11 @@ struct gb_pr {
     std::vector<uint32_t> gsSetStart;    // colored: set k = ids [start[k], start[k+1])
     gb::DevBuf<uint32_t> rowGS, colGS, outdegGS;
     std::vector<uint32_t> gsNewId;
+    gb::DevBuf<uint32_t> gsNewIdDev;
     bool gsLastRun = false;
     int lastVariant = -1;
+    int lastCur = 0;                     // rank buffer of the last run
+    gb::StagedCopy staged;
 
     // blocked pull: packed (row in block << 16 | column in part) per edge,
     // grouped by row block then part; blkOff[k * nParts + p] starts tile

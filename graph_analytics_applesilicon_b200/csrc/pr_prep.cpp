@@ -103,6 +103,7 @@ void gb_pr::prepareAdaptive(uint32_t smallMax, uint32_t largeMin) {
     upload(rowA, row);
     upload(colA, col);
     upload(outdegA, od);
+    upload(permADev, permA);
     upload(hubChunks, chunks);
     upload(hubFirst, first);
     hubDone.ensure(nHubs + 1);
@@ -204,6 +205,7 @@ void gb_pr::prepareGS(uint32_t pairMaxOutdeg) {
         GB_CUDA(cudaMemcpy(rowGS.get(), row.data(), (n + 1) * 4, cudaMemcpyHostToDevice));
         GB_CUDA(cudaMemcpy(colGS.get(), col.data(), col.size() * 4, cudaMemcpyHostToDevice));
         GB_CUDA(cudaMemcpy(outdegGS.get(), deg.data(), n * 4, cudaMemcpyHostToDevice));
+        upload(gsNewIdDev, gsNewId);
         // per set: split hubs (>= kGsHubMin in-edges) into warp chunks, the rest
         // into group-size classes (thread per vertex below 16 in-edges)
         gsSetLayout.clear();
