@@ -63,7 +63,10 @@ int gb_pr_create(uint64_t n, const uint32_t* out_row_ptr, const uint32_t* out_co
         h->hostOutdeg.assign(outdeg, outdeg + n);
         for (int i = 0; i < 2; ++i) {
             h->r[i].ensure(n + 1);
-            h->contrib[i].ensure(n + 4);  // the blocked pull copies whole 16-byte groups past n
+            // 4 floats of slack: the blocked pull copies whole 16-byte groups past
+            // n, and the adaptive lists' padding gathers entry n, which is 0
+            h->contrib[i].ensure(n + 4);
+            GB_CUDA(cudaMemset(h->contrib[i].get() + n, 0, 16));
         }
         h->ctl.ensure(1);
         h->partF.ensure(2 * 4096);

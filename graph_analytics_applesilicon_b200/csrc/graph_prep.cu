@@ -258,6 +258,12 @@ int keyBits(uint64_t n) {
     return b;
 }
 
+void permutedKeys(const uint32_t* rp, const uint32_t* ci, uint64_t n, uint64_t m, int b, const uint32_t* perm,
+                  unsigned long long* keys, cudaStream_t st) {
+    csrKeysKernel<<<prepGrid(n * 32, 256), 256, 0, st>>>(rp, ci, n, m, b, 2, perm, keys);
+    GB_LAUNCH_CHECK();
+}
+
 // Sorts N keys whose used bits are [0, bits) in place (a holds the result).
 void radixSortKeys(DevBuf<unsigned long long>& a, DevBuf<unsigned long long>& tmp, uint64_t N, int bits,
                    ScanScratch& sc, cudaStream_t st, DevBuf<uint32_t>* countsScratch) {

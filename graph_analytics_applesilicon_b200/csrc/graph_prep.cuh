@@ -17,6 +17,12 @@ int keyBits(uint64_t n);
 // countsScratch (optional) is reused for the digit histograms across calls.
 void radixSortKeys(DevBuf<unsigned long long>& a, DevBuf<unsigned long long>& tmp, uint64_t N, int bits,
                    ScanScratch& sc, cudaStream_t st, DevBuf<uint32_t>* countsScratch = nullptr);
+// One key (perm[row] << b) | perm[column] per entry of a device CSR.
+void permutedKeys(const uint32_t* rp, const uint32_t* ci, uint64_t n, uint64_t m, int b, const uint32_t* perm,
+                  unsigned long long* keys, cudaStream_t st);
+// Vertices by descending degree, ties by id: order[i] = the i-th, rank its
+// inverse (either may be null).
+void degreeRank(const uint32_t* rp, uint64_t n, uint32_t* order, uint32_t* rank, ScanScratch& sc, cudaStream_t st);
 // Sorted keys -> host CSR in *out (n rows, b column bits), dropping repeated
 // keys (unique) and self-loops (dropSelf); out->flags = flags.
 void keysToCsr(DevBuf<unsigned long long>& keys, uint64_t N, uint64_t n, int b, bool unique, bool dropSelf,

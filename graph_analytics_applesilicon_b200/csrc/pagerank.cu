@@ -118,6 +118,23 @@ __device__ __forceinline__ void storeJacobi(const PrArgs& a, int cur, bool withD
     }
 }
 
+// The same with the out-degree and the old rank already loaded (a pull asks for
+// them before its gathers); INPLACE: the contribution goes back to contrib[0],
+// and the dangling mass and residual are left to later kernels.
+template <bool INPLACE>
+__device__ __forceinline__ void storePulled(const PrArgs& a, int cur, bool withDelta, uint32_t v, float val,
+                                            uint32_t od, float old, IterAcc& acc) {
+    a.r[cur ^ 1][v] = val;
+    a.contrib[INPLACE ? 0 : cur ^ 1][v] = od ? val / (float)od : 0.0f;
+    if (INPLACE) return;
+    if (!od) acc.dang.add(val);
+    if (withDelta) {
+        const double d = fabs((double)val - (double)old);
+        acc.dsum += d;
+        acc.dmax = fmaxf(acc.dmax, (float)d / fmaxf(val, a.invN));
+    }
+}
+
 // Block-wide reduction of IterAcc into thread 0 (fixed order: deterministic).
 __device__ __forceinline__ IterAcc blockReduceAcc(IterAcc acc) {
     __shared__ float sHi[32], sLo[32], sMax[32];
@@ -253,9 +270,6 @@ __global__ void prInit64Kernel(PrArgs a) {
     finishBlock<5>(a, acc);
 }
 
-// Kahan sum of contrib over v's in-list [b, e), lanes of a group of G threads
-// striding it; 16-byte aligned vector loads of col_idx (entries outside
-// [b, e) are masked; the array is padded so the last vector stays in bounds).
 // Adjacency (col_idx) is read once per sweep: load it without allocating in
 // L1, so L1 keeps the contributions that many rows gather (hub-first order
 // puts the most-gathered ones together).
@@ -278,32 +292,11 @@ __device__ __forceinline__ float ldContrib(const float* p) {
     return __ldg(p);
 }
 
-template <int G, bool COHERENT = false>
-__device__ __forceinline__ float gatherStrided(const uint32_t* __restrict__ ci, const float* contrib, uint32_t b,
-                                               uint32_t e, unsigned rank) {
-    Kahan k;
-    for (uint32_t i = (b & ~3u) + 4 * rank; i < e; i += 4 * G) {
-        const uint4 q = ldStream4(ci + i);
-        if (i >= b) k.add(ldContrib<COHERENT>(contrib + q.x));
-        if (i + 1 >= b && i + 1 < e) k.add(ldContrib<COHERENT>(contrib + q.y));
-        if (i + 2 >= b && i + 2 < e) k.add(ldContrib<COHERENT>(contrib + q.z));
-        if (i + 3 >= b && i + 3 < e) k.add(ldContrib<COHERENT>(contrib + q.w));
-    }
-    return k.sum;
-}
-
-template <bool COHERENT = false>
-__device__ __forceinline__ float gatherSerial(const uint32_t* __restrict__ ci, const float* contrib, uint32_t b,
-                                              uint32_t e) {
-    Kahan k;
-    for (uint32_t i = b; i < e; ++i) k.add(ldContrib<COHERENT>(contrib + ldStream(ci + i)));
-    return k.sum;
-}
-
 // Kahan sum of contrib over [b, e) by group rank `rank` of G lanes (runtime
-// G), 16-byte aligned vector loads of col_idx.
+// G), 16-byte aligned vector loads of col_idx (entries outside [b, e) are
+// masked; the array is padded so the last vector stays in bounds).
 template <bool COHERENT>
-__device__ __forceinline__ float gatherGroup(const uint32_t* __restrict__ ci, const float* contrib, uint32_t b,
+__device__ __forceinline__ Kahan gatherKahan(const uint32_t* __restrict__ ci, const float* contrib, uint32_t b,
                                              uint32_t e, unsigned rank, unsigned G) {
     // Two 16-byte vectors per lane per step (8 gathers in flight); entries
     // are added in the same per-lane order as a one-vector loop.
@@ -330,7 +323,13 @@ __device__ __forceinline__ float gatherGroup(const uint32_t* __restrict__ ci, co
         k.add(b2);
         k.add(b3);
     }
-    return k.sum;
+    return k;
+}
+
+template <bool COHERENT>
+__device__ __forceinline__ float gatherGroup(const uint32_t* __restrict__ ci, const float* contrib, uint32_t b,
+                                             uint32_t e, unsigned rank, unsigned G) {
+    return gatherKahan<COHERENT>(ci, contrib, b, e, rank, G).sum;
 }
 
 // One warp chunk of a split vertex: the warp's sum goes to the chunk's
@@ -356,15 +355,147 @@ __device__ __forceinline__ void chunkTask(const PrArgs& a, uint32_t t, const flo
     }
 }
 
-// Jacobi pull iteration.  MODE 0: thread per vertex (gpu_pull_scalar);
-// 1: warp per vertex (gpu_pull_vector); 2: degree-adaptive over the three
-// in-degree bins in one launch (block per large, warp per medium, thread per
-// small vertex; gpu_pull_adaptive).  INPLACE: the sweep of an in-place
-// variant -- contributions are read and rewritten in contrib[0] as vertices
-// are updated, and dangling / residual / control are left to the
-// contribution, sum and scale kernels.
-template <int MODE, bool INPLACE>
-__global__ void prPullKernel(PrArgs a) {
+// The lanes' float-float values summed, in every lane 0 (a fixed order).
+__device__ __forceinline__ FF warpSumFF(float hi, float lo) {
+    FF f;
+    f.hi = hi;
+    f.lo = lo;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        FF x;
+        x.hi = __shfl_xor_sync(kFull, f.hi, o);
+        x.lo = __shfl_xor_sync(kFull, f.lo, o);
+        f.add(x);
+    }
+    return f;
+}
+
+// Chunk t of a split list (hub `hub`, chunks [first, first + cnt)), summed by a
+// warp: k is the lane's part.  True, with the list's sum in lane 0's f, in the
+// warp that finishes the list's last chunk: the chunks' sums are float-float and
+// are added by lane, then across the lanes, in a fixed order.
+__device__ __forceinline__ bool splitSum(const PrArgs& a, uint32_t t, uint32_t hub, uint32_t first, uint32_t cnt,
+                                         const Kahan& k, FF& f) {
+    const unsigned lane = laneId();
+    f = warpSumFF(k.sum, -k.comp);
+    if (cnt == 1) return true;
+    unsigned old = 0;
+    if (lane == 0) {
+        a.hubPart[2 * t] = f.hi;
+        a.hubPart[2 * t + 1] = f.lo;
+        __threadfence();
+        old = atomicAdd(&a.hubDone[hub], 1u);
+    }
+    if (__shfl_sync(kFull, old, 0) != cnt - 1) return false;
+    __threadfence();
+    FF g;
+    for (uint32_t i = lane; i < cnt; i += 32) {
+        FF x;
+        x.hi = __ldcg(&a.hubPart[2 * (first + i)]);
+        x.lo = __ldcg(&a.hubPart[2 * (first + i) + 1]);
+        g.add(x);
+    }
+    f = warpSumFF(g.hi, g.lo);
+    if (lane == 0) a.hubDone[hub] = 0;
+    return true;
+}
+
+// The adaptive pull over the relabeled, padded lists (pr_layout.cu): warp tasks
+// are the chunks of the split lists, then the runs' tasks.  A list's place and
+// length come from its run, and the vertex's out-degree and old rank are
+// requested before the gathers, so a task's chain is vectors, contributions,
+// store.  Two vectors per lane and step (8 gathers in flight).
+// Kahan sum over `count` vectors at p, p + step, ...
+template <bool COHERENT>
+__device__ __forceinline__ Kahan gatherVecs(const uint4* p, uint32_t count, uint32_t step, const float* contrib) {
+    Kahan k;
+    for (uint32_t i = 0; i < count; i += 2, p += 2 * step) {
+        const bool two = i + 1 < count;
+        const uint4 q = ldStream4(reinterpret_cast<const uint32_t*>(p));
+        const uint4 r = two ? ldStream4(reinterpret_cast<const uint32_t*>(p + step)) : make_uint4(0, 0, 0, 0);
+        const float a0 = ldContrib<COHERENT>(contrib + q.x), a1 = ldContrib<COHERENT>(contrib + q.y);
+        const float a2 = ldContrib<COHERENT>(contrib + q.z), a3 = ldContrib<COHERENT>(contrib + q.w);
+        const float b0 = two ? ldContrib<COHERENT>(contrib + r.x) : 0.f, b1 = two ? ldContrib<COHERENT>(contrib + r.y) : 0.f;
+        const float b2 = two ? ldContrib<COHERENT>(contrib + r.z) : 0.f, b3 = two ? ldContrib<COHERENT>(contrib + r.w) : 0.f;
+        k.add(a0);
+        k.add(a1);
+        k.add(a2);
+        k.add(a3);
+        if (two) {
+            k.add(b0);
+            k.add(b1);
+            k.add(b2);
+            k.add(b3);
+        }
+    }
+    return k;
+}
+
+// Bound by the rate of random 4-byte gathers: Chung-Lu, 233M entries, 816 us a
+// sweep = 285 G/s (1,047 with row pointers and ragged lists); web graph, 5M,
+// 34 us (48.7); R-MAT 18, 4M, 22 us (31).  56 registers, 36 warps per SM: capped
+// at 48 the sweeps take 836 / 34 / 22.4 us, at 40 883 / 38 / 26.
+template <bool INPLACE>
+__global__ void __maxnreg__(56) prAdaptiveKernel(PrArgs a, const uint4* __restrict__ vecs, const GbPrRun* __restrict__ runs,
+                                 uint32_t nRuns, uint32_t nRunTasks) {
+    const GbPrControl* c = a.ctl;
+    if (ldvi(&c->stopped)) return;
+    const int cur = c->cur;
+    const float dang = c->dangHi + c->dangLo;
+    const bool withDelta = !INPLACE && c->withDelta;
+    const float* contrib = INPLACE ? a.contrib[0] : a.contrib[cur];
+    const float* rOld = a.r[cur];
+    IterAcc acc;
+    auto store = [&](uint32_t v, float s, uint32_t od, float old) {
+        storePulled<INPLACE>(a, cur, withDelta, v, prValue(a, s, dang), od, old, acc);
+    };
+    const unsigned lane = laneId();
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5, total = a.nChunks + nRunTasks;
+    uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    for (; t < a.nChunks; t += nwarps) {  // warp-uniform
+        const uint4 h = a.chunks[t];  // vertex, first vector, end vector, hub
+        const uint32_t first = a.hubFirst[2 * h.w], cnt = a.hubFirst[2 * h.w + 1];
+        const Kahan k = gatherVecs<INPLACE>(vecs + h.y + lane, h.y + lane < h.z ? (h.z - h.y - lane + 31) / 32 : 0u, 32, contrib);
+        FF f;
+        if (splitSum(a, t, h.w, first, cnt, k, f) && lane == 0)
+            store(h.x, f.hi + f.lo, a.outdeg[h.x], withDelta ? rOld[h.x] : 0.f);
+    }
+    GbPrRun r{};
+    uint32_t end = 0;  // first task beyond run r
+    for (; t < total; t += nwarps) {
+        const uint32_t rt = t - a.nChunks;
+        if (rt >= end) {
+            uint32_t lo = 0, hi = nRuns - 1;
+            while (lo < hi) {  // last run with task0 <= rt
+                const uint32_t mid = (lo + hi + 1) >> 1;
+                if (runs[mid].task0 <= rt) lo = mid;
+                else hi = mid - 1;
+            }
+            r = runs[lo];
+            end = lo + 1 < nRuns ? runs[lo + 1].task0 : nRunTasks;
+        }
+        const unsigned G = 1u << r.lg, sub = lane & (G - 1);
+        const uint32_t idx = (rt - r.task0) * (32u >> r.lg) + (lane >> r.lg), v = r.v0 + idx;
+        const bool active = v < r.vEnd, lead = active && sub == 0;
+        const uint32_t od = lead ? a.outdeg[v] : 0u;
+        const float old = lead && withDelta ? rOld[v] : 0.f;
+        const uint4* p = vecs + r.e0 + (r.inter ? (uint64_t)(rt - r.task0) * 32 * r.vecs + lane : (uint64_t)idx * r.vecs + sub);
+        const uint32_t count = active && sub < r.vecs ? (r.vecs - sub + G - 1) >> r.lg : 0u;
+        float s = gatherVecs<INPLACE>(p, count, r.inter ? 32 : G, contrib).sum;
+        for (unsigned o = G >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+        if (lead) store(v, s, od, old);
+    }
+    if (!INPLACE) finishBlock<0>(a, acc);
+}
+
+// The scalar (lg = 0: a lane per list) and vector pulls over the graph as
+// given, 1 << lg lanes per list: warp tasks are the chunks of the split lists
+// (pr_layout.cu), then 32 >> lg vertices each, those with split lists left out.
+// A sweep of R-MAT 18 / web 875k / Chung-Lu 3.07M: vector 33 / 49 / 1,003 us (a
+// warp per list: 185 / 1,020 / 1,331), scalar 33 / 46 / 1,030 (a thread per list:
+// 1,176 / 8,646 / 4,655).
+template <bool INPLACE>
+__global__ void prGroupKernel(PrArgs a, uint32_t lg, uint32_t splitMin) {
     const GbPrControl* c = a.ctl;
     if (ldvi(&c->stopped)) return;
     const int cur = c->cur;
@@ -372,56 +503,72 @@ __global__ void prPullKernel(PrArgs a) {
     const bool withDelta = !INPLACE && c->withDelta;
     const float* contrib = INPLACE ? a.contrib[0] : a.contrib[cur];
     IterAcc acc;
-    auto store = [&](uint32_t v, float s) {
-        const float val = prValue(a, s, dang);
-        if (INPLACE) {
-            a.r[cur ^ 1][v] = val;
-            const uint32_t od = a.outdeg[v];
-            a.contrib[0][v] = od ? val / (float)od : 0.0f;
-        } else {
-            storeJacobi(a, cur, withDelta, v, val, acc);
-        }
+    auto store = [&](uint32_t v, float s, uint32_t od, float old) {
+        storePulled<INPLACE>(a, cur, withDelta, v, prValue(a, s, dang), od, old, acc);
     };
-    const uint64_t gthreads = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (MODE == 0) {
-        for (uint64_t v = gtid; v < a.n; v += gthreads)
-            store((uint32_t)v, gatherSerial<INPLACE>(a.ci, contrib, a.rp[v], a.rp[v + 1]));
-    } else if (MODE == 1) {
-        const uint64_t nwarps = gthreads >> 5;
-        for (uint64_t v = gtid >> 5; v < a.n; v += nwarps) {
-            float s = gatherStrided<32, INPLACE>(a.ci, contrib, a.rp[v], a.rp[v + 1], laneId());
-            s = warpSum(s);
-            if (laneId() == 0) store((uint32_t)v, s);
-        }
-    } else {
-        // degree-adaptive over the hub-first relabeled graph: task space =
-        // chunks of split vertices, then warp tasks of each degree class
-        uint64_t total = a.nChunks;
-        for (int b = 0; b < a.nBins; ++b) total += ((uint64_t)(a.binHi[b] - a.binLo[b]) * a.binG[b] + 31) / 32;
-        const uint64_t nwarps = gthreads >> 5;
-        const unsigned lane = laneId();
-        for (uint64_t t = gtid >> 5; t < total; t += nwarps) {  // warp-uniform
-            if (t < a.nChunks) {
-                chunkTask<INPLACE>(a, (uint32_t)t, contrib, store);
-                continue;
-            }
-            uint64_t tb = t - a.nChunks;
-            int b = 0;
-            for (; b < a.nBins; ++b) {
-                const uint64_t nt = ((uint64_t)(a.binHi[b] - a.binLo[b]) * a.binG[b] + 31) / 32;
-                if (tb < nt) break;
-                tb -= nt;
-            }
-            const unsigned G = a.binG[b];
-            const uint32_t v = a.binLo[b] + (uint32_t)tb * (32 / G) + lane / G;
-            const bool active = v < a.binHi[b];
-            float s = active ? gatherGroup<INPLACE>(a.ci, contrib, a.rp[v], a.rp[v + 1], lane & (G - 1), G) : 0.f;
-            for (unsigned o = G >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-            if (active && (lane & (G - 1)) == 0) store(v, s);
-        }
+    const unsigned lane = laneId(), G = 1u << lg, sub = lane & (G - 1);
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint64_t total = a.nChunks + (((uint64_t)a.n << lg) + 31) / 32;
+    uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    for (; t < a.nChunks; t += nwarps) {  // warp-uniform
+        const uint4 h = a.chunks[t];
+        const uint32_t first = a.hubFirst[2 * h.w], cnt = a.hubFirst[2 * h.w + 1];
+        const Kahan k = gatherKahan<INPLACE>(a.ci, contrib, h.y, h.z, lane, 32);
+        FF f;
+        if (splitSum(a, (uint32_t)t, h.w, first, cnt, k, f) && lane == 0)
+            store(h.x, f.hi + f.lo, a.outdeg[h.x], withDelta ? a.r[cur][h.x] : 0.f);
+    }
+    for (; t < total; t += nwarps) {
+        const uint64_t v = (t - a.nChunks) * (32u >> lg) + (lane >> lg);
+        const bool active = v < a.n;
+        const uint32_t b = active ? a.rp[v] : 0u, e = active ? a.rp[v + 1] : 0u;
+        const bool mine = active && e - b < splitMin, lead = mine && sub == 0;
+        const uint32_t od = lead ? a.outdeg[v] : 0u;
+        const float old = lead && withDelta ? a.r[cur][v] : 0.f;
+        float s = mine ? gatherGroup<INPLACE>(a.ci, contrib, b, e, sub, G) : 0.f;
+        for (unsigned o = G >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+        if (lead) store((uint32_t)v, s, od, old);
     }
     if (!INPLACE) finishBlock<0>(a, acc);
+}
+
+// In-place sweep of one colour set (relabeled, degree classes as id ranges):
+// chunks of its split vertices, then warp tasks of each class.
+__global__ void gsSetKernel(PrArgs a) {
+    const GbPrControl* c = a.ctl;
+    if (ldvi(&c->stopped)) return;
+    const int cur = c->cur;
+    const float dang = c->dangHi + c->dangLo;
+    const float* contrib = a.contrib[0];
+    auto store = [&](uint32_t v, float s) {
+        const float val = prValue(a, s, dang);
+        a.r[cur ^ 1][v] = val;
+        const uint32_t od = a.outdeg[v];
+        a.contrib[0][v] = od ? val / (float)od : 0.0f;
+    };
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const unsigned lane = laneId();
+    uint64_t total = a.nChunks;
+    for (int b = 0; b < a.nBins; ++b) total += ((uint64_t)(a.binHi[b] - a.binLo[b]) * a.binG[b] + 31) / 32;
+    for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < total; t += nwarps) {  // warp-uniform
+        if (t < a.nChunks) {
+            chunkTask<true>(a, (uint32_t)t, contrib, store);
+            continue;
+        }
+        uint64_t tb = t - a.nChunks;
+        int b = 0;
+        for (; b < a.nBins; ++b) {
+            const uint64_t nt = ((uint64_t)(a.binHi[b] - a.binLo[b]) * a.binG[b] + 31) / 32;
+            if (tb < nt) break;
+            tb -= nt;
+        }
+        const unsigned G = a.binG[b];
+        const uint32_t v = a.binLo[b] + (uint32_t)tb * (32 / G) + lane / G;
+        const bool active = v < a.binHi[b];
+        float s = active ? gatherGroup<true>(a.ci, contrib, a.rp[v], a.rp[v + 1], lane & (G - 1), G) : 0.f;
+        for (unsigned o = G >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+        if (active && (lane & (G - 1)) == 0) store(v, s);
+    }
 }
 
 // In-place sweep over a vertex list, warp per vertex (natural GS order; the
@@ -948,13 +1095,19 @@ static void enqueueIteration(gb_pr& h, int v, const gb_pr_options& o, PrArgs& a,
     const uint32_t tg = o.tg;
     cudaStream_t s = h.stream.s;
     const uint32_t gN = gridFor(h.n, 256);
-    auto pullGrid = [&](int mode) {
-        if (mode == 0) return residentGrid(prPullKernel<0, false>, h.n, tg);
-        if (mode == 1) return residentGrid(prPullKernel<1, false>, h.n * 32, tg);
-        uint64_t tasks = h.nChunks;  // adaptive: warp tasks
-        for (int b = 0; b < h.nBins; ++b) tasks += ((uint64_t)(h.binHi[b] - h.binLo[b]) * h.binG[b] + 31) / 32;
-        return residentGrid(prPullKernel<2, false>, tasks * 32, tg);
+    const uint64_t adaptiveWork = ((uint64_t)h.nChunks + h.nRunTasks) * 32;
+    // scalar / vector: the arguments with the variant's split lists, and its work in threads
+    const gb_pr::PrSplit& sp = h.split[v == GB_PR_PULL_VECTOR ? 1 : 0];
+    auto grouped = [&](const PrArgs& from) {
+        PrArgs g = from;
+        g.chunks = sp.chunks.get();
+        g.hubFirst = sp.first.get();
+        g.hubDone = sp.done.get();
+        g.hubPart = sp.part.get();
+        g.nChunks = sp.nChunks;
+        return g;
     };
+    const uint64_t groupWork = (uint64_t)sp.nChunks * 32 + ((uint64_t)h.n << sp.lg);
     const bool inplace = v == GB_PR_PULL_GS || (o.inplace && v != GB_PR_PUSH && v != GB_PR_PULL_F64);
     if (v == GB_PR_PUSH) {
         prPushKernel<<<gridFor(h.n, tg), tg, 0, s>>>(a, h.rowOut.get(), h.colOut.get());
@@ -968,9 +1121,10 @@ static void enqueueIteration(gb_pr& h, int v, const gb_pr_options& o, PrArgs& a,
                                                             (uint64_t)std::max(h.nRowBlocks, h.nBlkHubs)});
         prBlockedKernel<<<std::max(grid, 1u), kBlkThreads, blkSmemBytes(), s>>>(a, b);
     } else if (!inplace) {
-        if (v == GB_PR_PULL_SCALAR) prPullKernel<0, false><<<pullGrid(0), tg, 0, s>>>(a);
-        else if (v == GB_PR_PULL_VECTOR) prPullKernel<1, false><<<pullGrid(1), tg, 0, s>>>(a);
-        else prPullKernel<2, false><<<pullGrid(2), tg, 0, s>>>(ag);
+        if (v == GB_PR_PULL_SCALAR || v == GB_PR_PULL_VECTOR)
+            prGroupKernel<false><<<residentGrid(prGroupKernel<false>, groupWork, tg), tg, 0, s>>>(grouped(a), sp.lg, sp.splitMin);
+        else
+            prAdaptiveKernel<false><<<residentGrid(prAdaptiveKernel<false>, adaptiveWork, tg), tg, 0, s>>>(ag, h.vecA.get(), h.runsA.get(), h.nRuns, h.nRunTasks);
     } else {
         const bool colored = v == GB_PR_PULL_GS && h.gsColored;
         PrArgs& w = (colored || v == GB_PR_PULL_ADAPTIVE) ? ag : a;
@@ -995,7 +1149,7 @@ static void enqueueIteration(gb_pr& h, int v, const gb_pr_options& o, PrArgs& a,
                         ws.binG[b] = L.g[b];
                         if (b < L.nBins) tasks += ((uint64_t)(L.hi[b] - L.lo[b]) * L.g[b] + 31) / 32;
                     }
-                    prPullKernel<2, true><<<residentGrid(prPullKernel<2, true>, tasks * 32, tg), tg, 0, s>>>(ws);
+                    gsSetKernel<<<residentGrid(gsSetKernel, tasks * 32, tg), tg, 0, s>>>(ws);
                 }
             } else {
                 PrArgs wa = w;
@@ -1028,12 +1182,10 @@ static void enqueueIteration(gb_pr& h, int v, const gb_pr_options& o, PrArgs& a,
                     gsSweepListKernel<<<gridFor((uint64_t)h.gsNatB * 32, tg), tg, 0, s>>>(wa, h.gsNatB);
                 }
             }
-        } else if (v == GB_PR_PULL_SCALAR) {
-            prPullKernel<0, true><<<pullGrid(0), tg, 0, s>>>(w);
-        } else if (v == GB_PR_PULL_VECTOR) {
-            prPullKernel<1, true><<<pullGrid(1), tg, 0, s>>>(w);
+        } else if (v == GB_PR_PULL_SCALAR || v == GB_PR_PULL_VECTOR) {
+            prGroupKernel<true><<<residentGrid(prGroupKernel<true>, groupWork, tg), tg, 0, s>>>(grouped(w), sp.lg, sp.splitMin);
         } else {
-            prPullKernel<2, true><<<pullGrid(2), tg, 0, s>>>(w);
+            prAdaptiveKernel<true><<<residentGrid(prAdaptiveKernel<true>, adaptiveWork, tg), tg, 0, s>>>(w, h.vecA.get(), h.runsA.get(), h.nRuns, h.nRunTasks);
         }
         prSumKernel<<<gN, 256, 0, s>>>(w);
         prScaleKernel<<<gN, 256, 0, s>>>(w);
@@ -1049,6 +1201,7 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
     if (v != GB_PR_PUSH && !hasIn) throw Error(GB_ERR_ARG, "pull variants need the in-CSR");
     if (o.iters < 0) throw Error(GB_ERR_ARG, "iters must be >= 0");
     if (v == GB_PR_PULL_ADAPTIVE) prepareAdaptive(o.small_max, o.large_min);
+    if (v == GB_PR_PULL_SCALAR || v == GB_PR_PULL_VECTOR) prepareSplit(v == GB_PR_PULL_VECTOR);
     if (v == GB_PR_PULL_GS && !gsReady) prepareGS(2);
     if (v == GB_PR_PULL_BLOCKED) {
         prepareBlocked();
@@ -1096,20 +1249,12 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
     a.invN64 = 1.0 / (double)n;
     PrArgs ag = a;
     if (v == GB_PR_PULL_ADAPTIVE) {  // hub-first relabeled layout
-        ag.rp = rowA.get();
-        ag.ci = colA.get();
         ag.outdeg = outdegA.get();
         ag.chunks = hubChunks.get();
         ag.hubFirst = hubFirst.get();
         ag.hubDone = hubDone.get();
         ag.hubPart = hubPart.get();
         ag.nChunks = nChunks;
-        ag.nBins = nBins;
-        for (int b = 0; b < 8; ++b) {
-            ag.binLo[b] = binLo[b];
-            ag.binHi[b] = binHi[b];
-            ag.binG[b] = binG[b];
-        }
     } else if (gsColored && gsReady) {
         ag.rp = rowGS.get();
         ag.ci = colGS.get();

@@ -54,6 +54,15 @@ constexpr int kBlkConsumerWarps = kBlkThreads / 32 - 1;
 constexpr uint32_t kBlkChunk = kBlkConsumerWarps * 32;  // one 16-byte word per consumer thread
 constexpr uint32_t kBlkHub = 4096;  // rows with this many in-edges are summed apart, one block each
 
+// A run of the adaptive layout: vertices [v0, vEnd), all with lists of `vecs`
+// vectors, handled by groups of 1 << lg lanes.  Lists follow one another from
+// vector e0 on; `inter`: in blocks of 32 lists with vector k of the 32 lists
+// side by side, so a lane per list reads whole lines.  The run's warp tasks
+// (32 >> lg vertices each) are [task0, next run's task0).
+struct GbPrRun {
+    uint32_t task0, v0, vEnd, e0, vecs, lg, inter, pad;
+};
+
 struct gb_pr {
     uint64_t n = 0, mOut = 0, mIn = 0;
     bool hasOut = false, hasIn = false;
@@ -67,18 +76,28 @@ struct gb_pr {
     gb::EventPair ev;
     std::vector<uint32_t> hostRowIn, hostColIn, hostOutdeg;
 
-    // adaptive pull: hub-first relabeled in-CSR (new id = rank by descending
-    // in-degree), so every degree bin is a contiguous id range
-    gb::DevBuf<uint32_t> rowA, colA, outdegA;
-    gb::DevBuf<uint4> hubChunks;     // (vertex, start, end, hub index) per chunk
+    // adaptive pull (pr_layout.cu): vertices relabeled by descending in-degree
+    // (new id = rank), lists sorted and padded to whole 16-byte vectors, and a
+    // run per padded length, so a list's place follows from its id
+    gb::DevBuf<uint4> vecA;          // the lists
+    gb::DevBuf<uint32_t> outdegA;    // by new id
+    gb::DevBuf<uint32_t> permADev;   // old id -> new id
+    gb::DevBuf<GbPrRun> runsA;
+    uint32_t nRuns = 0, nRunTasks = 0;
+    gb::DevBuf<uint4> hubChunks;     // split lists: (vertex, first vector, end vector, hub index) per chunk
     gb::DevBuf<uint32_t> hubFirst;   // per hub: first chunk | chunk count
     gb::DevBuf<unsigned> hubDone;    // per hub: chunks finished (reset by the last)
-    gb::DevBuf<float> hubPart;       // per chunk: Kahan sum, compensation
-    std::vector<uint32_t> permA;     // old id -> new id
-    gb::DevBuf<uint32_t> permADev;
+    gb::DevBuf<float> hubPart;       // per chunk: its sum (float-float)
     uint32_t nHubs = 0, nChunks = 0;
-    uint32_t binLo[8] = {0}, binHi[8] = {0}, binG[8] = {0};  // group-size ranges (G = 1..32)
-    int nBins = 0;
+    // scalar and vector pulls: lanes per list (log2) and the split lists
+    struct PrSplit {
+        gb::DevBuf<uint4> chunks;  // (vertex, start, end, hub index)
+        gb::DevBuf<uint32_t> first;
+        gb::DevBuf<unsigned> done;
+        gb::DevBuf<float> part;
+        uint32_t nChunks = 0, lg = 0, splitMin = 0;
+        bool ready = false;
+    } split[2];
     uint32_t binSmall = 0, binLarge = 0;
     bool binsReady = false;
     // Gauss-Seidel natural order: vertices of in-degree >= kGsHubMin are split
@@ -126,6 +145,7 @@ struct gb_pr {
     void invalidateGraphs();
     void prepareAdaptive(uint32_t smallMax, uint32_t largeMin);
     void prepareGS(uint32_t pairMaxOutdeg);
+    void prepareSplit(bool vector);
     void prepareBlocked();
     gb_pr_result run(int variant, const gb_pr_options& o);
     void ranks(float* out);

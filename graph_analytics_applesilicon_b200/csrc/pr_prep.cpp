@@ -1,6 +1,6 @@
-// pr_prep.cpp -- host preprocessing for PageRank: in-degree bins of the
-// adaptive pull (GpuPageRank::prepareAdaptive, src/metal/pagerank_gpu.mm:70-86)
-// and the Gauss-Seidel update order (prepareGS, :88-192).
+// pr_prep.cpp -- host preprocessing for PageRank: the Gauss-Seidel update order
+// (GpuPageRank::prepareGS, src/metal/pagerank_gpu.mm:88-192) and the blocked
+// pull's tiles.
 #include <omp.h>
 
 #include <algorithm>
@@ -37,82 +37,6 @@ void upload(gb::DevBuf<T>& buf, const std::vector<T>& v) {
 }
 
 }  // namespace
-
-// Degree-adaptive pull layout.  Vertices are relabeled by descending in-degree
-// (stable), so each degree class is a contiguous id range and the hottest
-// contributions (the hubs') sit together at the front of the array.  Classes:
-//   in-degree >= large_min            split into warp chunks of 4096 edges;
-//   small_max <= in-degree < large_min a group of G = clamp(pow2ceil(deg/4), 2, 32)
-//                                      lanes per vertex (more vertices in flight
-//                                      per warp for short lists);
-//   in-degree < small_max             one thread per vertex.
-// (The reference's three bins, src/metal/pagerank_gpu.mm:70-86, with the
-// medium bin refined by list length and the large bin split across warps.)
-void gb_pr::prepareAdaptive(uint32_t smallMax, uint32_t largeMin) {
-    if (binsReady && binSmall == smallMax && binLarge == largeMin) return;
-    if (!hasIn) throw Error(GB_ERR_ARG, "gpu_pull_adaptive needs the in-CSR");
-    const uint32_t* rp = hostRowIn.data();
-    const uint32_t* ci = hostColIn.data();
-    auto deg = [&](uint32_t v) { return rp[v + 1] - rp[v]; };
-    std::vector<uint32_t> order(n);
-    for (uint32_t v = 0; v < n; ++v) order[v] = v;
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return deg(a) > deg(b); });
-    permA.assign(n, 0);
-    for (uint32_t i = 0; i < n; ++i) permA[order[i]] = i;
-    std::vector<uint32_t> row(n + 1, 0), od(n);
-    for (uint32_t i = 0; i < n; ++i) row[i + 1] = row[i] + deg(order[i]);
-    std::vector<uint32_t> col((size_t)row[n] + 4, 0);
-#pragma omp parallel for schedule(dynamic, 1024)
-    for (int64_t i = 0; i < (int64_t)n; ++i) {
-        const uint32_t v = order[i];
-        od[i] = hostOutdeg[v];
-        uint32_t* out = col.data() + row[i];
-        for (uint32_t e = rp[v]; e < rp[v + 1]; ++e) *out++ = permA[ci[e]];
-        std::sort(col.data() + row[i], out);
-    }
-    auto groupOf = [&](uint32_t d) -> uint32_t {  // 0 = split
-        if (d >= largeMin) return 0;
-        if (d < smallMax) return 1;
-        uint32_t g = 2;
-        while (g < 32 && 4 * g < d) g *= 2;
-        return g;
-    };
-    std::vector<uint32_t> hubs;
-    nBins = 0;
-    for (uint32_t i = 0; i < n;) {
-        const uint32_t g = groupOf(row[i + 1] - row[i]);
-        uint32_t j = i;
-        while (j < n && groupOf(row[j + 1] - row[j]) == g) ++j;
-        if (g == 0) {
-            for (uint32_t v = i; v < j; ++v) hubs.push_back(v);
-        } else {
-            if (nBins >= 8) throw Error(GB_ERR_STATE, "adaptive layout: degree classes are not contiguous");
-            binLo[nBins] = i;
-            binHi[nBins] = j;
-            binG[nBins] = g;
-            ++nBins;
-        }
-        i = j;
-    }
-    std::vector<uint4> chunks;
-    std::vector<uint32_t> first;
-    buildChunks(hubs, row.data(), chunks, first);
-    nHubs = (uint32_t)hubs.size();
-    nChunks = (uint32_t)chunks.size();
-    invalidateGraphs();
-    upload(rowA, row);
-    upload(colA, col);
-    upload(outdegA, od);
-    upload(permADev, permA);
-    upload(hubChunks, chunks);
-    upload(hubFirst, first);
-    hubDone.ensure(nHubs + 1);
-    GB_CUDA(cudaMemset(hubDone.get(), 0, (nHubs + 1) * sizeof(unsigned)));
-    hubPart.ensure(2 * (size_t)nChunks + 2);
-    binSmall = smallMax;
-    binLarge = largeMin;
-    binsReady = true;
-}
 
 // Update order of the in-place sweep.  A GPU sweep updates tens of thousands
 // of vertices concurrently, so an in-place update helps only where a vertex's

@@ -562,6 +562,18 @@ __global__ void rowRankDecodeKernel(const unsigned long long* keys, uint64_t m, 
 
 }  // namespace
 
+void degreeRank(const uint32_t* rp, uint64_t n, uint32_t* order, uint32_t* rank, ScanScratch& sc, cudaStream_t st) {
+    const int b = keyBits(n);
+    DevBuf<unsigned long long> keys, tmp;
+    keys.ensure(n);
+    degreeKeysKernel<<<prepGrid(n, 256), 256, 0, st>>>(rp, n, b, true, keys.get());
+    GB_LAUNCH_CHECK();
+    radixSortKeys(keys, tmp, n, 32 + b, sc, st);
+    keysToOrderKernel<<<prepGrid(n, 256), 256, 0, st>>>(keys.get(), n, b, order, rank, nullptr);
+    GB_LAUNCH_CHECK();
+    GB_CUDA(cudaStreamSynchronize(st));
+}
+
 void hubFirstAdjacency(const uint32_t* rp, uint32_t* ci, uint64_t n, uint64_t m, cudaStream_t st) {
     if (m < 2) return;
     const int b = keyBits(n);
