@@ -241,19 +241,37 @@ class Graph:
                 and np.array_equal(self.row_ptr, o.row_ptr) and np.array_equal(self.col_idx[: self.m], o.col_idx[: o.m]))
 
 
-def _take(c: _Csr) -> Graph:
-    n, m = int(c.n), int(c.m)
-    rp = np.ctypeslib.as_array(c.row_ptr, shape=(n + 1,)).copy()
-    ci = np.ctypeslib.as_array(c.col_idx, shape=(m,)).copy() if m else np.zeros(0, np.uint32)
-    g = Graph(n, m, int(c.flags), rp, ci)
-    lib().gb_csr_free(C.byref(c))
-    return g
+class _Array:
+    """One array the library allocated, as the owner behind a numpy array: it is
+    released (gb_csr_free) when the last numpy view of it is gone."""
+
+    def __init__(self, ptr, count):
+        self._csr = _Csr(row_ptr=ptr)
+        self._free = lib().gb_csr_free
+        self.__array_interface__ = {"shape": (count,), "typestr": "<u4", "version": 3,
+                                    "data": (C.cast(ptr, C.c_void_p).value, False)}
+
+    def __del__(self):
+        self._free(C.byref(self._csr))
 
 
-def _make(fn, *args) -> Graph:
+def _take(c: _Csr, copy: bool = False) -> Graph:
+    """The C graph's arrays as a Graph, without copying them (copy: page-locked
+    arrays, which a Graph should not keep)."""
+    n, m, flags = int(c.n), int(c.m), int(c.flags)
+    if copy or not m:
+        rp = np.ctypeslib.as_array(c.row_ptr, shape=(n + 1,)).copy()
+        ci = np.ctypeslib.as_array(c.col_idx, shape=(m,)).copy() if m else np.zeros(0, np.uint32)
+        lib().gb_csr_free(C.byref(c))
+    else:
+        rp, ci = np.asarray(_Array(c.row_ptr, n + 1)), np.asarray(_Array(c.col_idx, m))
+    return Graph(n, m, flags, rp, ci)
+
+
+def _make(fn, *args, copy: bool = False) -> Graph:
     out = _Csr()
     check(fn(*args, C.byref(out)))
-    return _take(out)
+    return _take(out, copy)
 
 
 class gen:
@@ -400,7 +418,7 @@ def load(path: str) -> Graph:
 def load_pinned(path: str) -> Graph:
     """graph::load into page-locked memory (returned here as numpy copies; C
     callers keep the pinned arrays and upload them at full PCIe speed)."""
-    return _make(lib().gb_csr_load_pinned, path.encode())
+    return _make(lib().gb_csr_load_pinned, path.encode(), copy=True)
 
 
 def save(g: Graph, path: str) -> None:

@@ -209,25 +209,28 @@ void copyDepthsToHost(gb_bfs* h, const uint32_t* d, uint64_t count, uint32_t* ou
 }
 
 void StagedCopy::run(const void* dev, size_t bytes, void* out, cudaStream_t st) {
+    constexpr size_t kChunk = 1u << 19;
     const size_t chunks = (bytes + kChunk - 1) / kChunk;
-    ring_.ensure(std::min(bytes, kSlots * kChunk));
+    hold_.ensure(1);
+    HostPinned<uint8_t> ring;
+    ring.ensure(std::min(bytes, kSlots * kChunk));
     for (cudaEvent_t& e : ev_)
         if (!e) GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     const uint8_t* src = static_cast<const uint8_t*>(dev);
     uint8_t* dst = static_cast<uint8_t*>(out);
     auto length = [&](size_t c) { return std::min(kChunk, bytes - c * kChunk); };
     auto enqueue = [&](size_t c) {
-        GB_CUDA(cudaMemcpyAsync(ring_.p + c % kSlots * kChunk, src + c * kChunk, length(c), cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaMemcpyAsync(ring.p + c % kSlots * kChunk, src + c * kChunk, length(c), cudaMemcpyDeviceToHost, st));
         GB_CUDA(cudaEventRecord(ev_[c % kSlots], st));
     };
     for (size_t c = 0; c < std::min<size_t>(chunks, kSlots); ++c) enqueue(c);
-    const int threads = hostThreads(4);
+    const int threads = hostThreads(8);
     for (size_t c = 0; c < chunks; ++c) {
         GB_CUDA(cudaEventSynchronize(ev_[c % kSlots]));
-        const uint8_t* from = ring_.p + c % kSlots * kChunk;
+        const uint8_t* from = ring.p + c % kSlots * kChunk;
         uint8_t* to = dst + c * kChunk;
         const size_t len = length(c);
-        constexpr size_t kPiece = 1 << 16;
+        constexpr size_t kPiece = 1 << 15;
         const int pieces = (int)((len + kPiece - 1) / kPiece);
 #pragma omp parallel for num_threads(threads) schedule(static) if (pieces > 3)
         for (int p = 0; p < pieces; ++p)

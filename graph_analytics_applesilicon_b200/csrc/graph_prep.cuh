@@ -12,8 +12,8 @@ namespace gb {
 uint32_t prepGrid(uint64_t work, uint32_t threads);
 // Bits of the largest id below n (at least 1): the column field of a key.
 int keyBits(uint64_t n);
-// Sorts N keys whose used bits are [0, bits) in place (a holds the result;
-// tmp is scratch of N keys).  N < 2^32.
+// Sorts N keys whose used bits are [0, bits): a holds the result, tmp is scratch
+// of N keys (the two buffers may change places).  N < 2^32.
 // countsScratch (optional) is reused for the digit histograms across calls.
 void radixSortKeys(DevBuf<unsigned long long>& a, DevBuf<unsigned long long>& tmp, uint64_t N, int bits,
                    ScanScratch& sc, cudaStream_t st, DevBuf<uint32_t>* countsScratch = nullptr);
@@ -24,9 +24,9 @@ void permutedKeys(const uint32_t* rp, const uint32_t* ci, uint64_t n, uint64_t m
 // inverse (either may be null).
 void degreeRank(const uint32_t* rp, uint64_t n, uint32_t* order, uint32_t* rank, ScanScratch& sc, cudaStream_t st);
 // Sorted keys -> host CSR in *out (n rows, b column bits), dropping repeated
-// keys (unique) and self-loops (dropSelf); out->flags = flags.
-void keysToCsr(DevBuf<unsigned long long>& keys, uint64_t N, uint64_t n, int b, bool unique, bool dropSelf,
-               uint32_t flags, ScanScratch& sc, cudaStream_t st, gb_csr* out);
+// keys (unique) and self-loops (dropSelf); out->flags = flags.  tmp is scratch.
+void keysToCsr(DevBuf<unsigned long long>& keys, DevBuf<unsigned long long>& tmp, uint64_t N, uint64_t n, int b,
+               bool unique, bool dropSelf, uint32_t flags, ScanScratch& sc, cudaStream_t st, gb_csr* out);
 
 // Uploads a host CSR and checks it on the device (row_ptr from 0 to m and
 // non-decreasing, every column below n); throws GB_ERR_ARG otherwise.

@@ -20,9 +20,8 @@ public:
     void run(const void* dev, size_t bytes, void* out, cudaStream_t st);
 
 private:
-    static constexpr int kSlots = 4;
-    static constexpr size_t kChunk = 1 << 18;
-    HostPinned<uint8_t> ring_;
+    static constexpr int kSlots = 2;
+    HostPinned<uint8_t> hold_;  // keeps the pool while this object lives; the ring itself is taken for a call
     cudaEvent_t ev_[kSlots] = {};
 };
 

@@ -440,7 +440,7 @@ void snapToCsr(const std::string& path, bool directed, uint64_t chunk, gb_csr* o
         radixSortKeys(keys, tmp, total, 2 * b, sc, st.s);
     }
     constexpr uint32_t kFlagDirected = 1u, kFlagSorted = 2u, kFlagDedup = 4u;
-    keysToCsr(keys, total, n, b, true, true, (directed ? kFlagDirected : 0u) | kFlagSorted | kFlagDedup, sc, st.s,
+    keysToCsr(keys, tmp, total, n, b, true, true, (directed ? kFlagDirected : 0u) | kFlagSorted | kFlagDedup, sc, st.s,
               out);
     if (stats) {
         stats->lines = edges;
