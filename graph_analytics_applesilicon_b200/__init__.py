@@ -247,12 +247,12 @@ class _Array:
 
     def __init__(self, ptr, count):
         self._csr = _Csr(row_ptr=ptr)
-        self._free = lib().gb_csr_free
+        self._free, self._ref = lib().gb_csr_free, C.byref(self._csr)  # both may outlive this module's globals
         self.__array_interface__ = {"shape": (count,), "typestr": "<u4", "version": 3,
                                     "data": (C.cast(ptr, C.c_void_p).value, False)}
 
     def __del__(self):
-        self._free(C.byref(self._csr))
+        self._free(self._ref)
 
 
 def _take(c: _Csr, copy: bool = False) -> Graph:

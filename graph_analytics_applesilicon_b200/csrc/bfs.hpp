@@ -95,6 +95,7 @@ struct gb_bfs {
     gb::DevBuf<uint32_t> pIso;           // degree-0 vertices, a bit each (visited from the start)
     bool pIsoReady = false;
     gb::DevBuf<GbPCounters> pctr;        // [3]
+    gb::DevBuf<unsigned long long> psolo;  // [2][8] what a stretch of single-block levels arrived at
     gb::DevBuf<unsigned> pctl;           // [0] barrier, [1] error, [2] levels, [3] flags
     gb::HostPinned<unsigned> pctlHost;
     gb::DevBuf<gb_level> ptrace;
@@ -106,6 +107,7 @@ struct gb_bfs {
         gb::DevBuf<uint32_t> q[2][3], hub[2][2], bm[3], visited;
         gb::DevBuf<unsigned long long> hubOff[2];
         gb::DevBuf<GbPCounters> ctr;
+        gb::DevBuf<unsigned long long> solo;
         gb::DevBuf<gb_level> trace;
         gb::DevBuf<double> state;
     };

@@ -994,7 +994,10 @@ void gb_bfs::runBatch(const uint32_t* src, int k, const gb_bfs_options& o, std::
     GB_CUDA(cudaStreamSynchronize(stream.s));
     lastGpuMs = ev.ms();
     lastLevels = ctl[2];
-    if (ctl[1]) throw Error(GB_ERR_TIMEOUT, "batched BFS: grid barrier wait exceeded its spin limit");
+    if (ctl[1]) {
+        GB_CUDA(cudaMemsetAsync(pctl.get(), 0, 4 * sizeof(unsigned), stream.s));  // shared with single-source runs
+        throw Error(GB_ERR_TIMEOUT, "batched BFS: grid barrier wait exceeded its spin limit");
+    }
     if (tr) {
         const uint32_t kk = std::min<uint32_t>(ctl[2], kTraceCap);
         std::vector<gb_level> t(kk);

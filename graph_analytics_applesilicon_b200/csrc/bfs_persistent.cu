@@ -9,8 +9,8 @@
 // learned selector, or a forced strategy) without a host round trip.
 //
 // Device state (n vertices, W = ceil(n/32) words):
-//   dist u32[n]; visited bitmap u32[W]; frontier bitmaps bm[3] u32[W]
-//   (level L reads bm[L%3], writes bm[(L+1)%3], clears bm[(L+2)%3]);
+//   dist u32[n]; visited bitmap u32[W]; frontier bitmaps bm[3] u32[W] in turn
+//   (a level reads bm[b], writes bm[b+1], clears bm[b+2], then b moves on by one);
 //   frontier queue q[2] = (vertex, adjacency start, degree) u32[n] each;
 //   hub list hub[2] = (vertex, start, exclusive offset in the hubs' edge space)
 //   for vertices of degree >= hub_min, whose edges are split across blocks;
@@ -30,6 +30,21 @@ constexpr unsigned long long kHubShift = 40;
 constexpr unsigned long long kHubMask = (1ull << kHubShift) - 1;
 constexpr uint32_t kTraceCap = kTraceLevels;
 constexpr uint64_t kEnqueueEdges = 1ull << 18;  // top-down levels with this many edges build no queue
+// Frontiers of at most this many edges per thread of one block run in one block
+// (soloLevels).  A level of 4 takes 5 us there against 6.5 on the grid, one of 8
+// 10 us (road 300 x 300, rule: 2.7 ms with 2 edges per thread, 1.8 with 4).
+constexpr uint32_t kSoloEdges = 4;
+// Depth arrays up to this size are filled by the kernel and, for a run that
+// returns them, packed by it into pinned host memory; larger ones by a memset
+// before the launch and a kernel and chunked copies after it, which the
+// widening overlaps.
+constexpr uint64_t kSmallDepths = 1ull << 20;
+constexpr unsigned kNotDone = 0xFFFFFFFFu;
+// At most so many levels at a time, which bounds the other blocks' wait (about
+// 0.3 ms, some 400 polls); a caller's spin limit under kSoloSpin polls, which may
+// be set for the grid's levels of a few us, keeps every level on the grid.
+constexpr uint32_t kSoloLevels = 64;
+constexpr unsigned long long kSoloSpin = 1ull << 14;
 
 enum { S_LEVEL, S_BOTTOMUP, S_SCOUT, S_TOCHECK, S_UNEXPLORED, S_REACHED, S_QVALID, S_LAST, S_COUNT };
 
@@ -47,7 +62,11 @@ struct PArgs {
     uint32_t* visited;
     const uint32_t* iso;  // bit per vertex of degree 0, or null
     GbPCounters* ctr;
+    unsigned long long* solo;  // [2][8], see soloLevels
     unsigned* ctl;  // [0] barrier word, [1] error flag, [2] levels run
+    bool fillDist;      // the kernel sets the depths to infinity (else a memset before the launch)
+    uint8_t* packHost;  // pinned host memory for the packed depths, or null
+    unsigned* ctlHost;  // pinned: [0] levels run, [1] width of the packed depths (with packHost), [2] a wait ran out
     gb_level* trace;
     const float* sel;
     double* state;
@@ -138,6 +157,16 @@ __device__ __forceinline__ void discoverN(const PArgs& a, const bool* has, const
         appendClaimed(a, !(old[k] & (1u << (u[k] & 31))), u[k], st[k], en[k], level, cur, bmNext, nq, acc, enq);
 }
 
+constexpr int kBuWords = 4;  // bitmap words per warp and round of a bottom-up level (buLevel)
+
+// A warp's open vertices of one round: list start, word and lane; and the
+// frontier bits they add.
+struct BuRest {
+    uint32_t start[32 * kBuWords];
+    uint8_t code[32 * kBuWords];
+    uint32_t bits[kBuWords];
+};
+
 template <int NT>
 struct Smem {
     uint32_t scan[NT / 32 + 1];
@@ -151,6 +180,14 @@ struct Smem {
     int strat;
     uint32_t base;
     int ok;
+    BuRest rest[NT / 32];
+    // single-block levels: vertices found, their degrees' sum and largest
+    uint32_t soCount[3], soMost[3];
+    unsigned long long soEdges[3];
+    unsigned long long state[8];  // what block 0's levels arrived at (see soloLevels)
+    // kept by thread 0, out of every thread's registers: adjacency entries and
+    // vertices not reached yet, and the time of the last level's end (block 0)
+    unsigned long long unexplored, unreached, tPrev;
 };
 
 // Grid barrier after which every thread of the block sees counters *c in
@@ -274,10 +311,6 @@ __device__ void tdHubChunk(const PArgs& a, Smem<NT>& sm, uint64_t e0, uint64_t e
     __syncthreads();
 }
 
-// Bottom-up: warp per visited-bitmap word; each unvisited lane scans its list
-// for the first neighbour in the frontier bitmap (early exit).  The found
-// lanes form the next frontier word (__ballot_sync); the owning warp writes
-// it and the visited word with plain stores.
 // The rest of one vertex's bottom-up scan after its first entry missed: the
 // first parent in the frontier, scanning in list order from i; aligned groups
 // of 4 entries are loaded at once and their 4 frontier words fetched
@@ -316,58 +349,84 @@ __device__ __forceinline__ uint32_t buScanFrom(const PArgs& a, const uint32_t* f
 // frontier bitmap.  A warp takes kBuWords bitmap words (32 vertices each, a
 // lane per vertex) per round and issues their loads stage by stage -- visited
 // words, then row bounds, then first entries, then frontier bits -- so the
-// four dependent loads of the words overlap instead of running one word
-// after another; a vertex whose first entry is not a parent (rare once lists
-// are hub-first) continues with buScanFrom.
-#ifndef GB_BU_WORDS
-#define GB_BU_WORDS 4
-#endif
-constexpr int kBuWords = GB_BU_WORDS;
-
-__device__ void buLevel(const PArgs& a, uint32_t level, Acc& acc) {
-    const uint32_t* front = a.bm[level % 3];
-    uint32_t* next = a.bm[(level + 1) % 3];
+// four dependent loads of the words overlap.  The vertices whose first entry is
+// no parent (a quarter to a half of them at the first bottom-up level) are then
+// put together in shared memory and taken 32 at a time: word by word, few lanes
+// would still be at work in each of four chains of dependent loads (R-MAT 22's
+// first bottom-up level: 62 us word by word, 48 us so).  With 2 words a round the
+// level takes 61 us, with 6 50 us; scanning long rests by the whole warp changes
+// nothing (the longest scan there has 16 entries; 139 on Chung-Lu 1M).
+__device__ void buLevel(const PArgs& a, uint32_t level, const uint32_t* front, uint32_t* next, BuRest* rests, Acc& acc) {
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const unsigned lane = laneId();
+    BuRest& rest = rests[threadIdx.x >> 5];
     for (uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w0 < a.words;
          w0 += nwarps * kBuWords) {
         uint32_t vw[kBuWords], b[kBuWords], e[kBuWords], u[kBuWords];
-        bool need[kBuWords], found[kBuWords];
+        unsigned F[kBuWords];
 #pragma unroll
         for (int k = 0; k < kBuWords; ++k) {
             const uint64_t w = w0 + (uint64_t)k * nwarps;
             vw[k] = w < a.words ? a.visited[w] : kFull;
-            need[k] = !((vw[k] >> lane) & 1u);
-            found[k] = false;
         }
 #pragma unroll
         for (int k = 0; k < kBuWords; ++k) {
+            const bool need = !((vw[k] >> lane) & 1u);
             const uint32_t v = (uint32_t)((w0 + (uint64_t)k * nwarps) * 32 + lane);
-            b[k] = need[k] ? a.row_ptr[v] : 0u;
-            e[k] = need[k] ? a.row_ptr[v + 1] : 0u;
+            b[k] = need ? a.row_ptr[v] : 0u;
+            e[k] = need ? a.row_ptr[v + 1] : 0u;
         }
 #pragma unroll
         for (int k = 0; k < kBuWords; ++k) u[k] = b[k] < e[k] ? a.col_idx[b[k]] : 0u;
 #pragma unroll
-        for (int k = 0; k < kBuWords; ++k) {
-            if (b[k] < e[k] && ((front[u[k] >> 5] >> (u[k] & 31)) & 1u)) {
-                found[k] = true;
-                acc.exam += 1;
-            }
-        }
+        for (int k = 0; k < kBuWords; ++k) u[k] = b[k] < e[k] ? (front[u[k] >> 5] >> (u[k] & 31)) & 1u : 0u;
+        uint32_t P = 0;
 #pragma unroll
         for (int k = 0; k < kBuWords; ++k) {
-            if (need[k] && !found[k]) acc.exam += (b[k] < e[k] ? buScanFrom(a, front, b[k] + 1, e[k], found[k]) : e[k]) - b[k];
-            const unsigned F = __ballot_sync(kFull, found[k]);
-            const uint64_t w = w0 + (uint64_t)k * nwarps;
-            if (found[k]) {
-                a.dist[w * 32 + lane] = level + 1;
+            const bool found = u[k] != 0, open = !found && b[k] + 1 < e[k];
+            F[k] = __ballot_sync(kFull, found);
+            const unsigned m = __ballot_sync(kFull, open);
+            if (open) {
+                const uint32_t p = P + __popc(m & lanemaskLt());
+                rest.start[p] = b[k];
+                rest.code[p] = (uint8_t)(32 * k + lane);
+            } else if (b[k] < e[k]) {
+                acc.exam += 1;
+            }
+            P += __popc(m);
+            if (found) {
+                a.dist[(w0 + (uint64_t)k * nwarps) * 32 + lane] = level + 1;
                 acc.deg += e[k] - b[k];
                 acc.found++;
             }
-            if (lane == 0 && F) {
-                next[w] = F;
-                a.visited[w] = vw[k] | F;
+        }
+        if (P) {  // warp-uniform
+            if (lane < kBuWords) rest.bits[lane] = 0;
+            __syncwarp();
+            for (uint32_t t = lane; t < P; t += 32) {
+                const uint32_t st = rest.start[t], code = rest.code[t];
+                const uint64_t v = (w0 + (uint64_t)(code >> 5) * nwarps) * 32 + (code & 31);
+                const uint32_t en = a.row_ptr[v + 1];
+                bool found = false;
+                acc.exam += buScanFrom(a, front, st + 1, en, found) - st;
+                if (found) {
+                    a.dist[v] = level + 1;
+                    acc.deg += en - st;
+                    acc.found++;
+                    atomicOr(&rest.bits[code >> 5], 1u << (code & 31));
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < kBuWords; ++k) F[k] |= rest.bits[k];
+            __syncwarp();  // the next round overwrites them
+        }
+#pragma unroll
+        for (int k = 0; k < kBuWords; ++k) {
+            const uint64_t w = w0 + (uint64_t)k * nwarps;
+            if (lane == 0 && F[k]) {
+                next[w] = F[k];
+                a.visited[w] = vw[k] | F[k];
             }
         }
     }
@@ -377,8 +436,7 @@ __device__ void buLevel(const PArgs& a, uint32_t level, Acc& acc) {
 // next level runs top-down).  Per block-round of NT words: per-thread counts,
 // a block scan, one atomic for the block's queue range.
 template <int NT>
-__device__ void bitmapToQueue(const PArgs& a, Smem<NT>& sm, uint32_t level, GbPCounters* prev) {
-    const uint32_t* bm = a.bm[level % 3];
+__device__ void bitmapToQueue(const PArgs& a, Smem<NT>& sm, uint32_t level, const uint32_t* bm, GbPCounters* prev) {
     const uint32_t qc = level & 1u;
     for (uint64_t t0 = (uint64_t)blockIdx.x * NT; t0 < a.words; t0 += (uint64_t)gridDim.x * NT) {
         const uint64_t w = t0 + threadIdx.x;
@@ -416,6 +474,203 @@ __device__ void bitmapToQueue(const PArgs& a, Smem<NT>& sm, uint32_t level, GbPC
     }
 }
 
+// barrierWithCounters for a stretch of single-block levels: every thread sees
+// what block 0 published (soloLevels) in sm.state.
+template <int NT>
+__device__ __forceinline__ bool barrierWithState(const PArgs& a, Smem<NT>& sm, const unsigned long long* from) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const bool ok = gridArriveWait(&a.ctl[0], &a.ctl[1], a.spinLimit, gridDim.x);
+        sm.ok = ok;
+        if (ok)
+            for (int i = 0; i < 8; ++i) sm.state[i] = ldv(&from[i]);
+    }
+    __syncthreads();
+    return sm.ok != 0;
+}
+
+// Top-down levels of at most kSoloEdges NT edges by one block (block 0, all its
+// threads), from `level` with the first S queue entries.  On the whole grid such
+// a level costs 6 us whatever its size: the work ticket, the queue tail's atomic,
+// the counters and the grid barrier are all round trips to L2.  Here the tail and
+// the counters are in shared memory and a block barrier ends the level: 1.7 us
+// for a few edges.  The stretch ends when the frontier is empty, has more edges or
+// a hub, turns bottom-up under the alpha/beta rule, or after kSoloLevels levels.
+// The frontier is then where the grid looks for it -- the queue of its level's parity, the hub
+// list, and the bitmap after `front`, whose own bits are cleared (`next` is all
+// zero before) -- and `out` gets (level, vertices, edges, queue entries, hubs,
+// toCheck before this level's rule, vertices found, their degrees).  The level
+// counters are not touched: other blocks may still be reading the last level's.
+template <int NT>
+__device__ void soloLevels(const PArgs& a, Smem<NT>& sm, uint32_t level, uint32_t endLevel, uint32_t S, uint64_t scout,
+                           uint64_t toCheck, uint32_t* front, uint32_t* next, unsigned long long* out) {
+    const unsigned tid = threadIdx.x, lane = laneId();
+    for (uint32_t i = tid; i < S; i += NT) front[a.qv[level & 1][i] >> 5] = 0;  // its bits are this frontier's only
+    if (tid < 3) {
+        sm.soCount[tid] = 0;
+        sm.soMost[tid] = 0;
+        sm.soEdges[tid] = 0;
+    }
+    __syncthreads();
+    uint64_t edges = scout, found = 0, degrees = 0;
+    uint32_t most = 0;
+    for (uint32_t k = 0;; ++k) {
+        const uint32_t c = level & 1u, i1 = k % 3, i2 = (k + 1) % 3;  // counters of the next frontier, and of the one after
+        if (tid == 0) {
+            sm.soCount[i2] = 0;
+            sm.soMost[i2] = 0;
+            sm.soEdges[i2] = 0;
+            if (a.trace && level < a.traceCap) {
+                gb_level r;
+                r.level = level;
+                r.direction = 'T';
+                r.device = 'G';
+                r.strategy = r.pad = (uint8_t)GB_STRAT_TD_EPT2;
+                r.frontier = S;
+                r.edges = edges;
+                r.time_ms = 0;
+                a.trace[level] = r;
+            }
+        }
+        // lanes per vertex: as many as give every vertex its lanes at once
+        const unsigned lg = S >= NT / 4 ? 2u : 31u - __clz(NT / S);
+        const unsigned G = 1u << lg, sub = tid & (G - 1);
+        unsigned long long e = 0;
+        uint32_t m = 0;
+        for (uint32_t base = (tid & ~31u) >> lg; base < S; base += NT >> lg) {  // warp-uniform
+            const uint32_t i = base + (lg < 5 ? lane >> lg : 0u);
+            const uint32_t st = i < S ? a.qs[c][i] : 0u, d = i < S ? a.qd[c][i] : 0u;
+            const uint32_t maxd = __reduce_max_sync(kFull, d);
+            for (uint32_t x = sub; x - (sub & 31u) < maxd; x += G) {  // warp-uniform
+                const bool has = x < d;
+                const uint32_t u = has ? a.col_idx[st + x] : 0u;
+                const uint32_t us = has ? a.row_ptr[u] : 0u, ue = has ? a.row_ptr[u + 1] : 0u;
+                const uint32_t old = has ? atomicOr(&a.visited[u >> 5], 1u << (u & 31)) : ~0u;
+                const bool won = !((old >> (u & 31)) & 1u);
+                const unsigned b = __ballot_sync(kFull, won);
+                if (!b) continue;
+                uint32_t p = 0;
+                if (lane == 0) p = atomicAdd(&sm.soCount[i1], (uint32_t)__popc(b));
+                p = __shfl_sync(kFull, p, 0) + __popc(b & lanemaskLt());
+                if (won) {
+                    a.dist[u] = level + 1;
+                    a.qv[c ^ 1][p] = u;
+                    a.qs[c ^ 1][p] = us;
+                    a.qd[c ^ 1][p] = ue - us;
+                    e += ue - us;
+                    m = max(m, ue - us);
+                }
+            }
+        }
+        e = warpSum(e);
+        m = __reduce_max_sync(kFull, m);
+        if (lane == 0 && e) {
+            atomicAdd(&sm.soEdges[i1], e);
+            atomicMax(&sm.soMost[i1], m);
+        }
+        __syncthreads();
+        S = sm.soCount[i1];
+        edges = sm.soEdges[i1];
+        most = sm.soMost[i1];
+        found += S;
+        degrees += edges;
+        ++level;
+        if (tid == 0) {
+            const uint64_t t = globaltimer();
+            if (a.trace && level - 1 < a.traceCap) a.trace[level - 1].time_ms = (double)(t - sm.tPrev) * 1e-6;
+            sm.tPrev = t;
+        }
+        if (S == 0 || edges > kSoloEdges * NT || most >= a.hubMin || k + 1 == kSoloLevels || level >= endLevel) break;
+        if ((double)edges > (double)toCheck / a.alpha) break;  // bottom-up next: the grid's
+        toCheck -= min(toCheck, edges);
+    }
+    const uint32_t q = level & 1u;
+    for (uint32_t i = tid; i < S; i += NT) {
+        const uint32_t v = a.qv[q][i];
+        atomicOr(&next[v >> 5], 1u << (v & 31));
+    }
+    uint32_t entries = S;
+    unsigned long long hubs = 0;
+    if (most >= a.hubMin) {  // hubs to their list (the frontier before had kSoloEdges NT edges at most, so S is no more)
+        if (tid == 0) {
+            sm.base = 0;
+            sm.acc[0] = 0;
+        }
+        constexpr int kPer = kSoloEdges;
+        uint32_t v[kPer], st[kPer], d[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const uint32_t i = tid + k * NT;
+            v[k] = i < S ? a.qv[q][i] : 0u;
+            st[k] = i < S ? a.qs[q][i] : 0u;
+            d[k] = i < S ? a.qd[q][i] : 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            if (tid + k * NT >= S) continue;
+            if (d[k] >= a.hubMin) {
+                const unsigned long long old = atomicAdd(&sm.acc[0], (1ull << kHubShift) | d[k]);
+                const uint32_t h = (uint32_t)(old >> kHubShift);
+                a.hv[q][h] = v[k];
+                a.hs[q][h] = st[k];
+                a.ho[q][h] = old & kHubMask;
+            } else {
+                const uint32_t p = atomicAdd(&sm.base, 1u);
+                a.qv[q][p] = v[k];
+                a.qs[q][p] = st[k];
+                a.qd[q][p] = d[k];
+            }
+        }
+        __syncthreads();
+        entries = sm.base;
+        hubs = sm.acc[0];
+    }
+    if (tid == 0) {
+        out[0] = level;
+        out[1] = S;
+        out[2] = edges;
+        out[3] = entries;
+        out[4] = hubs;
+        out[5] = toCheck;
+        out[6] = found;
+        out[7] = degrees;
+    }
+}
+
+// The depths packed straight into pinned host memory (at most kSmallDepths
+// vertices): the level count is known here, so the width is exact, and no
+// kernel or copy of its own follows the traversal.
+__device__ void packToHost(const PArgs& a, uint32_t level, uint64_t gtid, uint64_t gthreads) {
+    const int fmt = level < 15 ? 0 : level < 255 ? 1 : level < 65535 ? 2 : -1;  // packFormat
+    if (gtid == 0) a.ctlHost[1] = (unsigned)fmt;
+    if (fmt < 0) return;
+    const uint4* d4 = reinterpret_cast<const uint4*>(a.dist);
+    for (uint64_t g = gtid; g < (a.n + 7) / 8; g += gthreads) {
+        const uint4 x = __ldcg(d4 + 2 * g), y = 8 * g + 4 < a.n ? __ldcg(d4 + 2 * g + 1) : make_uint4(0, 0, 0, 0);
+        const uint32_t v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+        uint32_t w[4] = {0, 0, 0, 0};
+        if (fmt == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[0] |= (v[i] & 15u) << (4 * i);
+            reinterpret_cast<uint32_t*>(a.packHost)[g] = w[0];
+        } else if (fmt == 1) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i / 4] |= (v[i] & 255u) << (8 * (i % 4));
+            reinterpret_cast<uint2*>(a.packHost)[g] = make_uint2(w[0], w[1]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i / 2] |= (v[i] & 65535u) << (16 * (i % 2));
+            reinterpret_cast<uint4*>(a.packHost)[g] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+}
+
+// A block whose grid barrier's wait ran out says so to the host and ends.
+__device__ __forceinline__ void timedOut(const PArgs& a) {
+    if (threadIdx.x == 0 && a.ctlHost) a.ctlHost[2] = 1;
+}
+
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
     __shared__ Smem<NT> sm;
@@ -431,17 +686,26 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
 
     uint32_t level;
     bool bottomUp, qValid;
-    uint64_t scout, toCheck, unexplored, reached;
+    uint64_t scout, toCheck;
     int lastStrat;
     if (a.startLevel == 0) {
         // One pass writes the initial state with the source already placed
         // (depth 0, visited, frontier bit), so a single grid barrier ends the
         // prologue.  bm[2] needs no clearing: level 0 clears it.  The depth
-        // array was set to infinity by a memset before the launch (the copy
-        // engine's fill is faster than the kernel's stores).
+        // array is set to infinity here too, or, a large one, by a memset before
+        // the launch (faster from about 2^20 vertices on).
         const uint32_t src = a.source;
         const uint32_t st = a.row_ptr[src], d = a.row_ptr[src + 1] - st;
-        if (gtid == 0) a.dist[src] = 0;  // the rest is already infinity (memset before the launch)
+        if (a.fillDist) {
+            uint4* d4 = reinterpret_cast<uint4*>(a.dist);  // its buffer is a multiple of 16 bytes
+            for (uint64_t i = gtid; i < (a.n + 3) / 4; i += gthreads) {
+                const uint64_t v = 4 * i;
+                d4[i] = make_uint4(v == src ? 0u : kInf, v + 1 == src ? 0u : kInf, v + 2 == src ? 0u : kInf,
+                                   v + 3 == src ? 0u : kInf);
+            }
+        } else if (gtid == 0) {
+            a.dist[src] = 0;
+        }
         for (uint64_t w = gtid; w < a.words; w += gthreads) {
             uint32_t pad = 0;
             if (w == a.words - 1 && (a.n & 31)) pad = ~((1u << (a.n & 31)) - 1u);  // bits past n read as visited
@@ -471,29 +735,34 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
             }
         }
         if (learned) selectorStageWait();
-        if (!gridBarrier(bar, err, a.spinLimit)) return;
+        if (!gridBarrier(bar, err, a.spinLimit)) return timedOut(a);
         level = 0;
         bottomUp = false;
         qValid = true;
         scout = d;
         toCheck = a.m;
-        unexplored = a.m - d;
-        reached = 1;
+        if (tid == 0) {
+            sm.unexplored = a.m - d;
+            sm.unreached = a.n - 1;
+        }
         lastStrat = -1;
     } else {
         level = (uint32_t)a.state[S_LEVEL];
         bottomUp = a.state[S_BOTTOMUP] != 0;
         scout = (uint64_t)a.state[S_SCOUT];
         toCheck = (uint64_t)a.state[S_TOCHECK];
-        unexplored = (uint64_t)a.state[S_UNEXPLORED];
-        reached = (uint64_t)a.state[S_REACHED];
+        if (tid == 0) {
+            sm.unexplored = (uint64_t)a.state[S_UNEXPLORED];
+            sm.unreached = a.n - (uint64_t)a.state[S_REACHED];
+        }
         qValid = a.state[S_QVALID] != 0;
         lastStrat = (int)a.state[S_LAST];
         if (learned) selectorStageWait();
-        if (!gridBarrier(bar, err, a.spinLimit)) return;
+        if (!gridBarrier(bar, err, a.spinLimit)) return timedOut(a);
     }
     const uint32_t endLevel = a.maxLevels ? a.startLevel + a.maxLevels : 0xFFFFFFFFu;
-    uint64_t tPrev = globaltimer();
+    if (tid == 0) sm.tPrev = globaltimer();
+    __syncwarp();  // warp 0 reads what thread 0 keeps
     int selLast = -1;  // last evaluated learned decision and the frontier it was made for
     bool selLastBU = false;
     float selLastF = 0.0f, selLastE = 0.0f;
@@ -509,11 +778,16 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
         nextHub = ldv(&p0->hubPack);
     }
 
+    // the bitmap of the current frontier and the counters of the current level:
+    // both move on by one per level that the grid runs
+    uint32_t bi = level % 3, ci = level % 3, stretch = 0;
     for (;;) {
-        GbPCounters* prev = &a.ctr[(level + 2) % 3];
-        GbPCounters* cur = &a.ctr[level % 3];
+        const uint32_t ci1 = ci == 2 ? 0 : ci + 1;
+        GbPCounters* prev = &a.ctr[ci1 == 2 ? 0 : ci1 + 1];
+        GbPCounters* cur = &a.ctr[ci];
         const uint64_t size = nextSize, fedges = nextEdgesC;
         if (size == 0 || level >= endLevel) break;
+        const uint32_t bi1 = bi == 2 ? 0 : bi + 1, bi2 = bi1 == 2 ? 0 : bi1 + 1;
 
         // alpha/beta rule (src/cpu/bfs_cpu.cpp:247-279): always evaluated, it
         // is the fallback and the judge of the learned choice.
@@ -521,6 +795,40 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
         if (!bottomUp) toCheck -= min(toCheck, scout);
         const int ruleStrat = bottomUp ? GB_STRAT_BU : GB_STRAT_TD_EPT2;
         int strat = a.force >= 0 ? a.force : ruleStrat;
+        // A frontier of few edges (and no split hubs) in the queue: block 0 runs
+        // it, and the levels after it while they stay small, alone; the others
+        // clear their share of the third bitmap as ever and wait.  Every block
+        // then takes over what block 0 arrived at.
+        if (strat != GB_STRAT_BU && a.force < 0 && qValid && fedges <= kSoloEdges * NT && (nextHub >> kHubShift) == 0 &&
+            a.spinLimit >= kSoloSpin) {
+            if (gtid == 0 && a.trace && level > 0 && level - 1 < a.traceCap && lastStrat == GB_STRAT_BU)
+                a.trace[level - 1].edges = ldv(&prev->examined);
+            uint32_t* third = a.bm[bi2];
+            for (uint64_t w = gtid; w < a.words; w += gthreads) third[w] = 0;
+            // two places in turn: block 0 may end its next stretch before another block has read this one's
+            unsigned long long* from = a.solo + 8 * (stretch++ & 1u);
+            if (blockIdx.x == 0)
+                soloLevels<NT>(a, sm, level, endLevel, (uint32_t)nextQ, scout, toCheck, a.bm[bi], a.bm[bi1], from);
+            if (!barrierWithState<NT>(a, sm, from)) return timedOut(a);
+            level = (uint32_t)sm.state[0];
+            bottomUp = false;
+            nextSize = sm.state[1];
+            nextEdgesC = sm.state[2];
+            nextQ = sm.state[3];
+            nextHub = sm.state[4];
+            scout = sm.state[2];
+            toCheck = sm.state[5];
+            if (tid == 0) {
+                sm.unreached -= sm.state[6];
+                sm.unexplored -= min(sm.unexplored, sm.state[7]);
+                sm.tPrev = globaltimer();
+            }
+            __syncwarp();
+            qValid = true;
+            lastStrat = GB_STRAT_TD_EPT2;
+            bi = bi1;
+            continue;
+        }
         // Warp 0 evaluates the learned selector while the other warps do the
         // level's bookkeeping; one block barrier covers both.  A level whose
         // frontier differs from the last evaluated one by less than 0.25 in
@@ -550,7 +858,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
         }
         if (useSel && tid < 32) {
             float f[kSelFeatures];
-            selectorFeatures((double)size, (double)fedges, (double)unexplored, (double)(a.n - reached), (double)a.n,
+            selectorFeatures((double)size, (double)fedges, (double)sm.unexplored, (double)sm.unreached, (double)a.n,
                              (double)a.m, (double)level, f);
             // trust region: a top-down level may go bottom-up only when its
             // edges are within 4x of the rule's threshold (toCheck / alpha);
@@ -564,9 +872,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
         if (gtid == 0) {
             if (a.trace && level > 0 && level - 1 < a.traceCap && lastStrat == GB_STRAT_BU)
                 a.trace[level - 1].edges = ldv(&prev->examined);
-            a.ctr[(level + 1) % 3] = GbPCounters{};
+            a.ctr[ci1] = GbPCounters{};
         }
-        uint32_t* clearBm = a.bm[(level + 2) % 3];
+        uint32_t* clearBm = a.bm[bi2];
         for (uint64_t w = gtid; w < a.words; w += gthreads) clearBm[w] = 0;
         __syncthreads();
         if (useSel) {
@@ -588,13 +896,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
 
         Acc acc;
         if (strat == GB_STRAT_BU) {
-            buLevel(a, level, acc);
+            buLevel(a, level, a.bm[bi], a.bm[bi1], sm.rest, acc);
         } else {
             uint32_t S = (uint32_t)nextQ;
             unsigned long long hp = nextHub;
             if (!qValid) {
-                bitmapToQueue<NT>(a, sm, level, prev);
-                if (!barrierWithCounters<NT>(a, sm, prev)) return;
+                bitmapToQueue<NT>(a, sm, level, a.bm[bi], prev);
+                if (!barrierWithCounters<NT>(a, sm, prev)) return timedOut(a);
                 S = (uint32_t)sm.cnt[2];
                 hp = sm.cnt[3];
             }
@@ -613,7 +921,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
                 // group of at least twice the mean degree: most vertices take one round
                 const uint64_t want = S ? 2 * ((qEdges + S - 1) / S) : 1;
                 const unsigned G = want <= 4 ? 4u : want <= 8 ? 8u : want <= 16 ? 16u : 32u;
-                tdGroups(a, S, G, qc, level, cur, a.bm[(level + 1) % 3], acc, fedges >= 65536, enq);
+                tdGroups(a, S, G, qc, level, cur, a.bm[bi1], acc, fedges >= 65536, enq);
             }
             const uint32_t nt = warpMode ? 0u : (S + NT - 1) / NT;
             // fewer tiles than half the blocks (a small queue, often of
@@ -630,7 +938,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
             const uint64_t HC = (uint64_t)NT * kHubEdges;
             const bool pre = fedges >= 65536;
             const uint32_t nh = (uint32_t)((HE + HC - 1) / HC);
-            uint32_t* bmNext = a.bm[(level + 1) % 3];
+            uint32_t* bmNext = a.bm[bi1];
             // block b takes item b first; further items come from a ticket
             // (none when the first items cover the level), which thread 0
             // requests while the block still works on the current item
@@ -675,19 +983,22 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
             if (sm.acc[1]) atomicAdd(&cur->nextEdges, sm.acc[1]);
             if (sm.acc[2]) atomicAdd(&cur->examined, sm.acc[2]);
         }
-        if (!barrierWithCounters<NT>(a, sm, cur)) return;
+        if (!barrierWithCounters<NT>(a, sm, cur)) return timedOut(a);
         if (gtid == 0) {
             const uint64_t t = globaltimer();
-            if (a.trace && level < a.traceCap) a.trace[level].time_ms = (double)(t - tPrev) * 1e-6;
-            tPrev = t;
+            if (a.trace && level < a.traceCap) a.trace[level].time_ms = (double)(t - sm.tPrev) * 1e-6;
+            sm.tPrev = t;
         }
         const uint64_t found = sm.cnt[0], nextE = sm.cnt[1];
+        if (tid == 0) {
+            sm.unreached -= found;
+            sm.unexplored -= min(sm.unexplored, sm.cnt[1]);
+        }
+        __syncwarp();
         nextSize = found;
         nextEdgesC = nextE;
         nextQ = sm.cnt[2];
         nextHub = sm.cnt[3];
-        reached += found;
-        unexplored -= min(unexplored, nextE);
         if (bottomUp) {
             if (!(found >= size || (double)found > (double)a.n / a.beta)) {
                 bottomUp = false;
@@ -699,17 +1010,21 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
         qValid = strat != GB_STRAT_BU && fedges < kEnqueueEdges;
         lastStrat = strat;
         ++level;
+        bi = bi1;
+        ci = ci1;
     }
+    if (a.packHost) packToHost(a, level, gtid, gthreads);
     if (gtid == 0) {
+        if (a.ctlHost) a.ctlHost[0] = level;
         if (a.trace && level > 0 && level - 1 < a.traceCap && lastStrat == GB_STRAT_BU)
-            a.trace[level - 1].edges = ldv(&a.ctr[(level + 2) % 3].examined);
+            a.trace[level - 1].edges = ldv(&a.ctr[ci == 0 ? 2 : ci - 1].examined);
         a.ctl[2] = level;
         a.state[S_LEVEL] = level;
         a.state[S_BOTTOMUP] = bottomUp;
         a.state[S_SCOUT] = (double)scout;
         a.state[S_TOCHECK] = (double)toCheck;
-        a.state[S_UNEXPLORED] = (double)unexplored;
-        a.state[S_REACHED] = (double)reached;
+        a.state[S_UNEXPLORED] = (double)sm.unexplored;
+        a.state[S_REACHED] = (double)(a.n - sm.unreached);
         a.state[S_QVALID] = qValid;
         a.state[S_LAST] = lastStrat;
     }
@@ -757,7 +1072,11 @@ PArgs makeArgs(gb_bfs& h, const gb_bfs_options& o, uint32_t src) {
     a.visited = h.pvisited.get();
     a.iso = h.pIso.get();
     a.ctr = h.pctr.get();
+    a.solo = h.psolo.get();
     a.ctl = h.pctl.get();
+    a.fillDist = h.n <= kSmallDepths;
+    a.packHost = nullptr;
+    a.ctlHost = nullptr;
     a.trace = h.ptrace.get();
     a.traceCap = kTraceCap;
     a.sel = h.selLoaded[0] ? h.selParams[0].get() : nullptr;
@@ -799,6 +1118,7 @@ void useSlot(gb_bfs& h, PArgs& a, int slot) {
     for (int i = 0; i < 3; ++i) a.bm[i] = p.bm[i].get();
     a.visited = p.visited.get();
     a.ctr = p.ctr.get();
+    a.solo = p.solo.get();
     a.trace = p.trace.get();
     a.state = p.state.get();
 }
@@ -828,7 +1148,11 @@ void gb_bfs::ensurePersistent(const gb_bfs_options& o) {
         pIsoReady = true;
     }
     pctr.ensure(3);
-    pctl.ensure(4);
+    psolo.ensure(16);
+    if (!pctl.get()) {  // the barrier word works from any value, the error word is cleared after an error
+        pctl.ensure(4);
+        GB_CUDA(cudaMemsetAsync(pctl.get(), 0, 4 * sizeof(unsigned), stream.s));
+    }
     ptrace.ensure(kTraceCap);
     pstate.ensure(S_COUNT);
     for (uint32_t k = 1; k < std::max<uint32_t>(1, o.in_flight); ++k) {
@@ -841,6 +1165,7 @@ void gb_bfs::ensurePersistent(const gb_bfs_options& o) {
         for (auto& b : p.bm) b.ensure(words);
         p.visited.ensure(words);
         p.ctr.ensure(3);
+        p.solo.ensure(16);
         p.trace.ensure(kTraceCap);
         p.state.ensure(S_COUNT);
     }
@@ -871,29 +1196,41 @@ void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb
     }
     ensurePersistent(o);
     PArgs a = makeArgs(*this, o, src);
-    GB_CUDA(cudaMemsetAsync(pctl.get(), 0, 4 * sizeof(unsigned), stream.s));
+    pctlHost.ensure(4);
+    volatile unsigned* done = pctlHost.p;  // the kernel's last act: levels run, width of the packed depths
+    done[0] = kNotDone;
+    done[2] = 0;
+    a.ctlHost = pctlHost.p;
+    const bool packInKernel = out && n <= kSmallDepths;
+    if (packInKernel) {
+        packHost.ensure(2 * n + 16);
+        a.packHost = packHost.p;
+    }
     GB_CUDA(cudaEventRecord(ev.a, stream.s));
-    GB_CUDA(cudaMemsetAsync(dist.get(), 0xFF, n * 4, stream.s));  // every depth infinity (0xFFFFFFFF)
+    if (!a.fillDist) GB_CUDA(cudaMemsetAsync(dist.get(), 0xFF, n * 4, stream.s));  // every depth infinity (0xFFFFFFFF)
     launchFor(*this, a);
     GB_CUDA(cudaEventRecord(ev.b, stream.s));
-    pctlHost.ensure(4);
-    const unsigned* ctl = pctlHost.p;
-    GB_CUDA(cudaMemcpyAsync(pctlHost.p, pctl.get(), 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream.s));
-    // the depths follow on the stream, packed for as many levels as the last
-    // run had (else for one byte), so one wait covers traversal and copy
+    // a larger array's depths follow on the stream, packed for as many levels as
+    // the last run had (else for one byte), so one wait covers traversal and copy
     DepthReturn ret;
-    if (out) beginDepths(this, dist.get(), n, lastLevels ? lastLevels : 254, ret);
-    if (out) waitDepths(this, ret);
-    else GB_CUDA(cudaStreamSynchronize(stream.s));
+    if (out && !packInKernel) {
+        beginDepths(this, dist.get(), n, lastLevels ? lastLevels : 254, ret);
+        waitDepths(this, ret);
+    } else {
+        GB_CUDA(cudaStreamSynchronize(stream.s));
+    }
     lastGpuMs = ev.ms();
-    lastLevels = ctl[2];
-    if (ctl[1]) {
+    if (done[0] == kNotDone || done[2]) {
+        GB_CUDA(cudaMemsetAsync(pctl.get(), 0, 4 * sizeof(unsigned), stream.s));
         GB_CUDA(cudaStreamSynchronize(stream.s));
         throw Error(GB_ERR_TIMEOUT, "persistent BFS: grid barrier wait exceeded its spin limit");
     }
-    if (out) endDepths(this, ret, lastLevels, out);
+    lastLevels = done[0];
+    if (packInKernel && (int)done[1] >= 0) widenPacked((int)done[1], packHost.p, n, out);
+    else if (packInKernel) staged.run(dist.get(), n * 4, out, stream.s);
+    else if (out) endDepths(this, ret, lastLevels, out);
     if (tr) {
-        const uint32_t k = std::min<uint32_t>(ctl[2], kTraceCap);
+        const uint32_t k = std::min<uint32_t>(lastLevels, kTraceCap);
         std::vector<gb_level> t(k);
         if (k) GB_CUDA(cudaMemcpy(t.data(), ptrace.get(), k * sizeof(gb_level), cudaMemcpyDeviceToHost));
         for (auto& r : t) r.pad = 0;
@@ -991,7 +1328,7 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
             if (out) GB_CUDA(cudaStreamWaitEvent(st, copied, 0));
         }
         if (timed || i + 1 == count) GB_CUDA(cudaEventRecord(mEv[2 * i], st));
-        GB_CUDA(cudaMemsetAsync(bufs[b], 0xFF, n * 4, st));  // every depth infinity
+        if (!a.fillDist) GB_CUDA(cudaMemsetAsync(bufs[b], 0xFF, n * 4, st));  // every depth infinity
         launchFor(*this, a, grid, st);
         if (timed || i + 1 == count) GB_CUDA(cudaEventRecord(mEv[2 * i + 1], st));
         if (!out) {
