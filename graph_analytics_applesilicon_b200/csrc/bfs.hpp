@@ -66,6 +66,11 @@ int packFormat(uint32_t levels);
 uint64_t packedBytes(int fmt, uint64_t count);
 void enqueuePack(int fmt, const uint32_t* d, uint64_t count, uint8_t* dev, unsigned* overflow, cudaStream_t st);
 void widenPacked(int fmt, const uint8_t* in, uint64_t count, uint32_t* out);
+// Depth arrays up to this size are packed straight into pinned host memory, by
+// the traversal's kernel or one after it; larger ones into device memory, and
+// copied in chunks that the widening overlaps.
+constexpr uint64_t kSmallDepths = 1ull << 20;
+constexpr int kEdgeStatWords = 8;
 constexpr int kMaxInFlight = 16;              // traversals at once in gb_bfs::runPersistentMany
 constexpr int kManySlots = kMaxInFlight + 2;  // depth buffers it rotates (in flight + 2)
 }  // namespace gb
@@ -78,13 +83,16 @@ struct gb_bfs {
     uint32_t flags = 0;     // the graph's GGPUCSR1 flags when known (file handles)
     gb::Stream stream;
     gb::EventPair ev;
-    gb::ScanScratch scan;
 
     // host-driven forms
     gb::DevBuf<GbLevelStats> stats;
     gb::HostPinned<GbLevelStats> hstats;
     gb::HostPinned<uint32_t> hstage;
-    gb::DevBuf<uint32_t> qA, qB, degA, degB, bins[2][3], bmFront, bmNext;
+    gb::DevBuf<uint32_t> qA, qB, bins[2][3], bmFront, bmNext;
+    gb::DevBuf<uint32_t> offA, offB;               // gpu_edge, gpu_do: edge offsets of qA, qB
+    gb::DevBuf<unsigned long long> edgeStats;      // and their counters
+    gb::HostPinned<unsigned long long> edgePub;    // what a level leaves there
+    unsigned long long edgeSeq = 0;                // levels they have run
 
     // persistent single-source
     gb::DevBuf<uint32_t> pq[2][3];       // queue: vertex, adjacency start, degree
@@ -166,8 +174,9 @@ struct gb_bfs {
     void runVertex(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr);
     void runNaive(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr);
     void runBinned(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr);
-    void runEdge(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr);
-    void runDirOpt(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr);
+    // wait: return when the stream is idle; else the last level's kernel may still be ending
+    void runEdge(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr, bool wait = true);
+    void runDirOpt(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr, bool wait = true);
     // out: also return the depths there (host memory), the copy queued behind the traversal
     void runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr, uint32_t* out = nullptr);
     void runBatch(const uint32_t* src, int k, const gb_bfs_options& o, std::vector<gb_level>* tr);

@@ -1,5 +1,5 @@
-// bfs_levels.cu -- the host-driven BFS forms: one launch sequence and one host
-// synchronisation per level, as the reference's GpuBfs::run* loops
+// bfs_levels.cu -- the host-driven BFS forms: one launch or launch sequence and
+// one host wait per level, as the reference's GpuBfs::run* loops
 // (src/metal/bfs_gpu.mm:115-429).  They are the "plain" forms the persistent
 // kernel is measured against, and the drop-in for gpu_vertex / gpu_naive /
 // gpu_binned / gpu_edge / gpu_do.
@@ -8,10 +8,14 @@
 // + one atomic per warp), CAS claims on dist, shared-memory staging of the
 // scanned frontier degrees in the edge-balanced expansion, and bitmap
 // frontiers with __ballot_sync word assembly in the bottom-up step.
+#include <emmintrin.h>
+
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 
 #include "bfs.hpp"
+#include "bfs_device.cuh"
 
 namespace gb {
 
@@ -189,34 +193,98 @@ __global__ void binnedLargeKernel(BinArgs a) {
 
 // ------------------------------------------------------------- gpu_edge
 
-constexpr uint32_t kStageCap = 2048;
+// One launch per level (gpu_edge, gpu_do).  A level of these forms is short (a
+// few us on R-MAT 16), so what a call takes is what surrounds its kernels: with a
+// counter memset, a three-part scan of the frontier's degrees, a counter copy, two
+// events and a stream wait around each expansion a level cost 41 us (6 levels,
+// 265 us a call).  Here
+//  - an append reserves queue slots and edge offsets with one 64-bit atomic, so
+//    the next level's offsets are scanned as they are written;
+//  - the last block to finish stores the level's counters and its time into pinned
+//    memory, where the host polls for them, and zeroes them for the next level;
+//  - the first launch of a run does all the setting up.
+// A level takes 18 us so, a call 126.
 
-__device__ __forceinline__ uint32_t findOwner(const uint32_t* off, uint32_t lo, uint32_t hi, uint32_t e) {
-    while (lo < hi) {  // largest i in [lo, hi] with off[i] <= e
-        uint32_t mid = (lo + hi + 1) >> 1;
-        if (off[mid] <= e) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
+// Sums over a level, zero between levels.  `append` is (vertices << 32) | sum of
+// their degrees: at most n vertices and m adjacency entries, both below 2^32.
+struct EdgeStats {
+    unsigned long long append, examined, t0;
+    unsigned long long queued;  // queueFromBitmapKernel's append word
+    unsigned ticket;
+};
+static_assert(sizeof(EdgeStats) <= sizeof(unsigned long long) * kEdgeStatWords, "room in the handle's buffer");
+
+struct EdgeArgs {
+    const uint32_t* row_ptr;
+    const uint32_t* col_idx;
+    uint32_t* dist;
+    EdgeStats* s;
+    unsigned long long* pub;  // pinned: append, examined, device time in ns, sequence number
+    unsigned long long seq;
+    uint32_t level;
+    bool first;  // no launch of this level before this one
+};
+
+__device__ __forceinline__ void levelStart(const EdgeArgs& a) {
+    if (a.first && blockIdx.x == 0 && threadIdx.x == 0) a.s->t0 = globaltimer();
 }
+
+// Ends a level: every block calls it after its own additions to *a.s.
+__device__ __forceinline__ void levelEnd(const EdgeArgs& a) {
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&a.s->ticket, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    volatile EdgeStats* s = a.s;
+    volatile unsigned long long* pub = a.pub;
+    pub[0] = s->append;
+    pub[1] = s->examined;
+    pub[2] = globaltimer() - s->t0;
+    s->append = s->examined = s->queued = 0;
+    s->ticket = 0;
+    __threadfence_system();
+    pub[3] = a.seq;
+}
+
+// Depths to infinity, the source and its queue entry, the counters to zero.
+__global__ void edgeInitKernel(EdgeArgs a, uint64_t n, uint32_t source, uint32_t* queue, uint32_t* offsets) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint4* d4 = reinterpret_cast<uint4*>(a.dist);  // its buffer is a multiple of 16 bytes
+    for (uint64_t i = t; i < (n + 3) / 4; i += stride) {
+        const uint64_t v = 4 * i;
+        d4[i] = make_uint4(v == source ? 0u : kInf, v + 1 == source ? 0u : kInf, v + 2 == source ? 0u : kInf,
+                           v + 3 == source ? 0u : kInf);
+    }
+    if (t == 0) {
+        *a.s = EdgeStats{};
+        a.s->t0 = globaltimer();
+        queue[0] = source;
+        offsets[0] = 0;
+    }
+}
+
+constexpr uint32_t kStageCap = 2048;
 
 // Edge-balanced expansion: block b owns edges [b*chunk, (b+1)*chunk) of the
 // level (chunk = blockDim * ept); thread t takes edges t, t+blockDim, ... so a
-// warp reads 32 consecutive edges per round.  Thread 0 finds the chunk's
-// owner range once; the range's scanned offsets and adjacency starts are
-// staged in shared memory so every per-edge owner search runs there.
-__global__ void edgeExpandKernel(const uint32_t* row_ptr, const uint32_t* col_idx, uint32_t* dist, Stats* s,
-                                 const uint32_t* queue, const uint32_t* offsets, uint32_t* nextQ, uint32_t* nextDeg,
-                                 uint32_t size, uint32_t total, uint32_t level, uint32_t ept) {
+// warp reads 32 consecutive edges per round.  Two warps find the chunk's owner
+// range; the range's scanned offsets and adjacency starts are staged in shared
+// memory so every per-edge owner search runs there.  R rounds go through each
+// stage together (their loads and claims overlap, one append for all R).
+template <int R>
+__global__ void __launch_bounds__(1024) edgeExpandKernel(EdgeArgs a, const uint32_t* queue, const uint32_t* offsets,
+                                                         uint32_t* nextQ, uint32_t* nextOff, uint32_t size,
+                                                         uint32_t total, uint32_t ept) {
     __shared__ uint32_t sOff[kStageCap], sStart[kStageCap];
     __shared__ uint32_t sRange[2];
-    const uint32_t chunk = blockDim.x * ept;
-    const uint32_t c0 = blockIdx.x * chunk;
-    const uint32_t c1 = min(c0 + chunk, total);
-    if (threadIdx.x == 0) {
-        uint32_t lo = findOwner(offsets, 0, size - 1, c0);
-        sRange[0] = lo;
-        sRange[1] = findOwner(offsets, lo, size - 1, c1 - 1);
+    levelStart(a);
+    const uint64_t chunk = (uint64_t)blockDim.x * ept, c0 = blockIdx.x * chunk;
+    const uint64_t c1 = min(c0 + chunk, (uint64_t)total);
+    const unsigned warp = threadIdx.x >> 5, lane = laneId();
+    for (unsigned k = warp; k < 2; k += blockDim.x >> 5) {
+        const uint32_t o = warpOwnerOf(offsets, 0u, size - 1, (uint32_t)(k ? c1 - 1 : c0));
+        if (lane == 0) sRange[k] = o;
     }
     __syncthreads();
     const uint32_t lo = sRange[0], hi = sRange[1], cnt = hi - lo + 1;
@@ -224,33 +292,62 @@ __global__ void edgeExpandKernel(const uint32_t* row_ptr, const uint32_t* col_id
     if (staged)
         for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
             sOff[i] = offsets[lo + i];
-            sStart[i] = row_ptr[queue[lo + i]];
+            sStart[i] = a.row_ptr[queue[lo + i]];
         }
     __syncthreads();
-    for (uint32_t k = 0; k < ept; ++k) {  // block-uniform rounds: appends stay convergent
-        uint32_t e = c0 + k * blockDim.x + threadIdx.x;
-        bool has = e < c1;
-        uint32_t u = 0;
-        if (has) {
+    for (uint32_t k0 = 0; k0 < ept; k0 += R) {  // block-uniform rounds: appends stay convergent
+        uint32_t u[R], st[R], en[R];
+        bool has[R];
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const uint64_t e = c0 + (uint64_t)(k0 + k) * blockDim.x + threadIdx.x;
+            has[k] = k0 + k < ept && e < c1;
+            u[k] = 0;
+            if (!has[k]) continue;
             if (staged) {
-                uint32_t i = findOwner(sOff, 0, cnt - 1, e);
-                u = col_idx[sStart[i] + (e - sOff[i])];
+                const uint32_t i = ownerOf(sOff, 0u, cnt - 1, (uint32_t)e);
+                u[k] = a.col_idx[sStart[i] + ((uint32_t)e - sOff[i])];
             } else {
-                uint32_t i = findOwner(offsets, lo, hi, e);
-                u = col_idx[row_ptr[queue[i]] + (e - offsets[i])];
+                const uint32_t i = ownerOf(offsets, lo, hi, (uint32_t)e);
+                u[k] = a.col_idx[a.row_ptr[queue[i]] + ((uint32_t)e - offsets[i])];
             }
         }
-        bool claimed = has && claimDist(dist, u, level + 1);
-        if (!__any_sync(kFull, claimed)) continue;
-        uint32_t udeg = claimed ? row_ptr[u + 1] - row_ptr[u] : 0u;
-        uint32_t pos = warpAppend(claimed, &s->found);
-        if (claimed) {
-            nextQ[pos] = u;
-            nextDeg[pos] = udeg;
+#pragma unroll
+        for (int k = 0; k < R; ++k) has[k] = has[k] && *reinterpret_cast<volatile uint32_t*>(&a.dist[u[k]]) == kInf;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            st[k] = has[k] ? a.row_ptr[u[k]] : 0u;
+            en[k] = has[k] ? a.row_ptr[u[k] + 1] : 0u;
+            has[k] = has[k] && atomicCAS(&a.dist[u[k]], kInf, a.level + 1) == kInf;
         }
-        unsigned long long ne = warpSum((unsigned long long)udeg);
-        if (laneId() == 0 && ne) atomicAdd(&s->nextEdges, ne);
+        unsigned long long mine = 0;
+#pragma unroll
+        for (int k = 0; k < R; ++k) mine += has[k] ? (1ull << 32) | (en[k] - st[k]) : 0ull;
+        if (!__any_sync(kFull, mine != 0)) continue;
+        unsigned long long incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= (unsigned)o) incl += y;
+        }
+        unsigned long long at = 0;
+        if (lane == 31) at = atomicAdd(&a.s->append, incl);
+        at = __shfl_sync(kFull, at, 31) + incl - mine;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            if (!has[k]) continue;
+            nextQ[at >> 32] = u[k];
+            nextOff[at >> 32] = (uint32_t)at;
+            at += (1ull << 32) | (en[k] - st[k]);
+        }
     }
+    levelEnd(a);
+}
+
+// A top-down level whose frontier has no edges.
+__global__ void noEdgesKernel(EdgeArgs a) {
+    levelStart(a);
+    levelEnd(a);
 }
 
 // ------------------------------------------------------------- bottom-up
@@ -258,36 +355,80 @@ __global__ void edgeExpandKernel(const uint32_t* row_ptr, const uint32_t* col_id
 // Thread per vertex: an unreached vertex scans its list for the first parent
 // in the frontier bitmap (early exit).  The 32 lanes of a warp are one bitmap
 // word of the next frontier, assembled with __ballot_sync and stored by lane
-// 0, so every word of `next` is written and needs no clearing.
-__global__ void bottomUpKernel(const uint32_t* row_ptr, const uint32_t* col_idx, uint32_t* dist,
-                               const uint32_t* front, uint32_t* next, Stats* s, uint64_t n, uint32_t level) {
+// 0, so every word of `next` is written and needs no clearing.  One addition
+// per block and counter: per warp, an R-MAT 22 level's 113,000 additions to one
+// line take 80 us by themselves.
+__global__ void __launch_bounds__(1024) bottomUpKernel(EdgeArgs a, const uint32_t* front, uint32_t* next, uint64_t n) {
+    __shared__ unsigned long long sum[2];
+    levelStart(a);
+    if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+    __syncthreads();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    unsigned long long foundC = 0, examined = 0, ndeg = 0;
+    unsigned long long append = 0, examined = 0;
     for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint64_t v = base + threadIdx.x;
         bool found = false;
-        if (v < n && dist[v] == kInf) {
-            uint32_t b = row_ptr[v], e = row_ptr[v + 1];
-            for (uint32_t i = b; i < e; ++i) {
-                ++examined;
-                uint32_t u = col_idx[i];
-                if ((front[u >> 5] >> (u & 31)) & 1u) {
-                    found = true;
-                    break;
+        if (v < n && a.dist[v] == kInf) {
+            const uint32_t b = a.row_ptr[v], e = a.row_ptr[v + 1];
+            if (b < e) {
+                examined += buScanFrom(a.col_idx, front, b, e, found) - b;
+                if (found) {
+                    a.dist[v] = a.level + 1;
+                    append += (1ull << 32) | (e - b);
                 }
             }
-            if (found) {
-                dist[v] = level + 1;
-                ndeg += e - b;
-                ++foundC;
-            }
         }
-        unsigned word = __ballot_sync(kFull, found);
+        const unsigned word = __ballot_sync(kFull, found);
         if (laneId() == 0 && v < n) next[v >> 5] = word;
     }
-    foundC = warpSum(foundC);
-    if (laneId() == 0 && foundC) atomicAdd(&s->found, (unsigned)foundC);
-    addStats(s, 0, examined, ndeg);
+    append = warpSum(append);
+    examined = warpSum(examined);
+    if (laneId() == 0) {
+        if (append) atomicAdd(&sum[0], append);
+        if (examined) atomicAdd(&sum[1], examined);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (sum[0]) atomicAdd(&a.s->append, sum[0]);
+        if (sum[1]) atomicAdd(&a.s->examined, sum[1]);
+    }
+    levelEnd(a);
+}
+
+// The frontier's bitmap from the depths (the first bottom-up level).
+__global__ void frontBitmapKernel(EdgeArgs a, uint32_t* front, uint64_t n) {
+    levelStart(a);
+    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t v = base + threadIdx.x;
+        const unsigned word = __ballot_sync(kFull, v < n && a.dist[v] == a.level);
+        if (laneId() == 0 && v < n) front[v >> 5] = word;
+    }
+}
+
+// The frontier's queue and edge offsets from its bitmap (the first top-down
+// level after bottom-up ones): one append per block and 256 vertices.
+constexpr int kQueueThreads = 256;
+
+__global__ void queueFromBitmapKernel(EdgeArgs a, const uint32_t* front, uint64_t n, uint32_t* queue,
+                                      uint32_t* offsets) {
+    __shared__ unsigned long long scan[kQueueThreads / 32 + 1], at0;
+    levelStart(a);
+    for (uint64_t base = (uint64_t)blockIdx.x * kQueueThreads; base < n; base += (uint64_t)gridDim.x * kQueueThreads) {
+        const uint64_t v = base + threadIdx.x;
+        const bool in = v < n && ((front[v >> 5] >> (v & 31)) & 1u);
+        const unsigned long long mine = in ? (1ull << 32) | (a.row_ptr[v + 1] - a.row_ptr[v]) : 0ull;
+        unsigned long long total;
+        unsigned long long at = blockScan<kQueueThreads>(mine, &total, scan);
+        if (total == 0) continue;  // block-uniform
+        if (threadIdx.x == 0) at0 = atomicAdd(&a.s->queued, total);
+        __syncthreads();
+        at += at0;
+        if (in) {
+            queue[at >> 32] = (uint32_t)v;
+            offsets[at >> 32] = (uint32_t)at;
+        }
+        __syncthreads();  // at0 is the next round's
+    }
 }
 
 uint32_t gridCap(uint64_t work, uint32_t threads) {
@@ -326,8 +467,10 @@ void gb_bfs::endLevel() {
 void gb_bfs::ensureEdgeBuffers() {
     qA.ensure(n);
     qB.ensure(n);
-    degA.ensure(n);
-    degB.ensure(n);
+    offA.ensure(n);
+    offB.ensure(n);
+    edgeStats.ensure(kEdgeStatWords);
+    edgePub.ensure(4);
 }
 
 void gb_bfs::runVertex(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr) {
@@ -416,110 +559,140 @@ void gb_bfs::runBinned(uint32_t src, const gb_bfs_options& o, std::vector<gb_lev
 }
 
 namespace {
-// One gpu_edge level: scan degrees into offsets in place, then expand.
-void edgeLevel(gb_bfs& h, uint32_t* q, uint32_t* deg, uint32_t* qNext, uint32_t* degNext, uint32_t size,
-               uint64_t total, uint32_t level, uint32_t tg, uint32_t ept) {
-    scanExclusive(deg, deg, size, nullptr, h.scan, h.stream.s);
-    const uint64_t chunk = (uint64_t)tg * ept;
-    edgeExpandKernel<<<divUp(total, chunk), tg, 0, h.stream.s>>>(h.rowPtr.get(), h.colIdx.get(), h.dist.get(),
-                                                                 h.stats.get(), q, deg, qNext, degNext, size,
-                                                                 (uint32_t)total, level, ept);
-    GB_LAUNCH_CHECK();
-}
+// The levels of a gpu_edge or gpu_do run on the handle's stream.
+struct EdgeRun {
+    gb_bfs& h;
+    const uint32_t tg, ept;
+    EdgeArgs a{};
+    uint32_t *q, *off, *qNext, *offNext;
+    uint64_t size = 1, total;  // frontier: vertices, sum of their degrees
+    uint64_t examined = 0;     // by the last level, if bottom-up
+
+    EdgeRun(gb_bfs& h_, uint32_t src, const gb_bfs_options& o) : h(h_), tg(checkTg(o.tg)), ept(o.ept), total(h_.degree(src)) {
+        if (ept == 0) throw Error(GB_ERR_ARG, "ept must be >= 1");
+        h.ensureEdgeBuffers();
+        q = h.qA.get(), qNext = h.qB.get(), off = h.offA.get(), offNext = h.offB.get();
+        a.row_ptr = h.rowPtr.get();
+        a.col_idx = h.colIdx.get();
+        a.dist = h.dist.get();
+        a.s = reinterpret_cast<EdgeStats*>(h.edgeStats.get());
+        a.pub = h.edgePub.p;
+        h.edgePub.p[3] = 0;  // no level's number
+        h.lastGpuMs = 0;
+        h.lastLevels = 0;
+        edgeInitKernel<<<gridCap(h.n / 4 + 1, 256), 256, 0, h.stream.s>>>(a, h.n, src, q, off);
+        GB_LAUNCH_CHECK();
+    }
+
+    void begin(uint32_t level) {
+        a.level = level;
+        a.first = level > 0;  // the first level's time begins with the setting up
+        a.seq = ++h.edgeSeq;
+    }
+    void topDown() {
+        if (total == 0) {
+            noEdgesKernel<<<1, 32, 0, h.stream.s>>>(a);
+            GB_LAUNCH_CHECK();
+            return;
+        }
+        const uint32_t grid = divUp(total, (uint64_t)tg * ept);
+        if (ept <= 2)
+            edgeExpandKernel<2><<<grid, tg, 0, h.stream.s>>>(a, q, off, qNext, offNext, (uint32_t)size, (uint32_t)total, ept);
+        else
+            edgeExpandKernel<4><<<grid, tg, 0, h.stream.s>>>(a, q, off, qNext, offNext, (uint32_t)size, (uint32_t)total, ept);
+        GB_LAUNCH_CHECK();
+    }
+    // Waits for the level's counters; the frontier is then the next one.
+    void end() {
+        ++h.lastLevels;
+        const volatile unsigned long long* pub = h.edgePub.p;
+        for (uint64_t spins = 1; pub[3] != a.seq; ++spins) {
+            _mm_pause();
+            if (spins & 1023) continue;
+            const cudaError_t e = cudaStreamQuery(h.stream.s);
+            if (e == cudaErrorNotReady) continue;
+            GB_CUDA(e);
+            if (pub[3] != a.seq) throw Error(GB_ERR_CUDA, "a level ended without its counters");
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);
+        size = pub[0] >> 32;
+        total = (uint32_t)pub[0];
+        examined = pub[1];
+        h.lastGpuMs += pub[2] * 1e-6;
+    }
+    void swapQueues() {
+        std::swap(q, qNext);
+        std::swap(off, offNext);
+    }
+};
 }  // namespace
 
-void gb_bfs::runEdge(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr) {
-    const uint32_t tg = checkTg(o.tg);
-    if (o.ept == 0) throw Error(GB_ERR_ARG, "ept must be >= 1");
-    ensureEdgeBuffers();
-    uint32_t *q = qA.get(), *qNext = qB.get(), *deg = degA.get(), *degNext = degB.get();
-    hstage.p[0] = src;
-    hstage.p[1] = degree(src);
-    GB_CUDA(cudaMemcpyAsync(q, hstage.p, 4, cudaMemcpyHostToDevice, stream.s));
-    GB_CUDA(cudaMemcpyAsync(deg, hstage.p + 1, 4, cudaMemcpyHostToDevice, stream.s));
-    uint32_t size = 1;
-    uint64_t total = degree(src);
-    lastGpuMs = 0;
-    lastLevels = 0;
-    for (uint32_t level = 0; size > 0; ++level) {
+void gb_bfs::runEdge(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr, bool wait) {
+    EdgeRun r(*this, src, o);
+    for (uint32_t level = 0; r.size > 0; ++level) {
         auto t0 = std::chrono::steady_clock::now();
-        GB_CUDA(cudaEventRecord(ev.a, stream.s));
-        beginLevel();
-        if (level == 0) initDist(src);
-        if (total > 0) edgeLevel(*this, q, deg, qNext, degNext, size, total, level, tg, o.ept);
-        endLevel();
-        const GbLevelStats& s = *hstats.p;
+        const uint64_t size = r.size, total = r.total;
+        r.begin(level);
+        r.topDown();
+        r.end();
         if (tr) tr->push_back({level, 'T', 'G', 0, 0, size, total, msSince(t0)});
-        size = s.found;
-        total = s.nextEdges;
-        std::swap(q, qNext);
-        std::swap(deg, degNext);
+        r.swapQueues();
     }
+    if (wait) GB_CUDA(cudaStreamSynchronize(stream.s));
 }
 
 // gpu_do: the alpha/beta rule of cpu::bfsDO / GpuBfs::runDirOpt
 // (src/cpu/bfs_cpu.cpp:227-283, src/metal/bfs_gpu.mm:326-429), decided on the
-// host from the counters read back after every level.
-void gb_bfs::runDirOpt(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr) {
-    const uint32_t tg = checkTg(o.tg);
-    if (o.ept == 0) throw Error(GB_ERR_ARG, "ept must be >= 1");
-    ensureEdgeBuffers();
+// host from the counters each level leaves.
+void gb_bfs::runDirOpt(uint32_t src, const gb_bfs_options& o, std::vector<gb_level>* tr, bool wait) {
     const uint64_t words = (n + 31) / 32;
     bmFront.ensure(words);
     bmNext.ensure(words);
-    uint32_t *q = qA.get(), *qNext = qB.get(), *deg = degA.get(), *degNext = degB.get();
+    EdgeRun r(*this, src, o);
     uint32_t *front = bmFront.get(), *next = bmNext.get();
-    hstage.p[0] = src;
-    hstage.p[1] = degree(src);
-    GB_CUDA(cudaMemcpyAsync(q, hstage.p, 4, cudaMemcpyHostToDevice, stream.s));
-    GB_CUDA(cudaMemcpyAsync(deg, hstage.p + 1, 4, cudaMemcpyHostToDevice, stream.s));
-    uint64_t size = 1, total = degree(src), scout = total, toCheck = m;
+    uint64_t scout = r.total, toCheck = m;
     bool bottomUp = false, toBitmap = false, toQueue = false;
-    lastGpuMs = 0;
-    lastLevels = 0;
-    for (uint32_t level = 0; size > 0; ++level) {
+    for (uint32_t level = 0; r.size > 0; ++level) {
         auto t0 = std::chrono::steady_clock::now();
         if (!bottomUp && (double)scout > (double)toCheck / o.alpha) {
             bottomUp = true;
             toBitmap = true;
         }
         if (!bottomUp) toCheck -= std::min(toCheck, scout);
-        GB_CUDA(cudaEventRecord(ev.a, stream.s));
-        beginLevel();
-        if (level == 0) initDist(src);
+        const uint64_t size = r.size, total = r.total;
+        r.begin(level);
         if (bottomUp) {
-            if (toBitmap) queueToBitmap(q, size, front, n, stream.s);
-            bottomUpKernel<<<gridCap(n, tg), tg, 0, stream.s>>>(rowPtr.get(), colIdx.get(), dist.get(), front, next,
-                                                                stats.get(), n, level);
+            if (toBitmap) {
+                frontBitmapKernel<<<gridCap(n, 256), 256, 0, stream.s>>>(r.a, front, n);
+                GB_LAUNCH_CHECK();
+                r.a.first = false;
+            }
+            bottomUpKernel<<<gridCap(n, r.tg), r.tg, 0, stream.s>>>(r.a, front, next, n);
             GB_LAUNCH_CHECK();
         } else {
-            if (toQueue) {
-                // Bitmap -> queue with the degrees gpu_edge scans; the count
-                // lands in stats.bin[0] (unused by this form).
-                bitmapToQueue(front, n, q, &stats.get()->bin[0], rowPtr.get(), deg, stream.s);
+            if (toQueue && total > 0) {
+                queueFromBitmapKernel<<<gridCap(n, kQueueThreads), kQueueThreads, 0, stream.s>>>(r.a, front, n, r.q, r.off);
+                GB_LAUNCH_CHECK();
+                r.a.first = false;
             }
-            if (total > 0) edgeLevel(*this, q, deg, qNext, degNext, (uint32_t)size, total, level, tg, o.ept);
+            r.topDown();
         }
-        endLevel();
-        const GbLevelStats& s = *hstats.p;
+        r.end();
         toBitmap = toQueue = false;
         if (tr)
             tr->push_back({level, bottomUp ? 'B' : 'T', 'G', (uint8_t)(bottomUp ? GB_STRAT_BU : GB_STRAT_TD_EPT2), 0,
-                           size, bottomUp ? s.edges : total, msSince(t0)});
-        const uint64_t oldSize = size;
-        size = s.found;
-        total = s.nextEdges;
+                           size, bottomUp ? r.examined : total, msSince(t0)});
         if (bottomUp) {
             std::swap(front, next);
-            if (!(size >= oldSize || (double)size > (double)n / o.beta)) {
+            if (!(r.size >= size || (double)r.size > (double)n / o.beta)) {
                 bottomUp = false;
                 toQueue = true;
                 scout = 1;
             }
         } else {
-            scout = total;
-            std::swap(q, qNext);
-            std::swap(deg, degNext);
+            scout = r.total;
+            r.swapQueues();
         }
     }
+    if (wait) GB_CUDA(cudaStreamSynchronize(stream.s));
 }

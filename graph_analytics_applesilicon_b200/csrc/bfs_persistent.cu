@@ -34,11 +34,6 @@ constexpr uint64_t kEnqueueEdges = 1ull << 18;  // top-down levels with this man
 // (soloLevels).  A level of 4 takes 5 us there against 6.5 on the grid, one of 8
 // 10 us (road 300 x 300, rule: 2.7 ms with 2 edges per thread, 1.8 with 4).
 constexpr uint32_t kSoloEdges = 4;
-// Depth arrays up to this size are filled by the kernel and, for a run that
-// returns them, packed by it into pinned host memory; larger ones by a memset
-// before the launch and a kernel and chunked copies after it, which the
-// widening overlaps.
-constexpr uint64_t kSmallDepths = 1ull << 20;
 constexpr unsigned kNotDone = 0xFFFFFFFFu;
 // At most so many levels at a time, which bounds the other blocks' wait (about
 // 0.3 ms, some 400 polls); a caller's spin limit under kSoloSpin polls, which may
@@ -64,7 +59,7 @@ struct PArgs {
     GbPCounters* ctr;
     unsigned long long* solo;  // [2][8], see soloLevels
     unsigned* ctl;  // [0] barrier word, [1] error flag, [2] levels run
-    bool fillDist;      // the kernel sets the depths to infinity (else a memset before the launch)
+    bool fillDist;      // the kernel sets the depths to infinity (at most kSmallDepths; else a memset before the launch)
     uint8_t* packHost;  // pinned host memory for the packed depths, or null
     unsigned* ctlHost;  // pinned: [0] levels run, [1] width of the packed depths (with packHost), [2] a wait ran out
     gb_level* trace;
@@ -311,40 +306,6 @@ __device__ void tdHubChunk(const PArgs& a, Smem<NT>& sm, uint64_t e0, uint64_t e
     __syncthreads();
 }
 
-// The rest of one vertex's bottom-up scan after its first entry missed: the
-// first parent in the frontier, scanning in list order from i; aligned groups
-// of 4 entries are loaded at once and their 4 frontier words fetched
-// together, so a step costs two dependent loads for 4 entries.  Returns one
-// past the first hit, or e when there is none (found tells which).
-__device__ __forceinline__ uint32_t buScanFrom(const PArgs& a, const uint32_t* front, uint32_t i, uint32_t e,
-                                               bool& found) {
-    for (; i < e && (i & 3u); ++i) {
-        const uint32_t u = a.col_idx[i];
-        if ((front[u >> 5] >> (u & 31)) & 1u) {
-            found = true;
-            return i + 1;
-        }
-    }
-    for (; i + 4 <= e; i += 4) {
-        const uint4 q = *reinterpret_cast<const uint4*>(a.col_idx + i);
-        const uint32_t f0 = front[q.x >> 5], f1 = front[q.y >> 5], f2 = front[q.z >> 5], f3 = front[q.w >> 5];
-        const unsigned hits = ((f0 >> (q.x & 31)) & 1u) | (((f1 >> (q.y & 31)) & 1u) << 1) |
-                              (((f2 >> (q.z & 31)) & 1u) << 2) | (((f3 >> (q.w & 31)) & 1u) << 3);
-        if (hits) {
-            found = true;
-            return i + __ffs(hits);
-        }
-    }
-    for (; i < e; ++i) {
-        const uint32_t u = a.col_idx[i];
-        if ((front[u >> 5] >> (u & 31)) & 1u) {
-            found = true;
-            return i + 1;
-        }
-    }
-    return e;
-}
-
 // Bottom-up level: each unvisited vertex looks for its first parent in the
 // frontier bitmap.  A warp takes kBuWords bitmap words (32 vertices each, a
 // lane per vertex) per round and issues their loads stage by stage -- visited
@@ -408,7 +369,7 @@ __device__ void buLevel(const PArgs& a, uint32_t level, const uint32_t* front, u
                 const uint64_t v = (w0 + (uint64_t)(code >> 5) * nwarps) * 32 + (code & 31);
                 const uint32_t en = a.row_ptr[v + 1];
                 bool found = false;
-                acc.exam += buScanFrom(a, front, st + 1, en, found) - st;
+                acc.exam += buScanFrom(a.col_idx, front, st + 1, en, found) - st;
                 if (found) {
                     a.dist[v] = level + 1;
                     acc.deg += en - st;

@@ -284,8 +284,8 @@ int gb_bfs_run(gb_bfs* h, int variant, uint32_t source, uint32_t* out_host, cons
             case GB_BFS_VERTEX: h->runVertex(source, o, tp); break;
             case GB_BFS_NAIVE: h->runNaive(source, o, tp); break;
             case GB_BFS_BINNED: h->runBinned(source, o, tp); break;
-            case GB_BFS_EDGE: h->runEdge(source, o, tp); break;
-            case GB_BFS_DO: h->runDirOpt(source, o, tp); break;
+            case GB_BFS_EDGE: h->runEdge(source, o, tp, !out_host); break;
+            case GB_BFS_DO: h->runDirOpt(source, o, tp, !out_host); break;
             case GB_BFS_PERSISTENT: h->runPersistent(source, o, tp, out_host); break;
             default: throw Error(GB_ERR_ARG, "unknown BFS variant " + std::to_string(variant));
         }
@@ -322,8 +322,8 @@ int gb_bfs_run_many(gb_bfs* h, int variant, const uint32_t* sources, uint32_t co
                 case GB_BFS_VERTEX: h->runVertex(sources[i], o, nullptr); break;
                 case GB_BFS_NAIVE: h->runNaive(sources[i], o, nullptr); break;
                 case GB_BFS_BINNED: h->runBinned(sources[i], o, nullptr); break;
-                case GB_BFS_EDGE: h->runEdge(sources[i], o, nullptr); break;
-                case GB_BFS_DO: h->runDirOpt(sources[i], o, nullptr); break;
+                case GB_BFS_EDGE: h->runEdge(sources[i], o, nullptr, !out_host); break;
+                case GB_BFS_DO: h->runDirOpt(sources[i], o, nullptr, !out_host); break;
                 default: throw Error(GB_ERR_ARG, "unknown BFS variant " + std::to_string(variant));
             }
             if (out_host) copyDepthsToHost(h, h->dist.get(), h->n, out_host + (uint64_t)i * stride, h->lastLevels);

@@ -55,7 +55,7 @@ __global__ void packDepthsKernel(const uint32_t* d, uint64_t count, uint8_t* out
         else if (FMT == 1) reinterpret_cast<uint2*>(out)[g] = make_uint2(w[0], w[1]);
         else reinterpret_cast<uint4*>(out)[g] = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(overflow, 1u);
+    if (__syncthreads_or(bad) && threadIdx.x == 0) *overflow = 1u;  // may be pinned memory
 }
 
 inline uint32_t widenOne(int fmt, const uint8_t* in, uint64_t i) {
@@ -145,6 +145,12 @@ void enqueuePack(int fmt, const uint32_t* d, uint64_t count, uint8_t* dev, unsig
     GB_LAUNCH_CHECK();
 }
 
+static void addPackEvent(gb_bfs* h) {
+    cudaEvent_t e;
+    GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    h->packEv.push_back(e);
+}
+
 void beginDepths(gb_bfs* h, const uint32_t* d, uint64_t count, uint32_t levels, DepthReturn& r) {
     cudaStream_t st = h->stream.s;
     r.d = d;
@@ -152,21 +158,24 @@ void beginDepths(gb_bfs* h, const uint32_t* d, uint64_t count, uint32_t levels, 
     r.fmt = packFormat(levels);
     if (r.fmt < 0) return;
     const uint64_t bytes = packedBytes(r.fmt, count);
+    h->packHost.ensure(bytes + 16);
+    h->packFlagHost.ensure(1);
+    if (count <= kSmallDepths) {
+        *h->packFlagHost.p = 0;
+        enqueuePack(r.fmt, d, count, h->packHost.p, h->packFlagHost.p, st);
+        while (h->packEv.empty()) addPackEvent(h);
+        GB_CUDA(cudaEventRecord(h->packEv[0], st));
+        return;
+    }
     h->packDev.ensure(bytes + 16);
-    h->packHost.ensure(bytes);
     if (!h->packFlag.get()) {  // zero but after an overflow, which endDepths clears again
         h->packFlag.ensure(1);
         GB_CUDA(cudaMemsetAsync(h->packFlag.get(), 0, 4, st));
     }
-    h->packFlagHost.ensure(1);
     enqueuePack(r.fmt, d, count, h->packDev.get(), h->packFlag.get(), st);
     GB_CUDA(cudaMemcpyAsync(h->packFlagHost.p, h->packFlag.get(), 4, cudaMemcpyDeviceToHost, st));
     const uint64_t chunks = (count + kPackChunk - 1) / kPackChunk;
-    while (h->packEv.size() < chunks) {
-        cudaEvent_t e;
-        GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        h->packEv.push_back(e);
-    }
+    while (h->packEv.size() < chunks) addPackEvent(h);
     for (uint64_t c = 0; c < chunks; ++c) {
         const uint64_t lo = packedBytes(r.fmt, c * kPackChunk), hi = packedBytes(r.fmt, std::min(count, (c + 1) * kPackChunk));
         GB_CUDA(cudaMemcpyAsync(h->packHost.p + lo, h->packDev.get() + lo, hi - lo, cudaMemcpyDeviceToHost, st));

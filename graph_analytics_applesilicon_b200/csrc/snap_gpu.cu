@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kTileThreads) nlPosKernel(const uint8_t* txt, 
         const uint32_t off = vecOffset(blockIdx.x, r, threadIdx.x);
         uint32_t mask = off < len ? newlineMask(txt, off, len) : 0u;
         uint32_t total;
-        uint32_t pos = run + blockScan<kTileThreads>(__popc(mask), &total, sm);
+        uint32_t pos = run + blockScan<kTileThreads>((uint32_t)__popc(mask), &total, sm);
         while (mask) {
             const int j = __ffs(mask) - 1;
             nlPos[pos++] = off + (uint32_t)j;
