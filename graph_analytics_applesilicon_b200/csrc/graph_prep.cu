@@ -177,22 +177,44 @@ __global__ void initIotaKernel(uint32_t* p, uint64_t n) {
 // Keys of a CSR's entries: (map(row) or col-as-row) per mode.
 //   mode 0: (row, col)             mode 1: (col, row)  (transpose)
 //   mode 2: (perm[row], perm[col])  mode 3: (row, col) and (col, row) (symmetrize)
-// out has m (modes 0-2) or 2m (mode 3) keys; warp per row.
+// out has m (modes 0-2) or 2m (mode 3) keys; a warp per row, but rows of more
+// than kLongRow entries are left for the whole block at its end (by a warp, a row
+// of 2M entries takes 2.3 ms).
+constexpr uint32_t kLongRow = 4096, kLongRows = 64;
+
 __global__ void csrKeysKernel(const uint32_t* rp, const uint32_t* ci, uint64_t n, uint64_t m, int b, int mode,
                               const uint32_t* perm, unsigned long long* out) {
+    __shared__ uint32_t longRow[kLongRows], longs;
+    if (threadIdx.x == 0) longs = 0;
+    __syncthreads();
+    auto emit = [&](unsigned long long u, uint32_t i) {
+        const unsigned long long w = ci[i];
+        unsigned long long k;
+        if (mode == 1) k = (w << b) | u;
+        else if (mode == 2) k = ((unsigned long long)perm[u] << b) | perm[w];
+        else k = (u << b) | w;
+        out[i] = k;
+        if (mode == 3) out[m + i] = (w << b) | u;
+    };
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const unsigned lane = threadIdx.x & 31;
     for (uint64_t v = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += nw) {
         const uint32_t s = rp[v], e = rp[v + 1];
-        for (uint32_t i = s + lane; i < e; i += 32) {
-            const unsigned long long u = v, w = ci[i];
-            unsigned long long k;
-            if (mode == 1) k = (w << b) | u;
-            else if (mode == 2) k = ((unsigned long long)perm[u] << b) | perm[w];
-            else k = (u << b) | w;
-            out[i] = k;
-            if (mode == 3) out[m + i] = (w << b) | u;
+        if (e - s > kLongRow) {  // warp-uniform
+            uint32_t slot = 0;
+            if (lane == 0) slot = atomicAdd(&longs, 1u);
+            slot = __shfl_sync(kFull, slot, 0);
+            if (slot < kLongRows) {
+                if (lane == 0) longRow[slot] = (uint32_t)v;
+                continue;
+            }
         }
+        for (uint32_t i = s + lane; i < e; i += 32) emit(v, i);
+    }
+    __syncthreads();
+    for (uint32_t k = 0; k < min(longs, kLongRows); ++k) {
+        const uint32_t v = longRow[k], e = rp[v + 1];
+        for (uint64_t i = (uint64_t)rp[v] + threadIdx.x; i < e; i += blockDim.x) emit(v, (uint32_t)i);
     }
 }
 
