@@ -36,6 +36,8 @@ struct PrArgs {
     const uint32_t* rp;
     const uint32_t* ci;
     const uint32_t* outdeg;
+    const uint32_t* pos;  // adaptive: place of a vertex's contribution, or null (its id)
+    uint32_t hot;         // adaptive: the first `hot` contributions are worth a copy in shared memory
     float* r[2];
     float* contrib[2];
     double* r64[2];
@@ -47,7 +49,7 @@ struct PrArgs {
     float* partF;
     double* partD;
     uint32_t n;
-    float damping, base, invN;
+    float damping, dampingLo, base, invN;
     double base64, invN64, damping64;
     uint32_t lo, hi;  // GS colored: id range of the set
     // split vertices: chunk table, per-hub (first, count), tickets, partials
@@ -88,10 +90,22 @@ struct FF {
     }
 };
 
+__device__ __forceinline__ uint32_t smemAddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
 __device__ __forceinline__ int ldvi(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
 
 __device__ __forceinline__ float prValue(const PrArgs& a, float s, float dang) {
-    return a.base + a.damping * (s + dang * a.invN);  // pr_value, src/shaders/pagerank.metal:45-48
+    // pr_value, src/shaders/pagerank.metal:45-48, with what the float of the damping
+    // factor leaves out (0.85: 2.4e-8) added, so the ranks are not all off the same way
+    const float x = s + dang * a.invN;
+    return fmaf(a.damping, x, fmaf(a.dampingLo, x, a.base));
+}
+
+// The same of a split list's float-float sum, in FP64 and rounded once: the hubs
+// hold most of the ranks' norm.
+__device__ __forceinline__ float prValueSplit(const PrArgs& a, float hi, float lo, const GbPrControl* c) {
+    const double dang = (double)c->dangHi + (double)c->dangLo;
+    return (float)(a.base64 + a.damping64 * ((double)hi + (double)lo + dang * a.invN64));
 }
 
 // Per-thread accumulators of one iteration.
@@ -119,13 +133,14 @@ __device__ __forceinline__ void storeJacobi(const PrArgs& a, int cur, bool withD
 }
 
 // The same with the out-degree and the old rank already loaded (a pull asks for
-// them before its gathers); INPLACE: the contribution goes back to contrib[0],
-// and the dangling mass and residual are left to later kernels.
+// them before its gathers); the contribution's place is `at`.  INPLACE: the
+// contribution goes back to contrib[0], and the dangling mass and residual are
+// left to later kernels.
 template <bool INPLACE>
-__device__ __forceinline__ void storePulled(const PrArgs& a, int cur, bool withDelta, uint32_t v, float val,
+__device__ __forceinline__ void storePulled(const PrArgs& a, int cur, bool withDelta, uint32_t v, uint32_t at, float val,
                                             uint32_t od, float old, IterAcc& acc) {
     a.r[cur ^ 1][v] = val;
-    a.contrib[INPLACE ? 0 : cur ^ 1][v] = od ? val / (float)od : 0.0f;
+    a.contrib[INPLACE ? 0 : cur ^ 1][at] = od ? val / (float)od : 0.0f;
     if (INPLACE) return;
     if (!od) acc.dang.add(val);
     if (withDelta) {
@@ -249,7 +264,7 @@ __global__ void prInitKernel(PrArgs a) {
         if (v < a.n) {
             a.r[0][v] = a.invN;
             const uint32_t od = a.outdeg[v];
-            a.contrib[0][v] = od ? a.invN / (float)od : 0.0f;
+            a.contrib[0][a.pos ? a.pos[v] : v] = od ? a.invN / (float)od : 0.0f;
             if (!od) acc.dang.add(a.invN);
         }
     }
@@ -400,23 +415,16 @@ __device__ __forceinline__ bool splitSum(const PrArgs& a, uint32_t t, uint32_t h
     return true;
 }
 
-// The adaptive pull over the relabeled, padded lists (pr_layout.cu): warp tasks
-// are the chunks of the split lists, then the runs' tasks.  A list's place and
-// length come from its run, and the vertex's out-degree and old rank are
-// requested before the gathers, so a task's chain is vectors, contributions,
-// store.  Two vectors per lane and step (8 gathers in flight).
 // Kahan sum over `count` vectors at p, p + step, ...
-template <bool COHERENT>
-__device__ __forceinline__ Kahan gatherVecs(const uint4* p, uint32_t count, uint32_t step, const float* contrib) {
+template <class Gather>
+__device__ __forceinline__ Kahan gatherVecs(const uint4* p, uint32_t count, uint32_t step, Gather at) {
     Kahan k;
     for (uint32_t i = 0; i < count; i += 2, p += 2 * step) {
         const bool two = i + 1 < count;
         const uint4 q = ldStream4(reinterpret_cast<const uint32_t*>(p));
         const uint4 r = two ? ldStream4(reinterpret_cast<const uint32_t*>(p + step)) : make_uint4(0, 0, 0, 0);
-        const float a0 = ldContrib<COHERENT>(contrib + q.x), a1 = ldContrib<COHERENT>(contrib + q.y);
-        const float a2 = ldContrib<COHERENT>(contrib + q.z), a3 = ldContrib<COHERENT>(contrib + q.w);
-        const float b0 = two ? ldContrib<COHERENT>(contrib + r.x) : 0.f, b1 = two ? ldContrib<COHERENT>(contrib + r.y) : 0.f;
-        const float b2 = two ? ldContrib<COHERENT>(contrib + r.z) : 0.f, b3 = two ? ldContrib<COHERENT>(contrib + r.w) : 0.f;
+        const float a0 = at(q.x, true), a1 = at(q.y, true), a2 = at(q.z, true), a3 = at(q.w, true);
+        const float b0 = at(r.x, two), b1 = at(r.y, two), b2 = at(r.z, two), b3 = at(r.w, two);
         k.add(a0);
         k.add(a1);
         k.add(a2);
@@ -431,11 +439,37 @@ __device__ __forceinline__ Kahan gatherVecs(const uint4* p, uint32_t count, uint
     return k;
 }
 
-// Bound by the rate of random 4-byte gathers: Chung-Lu, 233M entries, 816 us a
-// sweep = 285 G/s (1,047 with row pointers and ragged lists); web graph, 5M,
-// 34 us (48.7); R-MAT 18, 4M, 22 us (31).  56 registers, 36 warps per SM: capped
-// at 48 the sweeps take 836 / 34 / 22.4 us, at 40 883 / 38 / 26.
-template <bool INPLACE>
+// Contribution i: from the copy of the first `hot` at shared address `copy`, the
+// others from memory; predicated, so that a warp's lanes of either kind take one
+// instruction each and the next gather need not wait.
+__device__ __forceinline__ float ldHot(const float* contrib, uint32_t copy, uint32_t hot, uint32_t i, bool want) {
+    float x;
+    asm volatile(
+        "{\n\t.reg .pred w, s, g;\n\t"
+        "setp.ne.u32 w, %5, 0;\n\t"
+        "setp.lt.and.u32 s, %1, %2, w;\n\t"
+        "setp.ge.and.u32 g, %1, %2, w;\n\t"
+        "mov.f32 %0, 0f00000000;\n\t"
+        "@s ld.shared.f32 %0, [%3];\n\t"
+        "@g ld.global.nc.L1::no_allocate.f32 %0, [%4];\n\t}"
+        : "=f"(x)
+        : "r"(i), "r"(hot), "r"(copy + 4 * i), "l"(contrib + i), "r"((unsigned)want));
+    return x;
+}
+
+// The adaptive pull over the relabeled, padded lists (pr_layout.cu): warp tasks
+// are the chunks of the split lists, then the runs' tasks.  A list's place and
+// length come from its run, and the vertex's out-degree and old rank are
+// requested before the gathers, so a task's chain is vectors, contributions,
+// store.  Two vectors per lane and step (8 gathers in flight).  HOT: the first
+// a.hot contributions are copied to shared memory first (pr_layout.cu: which).
+// Bound by what the L2 can return for random 4-byte gathers, a 32-byte sector
+// each: 285 G/s without HOT.  Us a sweep: Chung-Lu, 233M entries, 711 (816 without
+// HOT; 1,047 with row pointers and ragged lists); web graph, 5M, 34 (48.7); R-MAT
+// 18, 4M, 22 (31).  56 registers, 36 warps per SM: capped at 48 the sweeps take
+// 836 / 34 / 22.4 us, at 40 883 / 38 / 26 (without HOT).  Requesting the next
+// task's vectors during a task's gathers changes nothing.
+template <bool INPLACE, bool HOT>
 __global__ void __maxnreg__(56) prAdaptiveKernel(PrArgs a, const uint4* __restrict__ vecs, const GbPrRun* __restrict__ runs,
                                  uint32_t nRuns, uint32_t nRunTasks) {
     const GbPrControl* c = a.ctl;
@@ -446,8 +480,21 @@ __global__ void __maxnreg__(56) prAdaptiveKernel(PrArgs a, const uint4* __restri
     const float* contrib = INPLACE ? a.contrib[0] : a.contrib[cur];
     const float* rOld = a.r[cur];
     IterAcc acc;
-    auto store = [&](uint32_t v, float s, uint32_t od, float old) {
-        storePulled<INPLACE>(a, cur, withDelta, v, prValue(a, s, dang), od, old, acc);
+    auto store = [&](uint32_t v, uint32_t at, float val, uint32_t od, float old) {
+        storePulled<INPLACE>(a, cur, withDelta, v, at, val, od, old, acc);
+    };
+    extern __shared__ float4 hotCopy[];
+    const uint32_t copy = HOT ? smemAddr(hotCopy) : 0u;
+    if (HOT) {  // a.hot is a multiple of 4
+        const float4* from = reinterpret_cast<const float4*>(contrib);
+        for (uint32_t i = threadIdx.x; i < a.hot / 4; i += blockDim.x)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(copy + 16 * i), "l"(from + i) : "memory");
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+    }
+    auto gather = [&](uint32_t i, bool want) {
+        if (HOT) return ldHot(contrib, copy, a.hot, i, want);
+        return want ? ldContrib<INPLACE>(contrib + i) : 0.f;
     };
     const unsigned lane = laneId();
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5, total = a.nChunks + nRunTasks;
@@ -455,10 +502,10 @@ __global__ void __maxnreg__(56) prAdaptiveKernel(PrArgs a, const uint4* __restri
     for (; t < a.nChunks; t += nwarps) {  // warp-uniform
         const uint4 h = a.chunks[t];  // vertex, first vector, end vector, hub
         const uint32_t first = a.hubFirst[2 * h.w], cnt = a.hubFirst[2 * h.w + 1];
-        const Kahan k = gatherVecs<INPLACE>(vecs + h.y + lane, h.y + lane < h.z ? (h.z - h.y - lane + 31) / 32 : 0u, 32, contrib);
+        const Kahan k = gatherVecs(vecs + h.y + lane, h.y + lane < h.z ? (h.z - h.y - lane + 31) / 32 : 0u, 32, gather);
         FF f;
         if (splitSum(a, t, h.w, first, cnt, k, f) && lane == 0)
-            store(h.x, f.hi + f.lo, a.outdeg[h.x], withDelta ? rOld[h.x] : 0.f);
+            store(h.x, a.pos ? a.pos[h.x] : h.x, prValueSplit(a, f.hi, f.lo, c), a.outdeg[h.x], withDelta ? rOld[h.x] : 0.f);
     }
     GbPrRun r{};
     uint32_t end = 0;  // first task beyond run r
@@ -477,13 +524,13 @@ __global__ void __maxnreg__(56) prAdaptiveKernel(PrArgs a, const uint4* __restri
         const unsigned G = 1u << r.lg, sub = lane & (G - 1);
         const uint32_t idx = (rt - r.task0) * (32u >> r.lg) + (lane >> r.lg), v = r.v0 + idx;
         const bool active = v < r.vEnd, lead = active && sub == 0;
-        const uint32_t od = lead ? a.outdeg[v] : 0u;
+        const uint32_t od = lead ? a.outdeg[v] : 0u, at = lead && a.pos ? a.pos[v] : v;
         const float old = lead && withDelta ? rOld[v] : 0.f;
         const uint4* p = vecs + r.e0 + (r.inter ? (uint64_t)(rt - r.task0) * 32 * r.vecs + lane : (uint64_t)idx * r.vecs + sub);
         const uint32_t count = active && sub < r.vecs ? (r.vecs - sub + G - 1) >> r.lg : 0u;
-        float s = gatherVecs<INPLACE>(p, count, r.inter ? 32 : G, contrib).sum;
+        float s = gatherVecs(p, count, r.inter ? 32 : G, gather).sum;
         for (unsigned o = G >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-        if (lead) store(v, s, od, old);
+        if (lead) store(v, at, prValue(a, s, dang), od, old);
     }
     if (!INPLACE) finishBlock<0>(a, acc);
 }
@@ -503,8 +550,8 @@ __global__ void prGroupKernel(PrArgs a, uint32_t lg, uint32_t splitMin) {
     const bool withDelta = !INPLACE && c->withDelta;
     const float* contrib = INPLACE ? a.contrib[0] : a.contrib[cur];
     IterAcc acc;
-    auto store = [&](uint32_t v, float s, uint32_t od, float old) {
-        storePulled<INPLACE>(a, cur, withDelta, v, prValue(a, s, dang), od, old, acc);
+    auto store = [&](uint32_t v, float val, uint32_t od, float old) {
+        storePulled<INPLACE>(a, cur, withDelta, v, v, val, od, old, acc);
     };
     const unsigned lane = laneId(), G = 1u << lg, sub = lane & (G - 1);
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -516,7 +563,7 @@ __global__ void prGroupKernel(PrArgs a, uint32_t lg, uint32_t splitMin) {
         const Kahan k = gatherKahan<INPLACE>(a.ci, contrib, h.y, h.z, lane, 32);
         FF f;
         if (splitSum(a, (uint32_t)t, h.w, first, cnt, k, f) && lane == 0)
-            store(h.x, f.hi + f.lo, a.outdeg[h.x], withDelta ? a.r[cur][h.x] : 0.f);
+            store(h.x, prValueSplit(a, f.hi, f.lo, c), a.outdeg[h.x], withDelta ? a.r[cur][h.x] : 0.f);
     }
     for (; t < total; t += nwarps) {
         const uint64_t v = (t - a.nChunks) * (32u >> lg) + (lane >> lg);
@@ -527,7 +574,7 @@ __global__ void prGroupKernel(PrArgs a, uint32_t lg, uint32_t splitMin) {
         const float old = lead && withDelta ? a.r[cur][v] : 0.f;
         float s = mine ? gatherGroup<INPLACE>(a.ci, contrib, b, e, sub, G) : 0.f;
         for (unsigned o = G >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-        if (lead) store((uint32_t)v, s, od, old);
+        if (lead) store((uint32_t)v, prValue(a, s, dang), od, old);
     }
     if (!INPLACE) finishBlock<0>(a, acc);
 }
@@ -623,7 +670,7 @@ __global__ void gsContribKernel(PrArgs a) {
         if (v < a.n) {
             const float r = a.r[cur][v];
             const uint32_t od = a.outdeg[v];
-            a.contrib[0][v] = od ? r / (float)od : 0.0f;
+            a.contrib[0][a.pos ? a.pos[v] : v] = od ? r / (float)od : 0.0f;
             if (!od) acc.dang.add(r);
         }
     }
@@ -761,7 +808,6 @@ struct BlkArgs {
     unsigned long long spinLimit;
 };
 
-__device__ __forceinline__ uint32_t smemAddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Waits for the given phase parity of an mbarrier; gives up after `limit` polls.
 __device__ __forceinline__ bool blkWait(unsigned long long* mbar, uint32_t parity, unsigned long long limit) {
@@ -1090,6 +1136,23 @@ static size_t blkSmemBytes() {
     return bytes;
 }
 
+// Whether an adaptive iteration keeps the most-gathered contributions in shared
+// memory: blocks of 1,024 threads, one per SM, so it needs tasks for all of them.
+constexpr int kHotThreads = 1024;
+
+static bool hotFits(const gb_pr& h) {
+    return h.hotA && (uint64_t)h.nChunks + h.nRunTasks >= (uint64_t)deviceSmCount() * (kHotThreads / 32);
+}
+
+static void raiseHotLimit() {
+    static const bool raised = [] {
+        GB_CUDA(cudaFuncSetAttribute(prAdaptiveKernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(kPrHotMax * sizeof(float))));
+        return true;
+    }();
+    (void)raised;
+}
+
 // Enqueue one iteration of `variant` on the handle's stream (capturable).
 static void enqueueIteration(gb_pr& h, int v, const gb_pr_options& o, PrArgs& a, PrArgs& ag) {
     const uint32_t tg = o.tg;
@@ -1123,8 +1186,10 @@ static void enqueueIteration(gb_pr& h, int v, const gb_pr_options& o, PrArgs& a,
     } else if (!inplace) {
         if (v == GB_PR_PULL_SCALAR || v == GB_PR_PULL_VECTOR)
             prGroupKernel<false><<<residentGrid(prGroupKernel<false>, groupWork, tg), tg, 0, s>>>(grouped(a), sp.lg, sp.splitMin);
+        else if (hotFits(h))
+            prAdaptiveKernel<false, true><<<deviceSmCount(), kHotThreads, h.hotA * sizeof(float), s>>>(ag, h.vecA.get(), h.runsA.get(), h.nRuns, h.nRunTasks);
         else
-            prAdaptiveKernel<false><<<residentGrid(prAdaptiveKernel<false>, adaptiveWork, tg), tg, 0, s>>>(ag, h.vecA.get(), h.runsA.get(), h.nRuns, h.nRunTasks);
+            prAdaptiveKernel<false, false><<<residentGrid(prAdaptiveKernel<false, false>, adaptiveWork, tg), tg, 0, s>>>(ag, h.vecA.get(), h.runsA.get(), h.nRuns, h.nRunTasks);
     } else {
         const bool colored = v == GB_PR_PULL_GS && h.gsColored;
         PrArgs& w = (colored || v == GB_PR_PULL_ADAPTIVE) ? ag : a;
@@ -1185,7 +1250,7 @@ static void enqueueIteration(gb_pr& h, int v, const gb_pr_options& o, PrArgs& a,
         } else if (v == GB_PR_PULL_SCALAR || v == GB_PR_PULL_VECTOR) {
             prGroupKernel<true><<<residentGrid(prGroupKernel<true>, groupWork, tg), tg, 0, s>>>(grouped(w), sp.lg, sp.splitMin);
         } else {
-            prAdaptiveKernel<true><<<residentGrid(prAdaptiveKernel<true>, adaptiveWork, tg), tg, 0, s>>>(w, h.vecA.get(), h.runsA.get(), h.nRuns, h.nRunTasks);
+            prAdaptiveKernel<true, false><<<residentGrid(prAdaptiveKernel<true, false>, adaptiveWork, tg), tg, 0, s>>>(w, h.vecA.get(), h.runsA.get(), h.nRuns, h.nRunTasks);
         }
         prSumKernel<<<gN, 256, 0, s>>>(w);
         prScaleKernel<<<gN, 256, 0, s>>>(w);
@@ -1200,7 +1265,10 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
     if (v == GB_PR_PUSH && !hasOut) throw Error(GB_ERR_ARG, "gpu_push needs the out-CSR");
     if (v != GB_PR_PUSH && !hasIn) throw Error(GB_ERR_ARG, "pull variants need the in-CSR");
     if (o.iters < 0) throw Error(GB_ERR_ARG, "iters must be >= 0");
-    if (v == GB_PR_PULL_ADAPTIVE) prepareAdaptive(o.small_max, o.large_min);
+    if (v == GB_PR_PULL_ADAPTIVE) {
+        prepareAdaptive(o.small_max, o.large_min);
+        raiseHotLimit();  // before any capture
+    }
     if (v == GB_PR_PULL_SCALAR || v == GB_PR_PULL_VECTOR) prepareSplit(v == GB_PR_PULL_VECTOR);
     if (v == GB_PR_PULL_GS && !gsReady) prepareGS(2);
     if (v == GB_PR_PULL_BLOCKED) {
@@ -1236,20 +1304,23 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
     c.tolRel = o.tol_rel;
     PrArgs a = makeArgs(*this, false);
     a.damping = o.damping;
-    a.base = (1.0f - o.damping) / (float)n;
     a.invN = 1.0f / (float)n;
-    // The FP64 variant uses the decimal value the float option was written as
-    // (0.85f -> 0.85), as the double-precision CPU reference does.
+    // The decimal value the float option was written as (0.85f -> 0.85), as in the
+    // double-precision CPU reference.
     {
         char buf[32];
         std::snprintf(buf, sizeof buf, "%.7g", (double)o.damping);
         a.damping64 = std::strtod(buf, nullptr);
     }
     a.base64 = (1.0 - a.damping64) / (double)n;
+    a.base = (float)a.base64;
+    a.dampingLo = (float)(a.damping64 - (double)o.damping);
     a.invN64 = 1.0 / (double)n;
     PrArgs ag = a;
     if (v == GB_PR_PULL_ADAPTIVE) {  // hub-first relabeled layout
         ag.outdeg = outdegA.get();
+        ag.pos = hotA ? posA.get() : nullptr;
+        ag.hot = hotA;
         ag.chunks = hubChunks.get();
         ag.hubFirst = hubFirst.get();
         ag.hubDone = hubDone.get();

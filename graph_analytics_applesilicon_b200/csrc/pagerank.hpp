@@ -54,6 +54,11 @@ constexpr int kBlkConsumerWarps = kBlkThreads / 32 - 1;
 constexpr uint32_t kBlkChunk = kBlkConsumerWarps * 32;  // one 16-byte word per consumer thread
 constexpr uint32_t kBlkHub = 4096;  // rows with this many in-edges are summed apart, one block each
 
+// Contributions an adaptive sweep keeps in shared memory, at most (128 KB): more
+// leave the L1 too little room for the gathers in flight (Chung-Lu, 233M entries:
+// 24K 736 us a sweep, 32K 717, 40K 710, 48K 793, 56K 1,390; none 820).
+constexpr uint32_t kPrHotMax = 32u * 1024u;
+
 // A run of the adaptive layout: vertices [v0, vEnd), all with lists of `vecs`
 // vectors, handled by groups of 1 << lg lanes.  Lists follow one another from
 // vector e0 on; `inter`: in blocks of 32 lists with vector k of the 32 lists
@@ -81,6 +86,8 @@ struct gb_pr {
     // run per padded length, so a list's place follows from its id
     gb::DevBuf<uint4> vecA;          // the lists
     gb::DevBuf<uint32_t> outdegA;    // by new id
+    gb::DevBuf<uint32_t> posA;       // by new id: place of its contribution (with hotA > 0)
+    uint32_t hotA = 0;               // contributions worth a copy in shared memory; theirs are places [0, hotA)
     gb::DevBuf<uint32_t> permADev;   // old id -> new id
     gb::DevBuf<GbPrRun> runsA;
     uint32_t nRuns = 0, nRunTasks = 0;

@@ -23,6 +23,17 @@ namespace gb {
 namespace {
 
 constexpr uint32_t kPrInterVecs = 8;   // longest interleaved list, in vectors
+// An adaptive sweep of a large graph keeps the contributions that are gathered
+// most in shared memory, whose gathers cost the L1 and the L2 nothing.  A place
+// costs each SM 4 bytes of copying per sweep, as long as some 28 gathers
+// elsewhere on the GPU, so a vertex needs this out-degree to be worth one; and
+// the copying and the one block per SM it leaves room for need a sweep of this
+// many entries to pay (us a sweep without / with: Chung-Lu of 3M entries 19.1 /
+// 23.7, 9M 38.9 / 39.9, 30M 109 / 109, 76M 277 / 223; R-MAT of 4M 22.2 / 23.1,
+// 17M 56.4 / 48.4, 34M 123 / 98).
+constexpr uint64_t kPrHotEntries = 12ull << 20;
+constexpr uint32_t kPrHotMin = 32;
+constexpr uint32_t kPrHotBins = 1u << 14;
 constexpr uint32_t kPrLaneVecs = 4;    // vectors per lane a group is sized for
 
 // Vectors per chunk of a split list: as many as leave each of the GPU's warps
@@ -48,40 +59,38 @@ __global__ void orderedDegreesKernel(const uint32_t* __restrict__ rp, const uint
         deg[i] = rp[order[i] + 1] - rp[order[i]];
 }
 
-// Sorted keys to padded lists, a warp per list: row i's entries are the sorted
+// Sorted keys to padded lists, a block per split list (by a warp, a list of 2M
+// entries takes 1.7 ms), a warp per other list: row i's entries are the sorted
 // keys [start[i], start[i + 1]).  Runs are found by their first vertex; the
 // split lists' run (run 0 when hubs > 0) gives each list its own place.
 __global__ void fillListsKernel(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ start,
                                 uint64_t n, unsigned long long mask, const GbPrRun* __restrict__ runs, uint32_t nRuns,
-                                uint32_t hubs, const uint32_t* __restrict__ hubVec, uint32_t* out) {
+                                uint32_t hubs, const uint32_t* __restrict__ hubVec, const uint32_t* __restrict__ pos,
+                                uint32_t pad, uint32_t* out) {
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const unsigned lane = threadIdx.x & 31;
-    for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
+    auto entry = [&](uint32_t s, uint32_t d, uint32_t k) {
+        if (k >= d) return pad;
+        const uint32_t u = (uint32_t)(keys[s + k] & mask);
+        return pos ? pos[u] : u;
+    };
+    for (uint32_t i = blockIdx.x; i < hubs; i += gridDim.x) {
         const uint32_t s = start[i], d = start[i + 1] - s;
-        uint64_t base;       // first entry
-        uint32_t vecs, step = 4;  // entries from one vector to the next
-        if (i < hubs) {
-            base = 4ull * hubVec[i];
-            vecs = (d + 3) / 4;
-        } else {
-            uint32_t lo = 0, hi = nRuns - 1;
-            while (lo < hi) {  // last run with v0 <= i
-                const uint32_t mid = (lo + hi + 1) / 2;
-                if (runs[mid].v0 <= i) lo = mid;
-                else hi = mid - 1;
-            }
-            const GbPrRun r = runs[lo];
-            const uint32_t idx = (uint32_t)i - r.v0;
-            vecs = r.vecs;
-            if (r.inter) {
-                base = 4ull * (r.e0 + (uint64_t)(idx / 32) * 32 * vecs + idx % 32);
-                step = 128;
-            } else {
-                base = 4ull * (r.e0 + (uint64_t)idx * vecs);
-            }
+        uint32_t* to = out + 4ull * hubVec[i];
+        for (uint32_t k = threadIdx.x; k < (d + 3) / 4 * 4; k += blockDim.x) to[k] = entry(s, d, k);
+    }
+    for (uint64_t i = hubs + (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n; i += nw) {
+        const uint32_t s = start[i], d = start[i + 1] - s;
+        uint32_t lo = 0, hi = nRuns - 1;
+        while (lo < hi) {  // last run with v0 <= i
+            const uint32_t mid = (lo + hi + 1) / 2;
+            if (runs[mid].v0 <= i) lo = mid;
+            else hi = mid - 1;
         }
-        for (uint32_t k = lane; k < 4 * vecs; k += 32)
-            out[base + (uint64_t)(k / 4) * step + k % 4] = k < d ? (uint32_t)(keys[s + k] & mask) : (uint32_t)n;
+        const GbPrRun r = runs[lo];
+        const uint32_t idx = (uint32_t)i - r.v0, step = r.inter ? 128 : 4;  // entries from one vector to the next
+        uint32_t* to = out + 4ull * (r.e0 + (r.inter ? (uint64_t)(idx / 32) * 32 * r.vecs + idx % 32 : (uint64_t)idx * r.vecs));
+        for (uint32_t k = lane; k < 4 * r.vecs; k += 32) to[(uint64_t)(k / 4) * step + k % 4] = entry(s, d, k);
     }
 }
 
@@ -111,6 +120,27 @@ __global__ void fillSplitKernel(const uint32_t* __restrict__ rp, uint64_t n, uin
     }
 }
 
+// bins[d] += vertices of out-degree d, for d >= kPrHotMin; the last bin takes all beyond.
+__global__ void outdegreeBinsKernel(const uint32_t* __restrict__ outdeg, uint64_t n, uint32_t* bins) {
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
+        if (outdeg[v] >= kPrHotMin) atomicAdd(&bins[min(outdeg[v], kPrHotBins - 1)], 1u);
+}
+
+// Places of the contributions: the vertices of out-degree [lo, hi) get the first
+// free of the `hot` first places while there are any, all others (first launch)
+// the place hot + v.
+__global__ void hotPlacesKernel(const uint32_t* __restrict__ outdeg, uint64_t n, uint32_t lo, uint32_t hi, uint32_t hot,
+                                bool first, uint32_t* taken, uint32_t* pos) {
+    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t v = base + threadIdx.x;
+        const uint32_t d = v < n ? outdeg[v] : 0u;
+        const bool in = v < n && d >= lo && d < hi;
+        const uint32_t slot = warpAppend(in, taken);
+        if (in && slot < hot) pos[v] = slot;
+        else if (v < n && first) pos[v] = hot + (uint32_t)v;
+    }
+}
+
 template <class T>
 void upload(DevBuf<T>& buf, const std::vector<T>& v, cudaStream_t st) {
     buf.ensure(v.size() + 1);
@@ -123,6 +153,44 @@ uint32_t groupLog2(uint32_t d, uint32_t vecs, uint32_t smallMax, uint32_t largeM
     uint32_t lg = 1;
     while (lg < 5 && (kPrLaneVecs << lg) < vecs) ++lg;
     return lg;
+}
+
+// Chooses the contributions to keep in shared memory (h.hotA of them, 0 when they
+// are too few of the gathers to matter) and every contribution's place.
+void choosePlaces(gb_pr& h, cudaStream_t st) {
+    const uint64_t n = h.n;
+    h.hotA = 0;
+    if (h.mIn < kPrHotEntries || n + kPrHotMax + 4 >= (1ull << 32)) return;
+    DevBuf<uint32_t> bins;
+    std::vector<uint32_t> count(kPrHotBins);
+    bins.ensure(kPrHotBins);
+    GB_CUDA(cudaMemsetAsync(bins.get(), 0, kPrHotBins * 4, st));
+    outdegreeBinsKernel<<<prepGrid(n, 256), 256, 0, st>>>(h.outdegA.get(), n, bins.get());
+    GB_LAUNCH_CHECK();
+    GB_CUDA(cudaMemcpyAsync(count.data(), bins.get(), kPrHotBins * 4, cudaMemcpyDeviceToHost, st));
+    GB_CUDA(cudaStreamSynchronize(st));
+    // from the largest down: all of out-degree above `cut`, of `cut` as many as there is room for
+    uint64_t taken = 0, gathers = 0;
+    uint32_t cut = kPrHotBins - 1;
+    for (;; --cut) {
+        const uint64_t room = std::min<uint64_t>(count[cut], kPrHotMax - taken);
+        taken += room;
+        gathers += room * cut;
+        if (taken == kPrHotMax || cut == kPrHotMin) break;
+    }
+    if (gathers < h.mIn / 8) return;
+    const uint32_t hot = (uint32_t)((taken + 3) / 4 * 4);
+    for (auto& c : h.contrib) {
+        c.ensure(n + hot + 4);
+        GB_CUDA(cudaMemsetAsync(c.get() + n + hot, 0, 16, st));
+    }
+    h.posA.ensure(n);
+    GB_CUDA(cudaMemsetAsync(bins.get(), 0, 4, st));
+    hotPlacesKernel<<<prepGrid(n, 256), 256, 0, st>>>(h.outdegA.get(), n, cut + 1, 0xFFFFFFFFu, hot, true, bins.get(), h.posA.get());
+    GB_LAUNCH_CHECK();
+    hotPlacesKernel<<<prepGrid(n, 256), 256, 0, st>>>(h.outdegA.get(), n, cut, cut + 1, hot, false, bins.get(), h.posA.get());
+    GB_LAUNCH_CHECK();
+    h.hotA = hot;
 }
 
 }  // namespace
@@ -150,6 +218,8 @@ void gb_pr::prepareAdaptive(uint32_t smallMax, uint32_t largeMin) {
     outdegA.ensure(n);
     gatherU32Kernel<<<prepGrid(n, 256), 256, 0, st>>>(outdeg.get(), order.get(), n, outdegA.get());
     GB_LAUNCH_CHECK();
+
+    choosePlaces(*this, st);
 
     // how many vertices have each in-degree, from which the hubs and runs follow
     uint32_t longest = 0;
@@ -213,8 +283,8 @@ void gb_pr::prepareAdaptive(uint32_t smallMax, uint32_t largeMin) {
         permutedKeys(rowIn.get(), colIn.get(), n, mIn, b, permADev.get(), keys.get(), st);
         radixSortKeys(keys, tmp, mIn, 2 * b, sc, st);
         fillListsKernel<<<prepGrid(n * 32, 256), 256, 0, st>>>(keys.get(), start.get(), n, (1ull << b) - 1, runsA.get(),
-                                                               nRuns, nHubs, dHubVec.get(),
-                                                               reinterpret_cast<uint32_t*>(vecA.get()));
+                                                               nRuns, nHubs, dHubVec.get(), hotA ? posA.get() : nullptr,
+                                                               (uint32_t)n + hotA, reinterpret_cast<uint32_t*>(vecA.get()));
         GB_LAUNCH_CHECK();
     }
     GB_CUDA(cudaStreamSynchronize(st));
