@@ -64,8 +64,12 @@ void endDepths(gb_bfs* h, const DepthReturn& r, uint32_t levels, uint32_t* out);
 // back into uint32 on the host.
 int packFormat(uint32_t levels);
 uint64_t packedBytes(int fmt, uint64_t count);
-void enqueuePack(int fmt, const uint32_t* d, uint64_t count, uint8_t* dev, unsigned* overflow, cudaStream_t st);
+// Several rows (count apart in d, `pitch` bytes apart when packed, stride apart in
+// out) go through one launch and one widening.
+void enqueuePack(int fmt, const uint32_t* d, uint64_t count, uint8_t* dev, unsigned* overflow, cudaStream_t st,
+                 uint32_t rows = 1, uint64_t pitch = 0);
 void widenPacked(int fmt, const uint8_t* in, uint64_t count, uint32_t* out);
+void widenRows(int fmt, const uint8_t* in, uint64_t pitch, uint32_t rows, uint64_t count, uint32_t* out, uint64_t stride);
 // Depth arrays up to this size are packed straight into pinned host memory, by
 // the traversal's kernel or one after it; larger ones into device memory, and
 // copied in chunks that the widening overlaps.
@@ -127,6 +131,8 @@ struct gb_bfs {
     gb::DevBuf<uint32_t> bActive[2], bCand, bHubV[2];
     gb::DevBuf<unsigned long long> bHubOff[2];
     gb::DevBuf<uint32_t> bDist;          // k * n results
+    gb::DevBuf<uint32_t> bSrc;           // the sources
+    gb::DevBuf<unsigned long long> bCtr; // level counters
     gb::DevBuf<uint2> bDefer;            // bottom-up: lists whose rest a whole block scans
     int bGrid = 0, bBlock = 0, bMax = 0;
 

@@ -843,12 +843,10 @@ void gb_bfs::ensureBatch(const gb_bfs_options& o, int k) {
 }
 
 // gb_bfs_run_many for the batched kernel: one launch per group of up to 64
-// sources, then every row of the group returned to the host as the single-
-// source path does (packed to the width the batch's level count allows,
-// copied on the copy stream, widened by host threads) through a ring of
-// kRowRing buffers, so row j + 1's pack and copy overlap row j's widening.
-// The pack kernel checks every depth against the width; a row that does not
-// fit is copied whole.  gpu_ms[i]: the group's launch time shared evenly over
+// sources, then every row of the group returned to the host (returnRows), packed
+// to the width the batch's level count allows and widened by host threads.  The
+// pack kernel checks every depth against the width; rows that do not fit are
+// copied whole.  gpu_ms[i]: the group's launch time shared evenly over
 // its sources; levels[i]: the group's level count.  Without out the last
 // source's depths are left in the handle's depth buffer.
 void gb_bfs::runBatchMany(const uint32_t* src, uint32_t count, uint32_t* out, uint64_t stride,
@@ -872,53 +870,49 @@ void gb_bfs::runBatchMany(const uint32_t* src, uint32_t count, uint32_t* out, ui
     GB_CUDA(cudaStreamSynchronize(copyStream.s));
 }
 
-// The rows of the last batch to the host; the ring is described above.
+// The rows of the last batch to the host, in groups of about kRowGroup packed
+// bytes: a launch packs a group straight into one of kRowRing pinned buffers, and
+// the host widens it while the next groups are packed.  64 rows of 300,000
+// vertices took a memset, a launch, two copies, two events and a wait each: 1.1 ms
+// of calls beside a widening of 0.6 ms (1,417 us the call, 887 so).
 void gb_bfs::returnRows(uint32_t k, uint32_t* out, uint64_t stride) {
     constexpr uint32_t kRowRing = 4;
+    constexpr uint64_t kRowGroup = 1u << 20;
     static_assert(kRowRing <= kManySlots, "row ring exceeds the handle's pack buffers");
-    for (uint32_t b = 0; b < kRowRing; ++b) {
-        mPackDev[b].ensure(2 * n + 16);
-        mPackHost[b].ensure(2 * n + 16);
-    }
-    mFlag.ensure(kManySlots);
-    mFlagHost.ensure(64);
-    while (mSlotEv.size() < 3 * (size_t)kManySlots + 1 + kMaxInFlight) {
-        cudaEvent_t e;
-        GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        mSlotEv.push_back(e);
-    }
-    cudaStream_t cs = copyStream.s;
     const int fmt = packFormat(lastLevels);
     if (fmt < 0) {
         for (uint32_t j = 0; j < k; ++j)
             staged.run(bDist.get() + (uint64_t)j * n, n * 4, out + (uint64_t)j * stride, stream.s);
         return;
     }
-    auto enqueue = [&](uint32_t j) {
-        const uint32_t b = j % kRowRing;
-        cudaEvent_t packed = mSlotEv[b], copied = mSlotEv[kManySlots + b];
-        GB_CUDA(cudaMemsetAsync(mFlag.get() + b, 0, sizeof(unsigned), stream.s));
-        enqueuePack(fmt, bDist.get() + (uint64_t)j * n, n, mPackDev[b].get(), mFlag.get() + b, stream.s);
-        GB_CUDA(cudaEventRecord(packed, stream.s));
-        GB_CUDA(cudaStreamWaitEvent(cs, packed, 0));
-        GB_CUDA(cudaMemcpyAsync(mPackHost[b].p, mPackDev[b].get(), packedBytes(fmt, n), cudaMemcpyDeviceToHost, cs));
-        GB_CUDA(cudaMemcpyAsync(mFlagHost.p + j, mFlag.get() + b, sizeof(unsigned), cudaMemcpyDeviceToHost, cs));
-        GB_CUDA(cudaEventRecord(copied, cs));
+    const uint64_t pitch = (packedBytes(fmt, n) + 16 + 15) / 16 * 16;
+    const uint32_t per = (uint32_t)std::min<uint64_t>(k, std::max<uint64_t>(1, kRowGroup / pitch)), groups = (k + per - 1) / per;
+    for (uint32_t b = 0; b < std::min(kRowRing, groups); ++b) mPackHost[b].ensure(per * pitch);
+    mFlagHost.ensure(64);
+    std::fill(mFlagHost.p, mFlagHost.p + groups, 0u);
+    while (mSlotEv.size() < 3 * (size_t)kManySlots + 1 + kMaxInFlight) {
+        cudaEvent_t e;
+        GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        mSlotEv.push_back(e);
+    }
+    auto rows = [&](uint32_t g) { return std::min(per, k - g * per); };
+    auto enqueue = [&](uint32_t g) {
+        enqueuePack(fmt, bDist.get() + (uint64_t)g * per * n, n, mPackHost[g % kRowRing].p, mFlagHost.p + g, stream.s,
+                    rows(g), pitch);
+        GB_CUDA(cudaEventRecord(mSlotEv[g % kRowRing], stream.s));
     };
-    // buffer b is packed again only after the host has widened its last row
-    // (the host enqueues row j + kRowRing after widening row j)
+    // buffer b is packed again only after the host has widened its last group
     uint32_t queued = 0;
-    for (; queued < k && queued < kRowRing; ++queued) enqueue(queued);
-    for (uint32_t j = 0; j < k; ++j) {
-        const uint32_t b = j % kRowRing;
-        GB_CUDA(cudaEventSynchronize(mSlotEv[kManySlots + b]));
-        uint32_t* dst = out + (uint64_t)j * stride;
-        if (mFlagHost.p[j] == 0) {
-            widenPacked(fmt, mPackHost[b].p, n, dst);
-        } else {  // a depth did not fit the width: the row is still intact on the device
-            staged.run(bDist.get() + (uint64_t)j * n, n * 4, dst, cs);
-        }
-        if (queued < k) enqueue(queued++);
+    for (; queued < groups && queued < kRowRing; ++queued) enqueue(queued);
+    for (uint32_t g = 0; g < groups; ++g) {
+        GB_CUDA(cudaEventSynchronize(mSlotEv[g % kRowRing]));
+        uint32_t* dst = out + (uint64_t)g * per * stride;
+        if (*const_cast<volatile unsigned*>(mFlagHost.p + g) == 0)
+            widenRows(fmt, mPackHost[g % kRowRing].p, pitch, rows(g), n, dst, stride);
+        else  // a depth did not fit the width: the rows are still intact on the device
+            for (uint32_t r = 0; r < rows(g); ++r)
+                staged.run(bDist.get() + ((uint64_t)g * per + r) * n, n * 4, dst + r * stride, copyStream.s);
+        if (queued < groups) enqueue(queued++);
     }
 }
 
@@ -934,13 +928,12 @@ void gb_bfs::runBatch(const uint32_t* src, int k, const gb_bfs_options& o, std::
         if (runCluster(src, (uint32_t)k, bDist.get())) return;
     }
     ensureBatch(o, k);
-    DevBuf<BCounters> ctr;
-    ctr.ensure(4);
-    DevBuf<uint32_t> dsrc;
-    dsrc.ensure(64);
+    static_assert(sizeof(BCounters) % sizeof(unsigned long long) == 0, "whole words");
+    bCtr.ensure(4 * sizeof(BCounters) / sizeof(unsigned long long));
+    bSrc.ensure(64);
     hstage.ensure(64);
     std::memcpy(hstage.p, src, k * 4);
-    GB_CUDA(cudaMemcpyAsync(dsrc.get(), hstage.p, k * 4, cudaMemcpyHostToDevice, stream.s));
+    GB_CUDA(cudaMemcpyAsync(bSrc.get(), hstage.p, k * 4, cudaMemcpyHostToDevice, stream.s));
     BArgs a{};
     a.row_ptr = rowPtr.get();
     a.col_idx = colIdx.get();
@@ -961,8 +954,8 @@ void gb_bfs::runBatch(const uint32_t* src, int k, const gb_bfs_options& o, std::
     a.plane = bPlane.get();
     a.planeDepth = k >= kPlaneSources ? 1u << kPlanes : 1u;
     a.dist = bDist.get();
-    a.sources = dsrc.get();
-    a.ctr = ctr.get();
+    a.sources = bSrc.get();
+    a.ctr = reinterpret_cast<BCounters*>(bCtr.get());
     a.ctl = pctl.get();
     a.trace = ptrace.get();
     a.sel = selLoaded[1] ? selParams[1].get() : nullptr;
@@ -989,8 +982,9 @@ void gb_bfs::runBatch(const uint32_t* src, int k, const gb_bfs_options& o, std::
                         stream.s>>>(a);
     GB_LAUNCH_CHECK();
     GB_CUDA(cudaEventRecord(ev.b, stream.s));
-    unsigned ctl[4];
-    GB_CUDA(cudaMemcpyAsync(ctl, pctl.get(), sizeof ctl, cudaMemcpyDeviceToHost, stream.s));
+    pctlHost.ensure(4);
+    const unsigned* ctl = pctlHost.p;
+    GB_CUDA(cudaMemcpyAsync(pctlHost.p, pctl.get(), 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream.s));
     GB_CUDA(cudaStreamSynchronize(stream.s));
     lastGpuMs = ev.ms();
     lastLevels = ctl[2];

@@ -30,7 +30,9 @@ int hostThreads(int most) { return std::max(1, std::min(most, omp_get_max_thread
 // depths per byte, low nibble first; 1: a byte; 2: two bytes.  The last group
 // is filled up with the sentinel (out has room for it).
 template <int FMT>
-__global__ void packDepthsKernel(const uint32_t* d, uint64_t count, uint8_t* out, unsigned* overflow) {
+__global__ void packDepthsKernel(const uint32_t* d, uint64_t count, uint8_t* out, uint64_t pitch, unsigned* overflow) {
+    d += blockIdx.y * count;  // a row per y, `pitch` bytes apart when packed
+    out += blockIdx.y * pitch;
     constexpr uint32_t kBits = FMT == 0 ? 4 : FMT == 1 ? 8 : 16, kSentinel = (1u << kBits) - 1u;
     const bool aligned = (reinterpret_cast<uintptr_t>(d) & 15) == 0;
     bool bad = false;
@@ -126,6 +128,20 @@ void widenPacked(int fmt, const uint8_t* in, uint64_t count, uint32_t* out) {
     }
 }
 
+void widenRows(int fmt, const uint8_t* in, uint64_t pitch, uint32_t rows, uint64_t count, uint32_t* out, uint64_t stride) {
+    if (rows == 1 || stride == 0 || rows * count <= kOneThread) {  // stride 0: one row after the other, the last stays
+        for (uint32_t r = 0; r < rows; ++r) widenPacked(fmt, in + r * pitch, count, out + r * stride);
+        return;
+    }
+    constexpr uint64_t kPiece = 1u << 14;  // a multiple of 32
+    const uint64_t per = (count + kPiece - 1) / kPiece;
+#pragma omp parallel for num_threads(hostThreads(16)) schedule(static)
+    for (uint64_t t = 0; t < rows * per; ++t) {
+        const uint64_t r = t / per, lo = t % per * kPiece;
+        widenRange(fmt, in + r * pitch, lo, std::min(count, lo + kPiece), out + r * stride);
+    }
+}
+
 int packFormat(uint32_t levels) {
     if (levels < 15) return 0;
     if (levels < 255) return 1;
@@ -137,11 +153,13 @@ uint64_t packedBytes(int fmt, uint64_t count) {
     return fmt == 0 ? (count + 1) / 2 : fmt == 1 ? count : 2 * count;
 }
 
-void enqueuePack(int fmt, const uint32_t* d, uint64_t count, uint8_t* dev, unsigned* overflow, cudaStream_t st) {
-    const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((count / 8 + 255) / 256, (uint64_t)deviceSmCount() * 8));
-    if (fmt == 0) packDepthsKernel<0><<<grid, 256, 0, st>>>(d, count, dev, overflow);
-    else if (fmt == 1) packDepthsKernel<1><<<grid, 256, 0, st>>>(d, count, dev, overflow);
-    else packDepthsKernel<2><<<grid, 256, 0, st>>>(d, count, dev, overflow);
+void enqueuePack(int fmt, const uint32_t* d, uint64_t count, uint8_t* dev, unsigned* overflow, cudaStream_t st,
+                 uint32_t rows, uint64_t pitch) {
+    const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((count / 8 + 255) / 256, (uint64_t)deviceSmCount() * 8));
+    const dim3 grid(blocks, rows);
+    if (fmt == 0) packDepthsKernel<0><<<grid, 256, 0, st>>>(d, count, dev, pitch, overflow);
+    else if (fmt == 1) packDepthsKernel<1><<<grid, 256, 0, st>>>(d, count, dev, pitch, overflow);
+    else packDepthsKernel<2><<<grid, 256, 0, st>>>(d, count, dev, pitch, overflow);
     GB_LAUNCH_CHECK();
 }
 
