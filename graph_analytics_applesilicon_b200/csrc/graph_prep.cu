@@ -371,7 +371,7 @@ void radixSortKeys(DevBuf<unsigned long long>& a, DevBuf<unsigned long long>& tm
     }
 }
 
-constexpr uint64_t kStagedMin = 8u << 20;  // bytes of a result from which its copy is staged
+constexpr uint64_t kStagedMin = 16u << 20;  // bytes of a result from which its copy is staged
 
 // Sorted keys -> CSR (host arrays in *out), optionally unique / without
 // self-loops.  The columns take the sort's second buffer.
@@ -410,8 +410,9 @@ void keysToCsr(DevBuf<unsigned long long>& keys, DevBuf<unsigned long long>& tmp
     }
     try {
         // A ring of its own has to be page-locked, 2.5 ms, which a small result's
-        // slower plain copies do not cost (275,000 edges: 3.2 ms a build with
-        // plain copies, 6.6 with the ring; 17M: 72 and 28).
+        // slower plain copies do not cost (ms a build with plain copies / with the
+        // ring, by bytes of the result: 1.3 MB 3.2 / 6.6, 12 MB 6.6 / 9.5, 16 MB
+        // 7.4 / 10.8, 22 MB 27 / 17, 130 MB 72 / 28).
         if ((n + m2) * 4 < kStagedMin) {
             GB_CUDA(cudaMemcpyAsync(hrp, rp.get(), (n + 1) * 4, cudaMemcpyDeviceToHost, st));
             GB_CUDA(cudaMemcpyAsync(hci, col, (uint64_t)m2 * 4, cudaMemcpyDeviceToHost, st));
