@@ -134,12 +134,12 @@ def build_graph(G, scale=SCALE, nsrc=NSRC, gpu_prep=True):
 
 def depth_wire_bytes(n, levels):
     """Bytes per depth on the PCIe wire: the library packs depths to 4 bits,
-    1 or 2 bytes when the level count allows (arrays of 2^18 vertices or more)."""
-    if n >= (1 << 18) and levels < 15:
+    1 or 2 bytes when the level count allows."""
+    if levels < 15:
         return 0.5
-    if n >= (1 << 18) and levels < 255:
+    if levels < 255:
         return 1
-    if n >= (1 << 18) and levels < 65535:
+    if levels < 65535:
         return 2
     return 4
 
@@ -504,7 +504,7 @@ def bfs_config_workload(args, world, rank, local, g=None):
             "e2e": {"value": world * e64 / (e2e * 1e-3) / 1e9, "unit": "GTEPS", "h2d_bytes_per_step": 256,
                     "d2h_bytes_per_step": int(depth_wire_bytes(g.n, batch_levels) * 64 * g.n),
                     "result_bytes_per_step": 4 * 64 * g.n},
-            "gpu_launches": args.steps,
+            "gpu_launches": args.steps * (1 if road else 2),  # the cluster kernel; the traversal and its rows
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "peak_source": peak_kind, "kernel": "batchBfsKernel",
                          "bytes_per_launch": 64 * bytes_per_trav, "mean_launch_ms": batch_t,
@@ -800,11 +800,11 @@ def pagerank_workload(args, world, rank, local, g=None):
                     "d2h_bytes_per_step": 4 * g.n},
             "gpu_launches": 21 * args.steps,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": (measured_traffic("prPullKernel<2>" if variant == "gpu_pull_adaptive"
+                         "traffic": (measured_traffic("prAdaptiveKernel" if variant == "gpu_pull_adaptive"
                                                       else "prBlockedKernel", "chunglu_pr20", None)
                                      if args.n == 3070000 else None),
                          "peak_source": peak_kind,
-                         "kernel": "prPullKernel<2,false>" if variant == "gpu_pull_adaptive" else "prBlockedKernel",
+                         "kernel": "prAdaptiveKernel" if variant == "gpu_pull_adaptive" else "prBlockedKernel",
                          "bytes_per_launch": bytes_sweep, "mean_launch_ms": kernel_ms},
             "cpu_baseline": cpu, "clocks": clocks.summary(),
             "accuracy": {"l1_vs_fp64_gpu": l1, "ok": l1 < 1e-4}, "reference_check": reference,
@@ -1083,8 +1083,9 @@ def headline_workload(args, world, rank, local):
         "e2e_distinct_buffers": {"value": e2e_distinct, "unit": "GTEPS", "h2d_bytes_per_step": 4 * len(srcs),
                                  "d2h_bytes_per_step": wire, "result_bytes_per_step": 4 * g.n * len(srcs),
                                  "host_output": "a separate uint32[n] array per source (1 GB per step)"},
-        "gpu_launches": launches_per_step * args.steps,
-        "gpu_launches_e2e": (launches_per_step + len(srcs)) * args.steps,
+        # a batch: the traversal, its rows and, end to end, a pack for each row (1 MB or more)
+        "gpu_launches": launches_per_step * (2 if batched else 1) * args.steps,
+        "gpu_launches_e2e": (launches_per_step * (2 if batched else 1) + len(srcs)) * args.steps,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak if achieved else None, "traffic": traffic, "peak_source": peak_kind,
                      "kernel": kernel, "bytes_per_launch": bytes_per_trav,
