@@ -1215,7 +1215,11 @@ void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb
 // copied to pinned memory on the copy stream, and widened by host threads
 // while the next traversals run.  The host finishes source i before it queues
 // traversal i + B, the next user of buffer i % B, so an overflowing source can
-// still be copied whole from its depth buffer.
+// still be copied whole from its depth buffer.  Up to kSmallDepths vertices the
+// traversal packs its depths into pinned memory itself and leaves its level count
+// there (as in runPersistent): a launch and an event per source instead of a
+// dozen calls, which bound short traversals (R-MAT 18, 24 sources, 8 in flight:
+// 710 us a call, 626 so).
 void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* out, uint64_t stride,
                                const gb_bfs_options& o, float* msOut, uint32_t* levelsOut) {
     validateOptions(o);
@@ -1234,9 +1238,10 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
         grid = pWant > 0 ? std::min(pWant, share) : share;
     }
     for (uint32_t b = 1; b < B; ++b) mDist[b - 1].ensure(n + 4);
+    const bool direct = out && n <= kSmallDepths;  // the kernel packs, and its words are (levels, width, timed out)
     if (out)
         for (uint32_t b = 0; b < B; ++b) {  // sized for the widest packed form up front
-            mPackDev[b].ensure(2 * n + 16);
+            if (!direct) mPackDev[b].ensure(2 * n + 16);
             mPackHost[b].ensure(2 * n + 16);
         }
     mCtl.ensure((size_t)count * 4);
@@ -1272,6 +1277,11 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
     const bool timed = msOut != nullptr;
     cudaStream_t cs = copyStream.s;
 
+    if (direct)
+        for (uint32_t i = 0; i < count; ++i) {
+            mCtlHost.p[4 * (size_t)i] = kNotDone;
+            mCtlHost.p[4 * (size_t)i + 2] = 0;
+        }
     GB_CUDA(cudaMemsetAsync(mCtl.get(), 0, (size_t)count * 4 * sizeof(unsigned), stream.s));
     // the other streams start after the work queued before this call on the handle's stream
     GB_CUDA(cudaEventRecord(startEv, stream.s));
@@ -1284,7 +1294,10 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
         a.dist = bufs[b];
         a.ctl = mCtl.get() + 4 * (size_t)i;
         cudaEvent_t packed = mSlotEv[b], copied = mSlotEv[kManySlots + b], released = mSlotEv[2 * kManySlots + b];
-        if (i >= B) {  // buffer b's previous traversal (and its pack and copy) first
+        if (direct) {
+            a.packHost = mPackHost[b].p;
+            a.ctlHost = mCtlHost.p + 4 * (size_t)i;
+        } else if (i >= B) {  // buffer b's previous traversal (and its pack and copy) first
             GB_CUDA(cudaStreamWaitEvent(st, released, 0));
             if (out) GB_CUDA(cudaStreamWaitEvent(st, copied, 0));
         }
@@ -1292,6 +1305,10 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
         if (!a.fillDist) GB_CUDA(cudaMemsetAsync(bufs[b], 0xFF, n * 4, st));  // every depth infinity
         launchFor(*this, a, grid, st);
         if (timed || i + 1 == count) GB_CUDA(cudaEventRecord(mEv[2 * i + 1], st));
+        if (direct) {  // the host has widened buffer b's previous depths before it gets here
+            GB_CUDA(cudaEventRecord(copied, st));
+            return;
+        }
         if (!out) {
             GB_CUDA(cudaEventRecord(released, st));
             return;
@@ -1337,11 +1354,19 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
             for (; queued < count && queued < i + B; ++queued) enqueue(queued);
             const uint32_t b = i % B;
             GB_CUDA(cudaEventSynchronize(mSlotEv[kManySlots + b]));
-            const unsigned* c = mCtlHost.p + 4 * (size_t)i;
-            if (c[1]) throw timeout();
-            maxSeen = std::max(maxSeen, c[2]);
-            anySeen = true;
+            volatile unsigned* c = mCtlHost.p + 4 * (size_t)i;
             uint32_t* dst = out + (uint64_t)i * stride;
+            if (direct) {
+                if (c[0] == kNotDone || c[2]) throw timeout();
+                if ((int)c[1] >= 0) widenPacked((int)c[1], mPackHost[b].p, n, dst);
+                else staged.run(bufs[b], n * 4, dst, cs);
+                c[2] = c[0];  // as the control words read below
+                c[1] = 0;
+                continue;
+            }
+            if (c[1]) throw timeout();
+            maxSeen = std::max(maxSeen, (uint32_t)c[2]);
+            anySeen = true;
             if (fmt[i] >= 0 && mFlagHost.p[i] == 0) {
                 widenPacked(fmt[i], mPackHost[b].p, n, dst);
             } else {  // too many levels for the predicted width: the buffer is still intact
