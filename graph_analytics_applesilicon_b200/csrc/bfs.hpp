@@ -70,9 +70,9 @@ void enqueuePack(int fmt, const uint32_t* d, uint64_t count, uint8_t* dev, unsig
                  uint32_t rows = 1, uint64_t pitch = 0);
 void widenPacked(int fmt, const uint8_t* in, uint64_t count, uint32_t* out);
 void widenRows(int fmt, const uint8_t* in, uint64_t pitch, uint32_t rows, uint64_t count, uint32_t* out, uint64_t stride);
-// Depth arrays up to this size are packed straight into pinned host memory, by
-// the traversal's kernel or one after it; larger ones into device memory, and
-// copied in chunks that the widening overlaps.
+// Depth arrays up to this size are packed straight into pinned host memory;
+// larger ones into device memory, and copied in chunks that the widening overlaps
+// (single persistent calls: bfs_persistent.cu).
 constexpr uint64_t kSmallDepths = 1ull << 20;
 constexpr int kEdgeStatWords = 8;
 constexpr int kMaxInFlight = 16;              // traversals at once in gb_bfs::runPersistentMany

@@ -34,6 +34,7 @@ constexpr uint64_t kEnqueueEdges = 1ull << 18;  // top-down levels with this man
 // (soloLevels).  A level of 4 takes 5 us there against 6.5 on the grid, one of 8
 // 10 us (road 300 x 300, rule: 2.7 ms with 2 edges per thread, 1.8 with 4).
 constexpr uint32_t kSoloEdges = 4;
+constexpr uint64_t kPackInKernel = 1ull << 23;  // depth arrays up to this size are packed by a single call's kernel
 constexpr unsigned kNotDone = 0xFFFFFFFFu;
 // At most so many levels at a time, which bounds the other blocks' wait (about
 // 0.3 ms, some 400 polls); a caller's spin limit under kSoloSpin polls, which may
@@ -61,6 +62,7 @@ struct PArgs {
     unsigned* ctl;  // [0] barrier word, [1] error flag, [2] levels run
     bool fillDist;      // the kernel sets the depths to infinity (at most kSmallDepths; else a memset before the launch)
     uint8_t* packHost;  // pinned host memory for the packed depths, or null
+    int packMax;        // and the widest form (packFormat) it has room for
     unsigned* ctlHost;  // pinned: [0] levels run, [1] width of the packed depths (with packHost), [2] a wait ran out
     gb_level* trace;
     const float* sel;
@@ -599,13 +601,15 @@ __device__ void soloLevels(const PArgs& a, Smem<NT>& sm, uint32_t level, uint32_
     }
 }
 
-// The depths packed straight into pinned host memory (at most kSmallDepths
+// The depths packed straight into pinned host memory (at most kPackInKernel
 // vertices): the level count is known here, so the width is exact, and no
-// kernel or copy of its own follows the traversal.
+// kernel or copy of its own follows the traversal.  Us a call against a pack
+// kernel and chunked copies, which the widening overlaps: R-MAT of 1.5M vertices
+// 192 / 217, of 2M 167 / 189, of 4.2M 270 / 291.
 __device__ void packToHost(const PArgs& a, uint32_t level, uint64_t gtid, uint64_t gthreads) {
     const int fmt = level < 15 ? 0 : level < 255 ? 1 : level < 65535 ? 2 : -1;  // packFormat
     if (gtid == 0) a.ctlHost[1] = (unsigned)fmt;
-    if (fmt < 0) return;
+    if (fmt < 0 || fmt > a.packMax) return;
     const uint4* d4 = reinterpret_cast<const uint4*>(a.dist);
     for (uint64_t g = gtid; g < (a.n + 7) / 8; g += gthreads) {
         const uint4 x = __ldcg(d4 + 2 * g), y = 8 * g + 4 < a.n ? __ldcg(d4 + 2 * g + 1) : make_uint4(0, 0, 0, 0);
@@ -1037,6 +1041,7 @@ PArgs makeArgs(gb_bfs& h, const gb_bfs_options& o, uint32_t src) {
     a.ctl = h.pctl.get();
     a.fillDist = h.n <= kSmallDepths;
     a.packHost = nullptr;
+    a.packMax = 2;
     a.ctlHost = nullptr;
     a.trace = h.ptrace.get();
     a.traceCap = kTraceCap;
@@ -1162,9 +1167,13 @@ void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb
     done[0] = kNotDone;
     done[2] = 0;
     a.ctlHost = pctlHost.p;
-    const bool packInKernel = out && n <= kSmallDepths;
+    const bool packInKernel = out && n <= kPackInKernel;
     if (packInKernel) {
-        packHost.ensure(2 * n + 16);
+        // room for the widest form, or, page-locking being dear (14 ms for 4 MB), for
+        // a large array for the one that the last run needed
+        const uint64_t n8 = (n + 7) / 8 * 8;
+        if (n > kSmallDepths) a.packMax = std::max(0, packFormat(lastLevels));
+        packHost.ensure(packedBytes(a.packMax, n8));
         a.packHost = packHost.p;
     }
     GB_CUDA(cudaEventRecord(ev.a, stream.s));
@@ -1187,8 +1196,9 @@ void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb
         throw Error(GB_ERR_TIMEOUT, "persistent BFS: grid barrier wait exceeded its spin limit");
     }
     lastLevels = done[0];
-    if (packInKernel && (int)done[1] >= 0) widenPacked((int)done[1], packHost.p, n, out);
-    else if (packInKernel) staged.run(dist.get(), n * 4, out, stream.s);
+    const int width = packInKernel ? (int)done[1] : -1;
+    if (width >= 0 && width <= a.packMax) widenPacked(width, packHost.p, n, out);
+    else if (packInKernel) copyDepthsToHost(this, dist.get(), n, out, lastLevels);
     else if (out) endDepths(this, ret, lastLevels, out);
     if (tr) {
         const uint32_t k = std::min<uint32_t>(lastLevels, kTraceCap);

@@ -176,7 +176,7 @@ void beginDepths(gb_bfs* h, const uint32_t* d, uint64_t count, uint32_t levels, 
     r.fmt = packFormat(levels);
     if (r.fmt < 0) return;
     const uint64_t bytes = packedBytes(r.fmt, count);
-    h->packHost.ensure(bytes + 16);
+    h->packHost.ensure(count <= kSmallDepths ? bytes + 16 : bytes);
     h->packFlagHost.ensure(1);
     if (count <= kSmallDepths) {
         *h->packFlagHost.p = 0;
