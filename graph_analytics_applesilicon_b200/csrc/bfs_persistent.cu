@@ -1169,10 +1169,10 @@ void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb
     a.ctlHost = pctlHost.p;
     const bool packInKernel = out && n <= kPackInKernel;
     if (packInKernel) {
-        // room for the widest form, or, page-locking being dear (14 ms for 4 MB), for
-        // a large array for the one that the last run needed
+        // room for the widest form (up to 128 KB), or, page-locking a larger block
+        // being dear, for the one that the last run needed
         const uint64_t n8 = (n + 7) / 8 * 8;
-        if (n > kSmallDepths) a.packMax = std::max(0, packFormat(lastLevels));
+        if (n > (1u << 16)) a.packMax = std::max(0, packFormat(lastLevels));
         packHost.ensure(packedBytes(a.packMax, n8));
         a.packHost = packHost.p;
     }

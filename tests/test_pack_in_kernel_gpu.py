@@ -1,5 +1,5 @@
 """Depths that the traversal's kernel packs into pinned memory, around the sizes
-where its room is for the last run's width (over 2^20) and where it no longer packs
+where its room is for the last run's width (over 2^16) and where it no longer packs
 (over 2^23): runs of few, more than 14, 254 and 65,534 levels in every order, sizes
 that are not a multiple of 8."""
 import numpy as np
