@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "bfs.hpp"
+#include "cluster_leave.hpp"
 
 namespace cg = cooperative_groups;
 
@@ -42,7 +43,11 @@ constexpr uint32_t kClLanes = 4;     // lanes per queue entry, a neighbour slot 
 // col_idx, which bounds the degree (31) and m (2^26).
 constexpr uint32_t kClMore = 0x80000000u, kClPosBits = 26, kClMaxDegree = 31;
 constexpr size_t kClSmem = 220 * 1024;  // queues and bitmap of one block
+// A wait gives up after this time and then this many polls: the timer runs on
+// while the process is preempted, the polls do not.
 constexpr unsigned long long kClWaitNs = 2000000000ull;
+constexpr uint32_t kClWaitPolls = 1u << 14;
+constexpr unsigned long long kClSettleNs = 20000ull;  // a count takes under a microsecond to arrive
 
 struct ClArgs {
     const uint4* __restrict__ nbr;  // neighbour table
@@ -86,6 +91,24 @@ __device__ __forceinline__ bool claim(uint32_t bmAddr, uint32_t u) {
     return !((old >> (u & 31)) & 1u);
 }
 
+// The cluster as one block sees it when blocks give up (cluster_leave.hpp):
+// `flag` is a word of this block's shared memory, 0 until a block gives up.
+template <uint32_t NC>
+struct ClusterEnd {
+    cg::cluster_group& cl;
+    uint32_t flag;
+    __device__ void sync() { cl.sync(); }
+    __device__ void raise() {
+        if (threadIdx.x < NC)
+            asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(mapaAddr(flag, threadIdx.x)), "r"(1u)
+                         : "memory");
+    }
+    __device__ bool raised() { return __syncthreads_or(ldShared(flag) != 0); }
+    __device__ void settle() {
+        for (const uint64_t t = globaltimer(); globaltimer() - t < kClSettleNs;) __nanosleep(1000);
+    }
+};
+
 // Level L reads the queue parts of parity L & 1 and appends to the others, a
 // block always to its own part.  Block r's count for level L is cnt[L % 3]
 // (the count level L + 2 will fill is zeroed during level L) and reaches block
@@ -96,21 +119,24 @@ __device__ __forceinline__ bool claim(uint32_t bmAddr, uint32_t u) {
 // list instead, entry i of the concatenation going to lane group i; only then
 // is a cluster barrier needed, for the other blocks' queue entries.  Entries
 // beyond a part's room are dropped but counted: every block sees that count,
-// all leave together, and the caller runs the sources another way.
+// all leave together, and the caller runs the sources another way.  A block
+// whose wait runs out takes all others with it (cluster_leave.hpp).
 template <uint32_t NC>
 __global__ void __launch_bounds__(kClThreads, 2) clusterBfsKernel(ClArgs a) {
     extern __shared__ __align__(16) uint4 clMem[];  // [2][kClQueue] entries, then the bitmap
-    __shared__ uint32_t cnt[3];
+    __shared__ uint32_t cnt[3], gaveUp;
     __shared__ __align__(8) unsigned long long slot[2][NC], mbar[2];
     cg::cluster_group cl = cg::this_cluster();
     const uint32_t rank = cl.block_rank(), s = blockIdx.x / NC;
     const unsigned tid = threadIdx.x, lane = laneId();
     uint32_t* dist = a.dist + (uint64_t)s * a.n;
     uint32_t* bitmap = reinterpret_cast<uint32_t*>(clMem + 2 * kClQueue);
-    const uint32_t bmAddr = smemAddr(bitmap), qAddr = smemAddr(clMem), slotAddr = smemAddr(slot);
+    const uint32_t bmAddr = smemAddr(bitmap), qAddr = smemAddr(clMem), slotAddr = smemAddr(slot), flagAddr = smemAddr(&gaveUp);
+    ClusterEnd<NC> end{cl, flagAddr};
     const uint64_t t0 = globaltimer();
     for (uint32_t i = tid; i < a.words; i += kClThreads) bitmap[i] = 0;
     if (tid < 3) cnt[tid] = 0;
+    if (tid == 0) gaveUp = 0;
     if (tid < 2) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smemAddr(&mbar[tid])) : "memory");
     if (tid < NC) slot[0][tid] = tid == 0;  // level 0: the source, in block 0's part
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -169,7 +195,7 @@ __global__ void __launch_bounds__(kClThreads, 2) clusterBfsKernel(ClArgs a) {
         const uint32_t over = most - total / NC;
         if (NC > 1 && (over > 256 || (over > 32 && level - spreadAt >= 16))) {
             spreadAt = level;
-            cl.sync();
+            if (!clusterMeet(end)) break;  // block-uniform
             uint32_t x = mine;
 #pragma unroll
             for (int o = 1; o < (int)NC; o <<= 1) {
@@ -191,9 +217,9 @@ __global__ void __launch_bounds__(kClThreads, 2) clusterBfsKernel(ClArgs a) {
                 expand(i < total ? ldCluster(mapaAddr(qc + (i - p) * 16 + sub * 4, j)) : kInf);
             }
         } else {
-            const uint32_t end = __shfl_sync(kFull, mine, rank);
-            for (uint32_t i0 = 0; i0 + first < end; i0 += kGroups)
-                expand(i0 + grp < end ? ldShared(qc + (i0 + grp) * 16 + sub * 4) : kInf);
+            const uint32_t own = __shfl_sync(kFull, mine, rank);
+            for (uint32_t i0 = 0; i0 + first < own; i0 += kGroups)
+                expand(i0 + grp < own ? ldShared(qc + (i0 + grp) * 16 + sub * 4) : kInf);
         }
         __syncthreads();  // the block's appends are counted
         const uint32_t mb = smemAddr(&mbar[par ^ 1]);
@@ -207,7 +233,7 @@ __global__ void __launch_bounds__(kClThreads, 2) clusterBfsKernel(ClArgs a) {
                              "l"(c), "r"(mapaAddr(mb, lane))
                              : "memory");
         }
-        uint32_t done = 0;
+        uint32_t done = 0, polls = 0;
         for (uint64_t tw = 0; !done;) {  // bounded
             asm volatile(
                 "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -217,7 +243,7 @@ __global__ void __launch_bounds__(kClThreads, 2) clusterBfsKernel(ClArgs a) {
             if (done) break;
             const uint64_t t = globaltimer();
             if (!tw) tw = t;
-            if (t - tw > kClWaitNs) break;
+            if ((t - tw > kClWaitNs && ++polls > kClWaitPolls) || ldShared(flagAddr)) break;
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         if (__syncthreads_or(!done)) {  // also: every thread's copies into the queue have landed
@@ -226,7 +252,8 @@ __global__ void __launch_bounds__(kClThreads, 2) clusterBfsKernel(ClArgs a) {
         }
         c0 = c1;
     }
-    cl.sync();  // no block leaves while another may still send to it or read its queue
+    // no block leaves while another may still send to it or read its queue
+    if (clusterLeave(end, status == kClusterTimeout)) status = kClusterTimeout;
     if (rank == 0 && tid == 0) a.stat[s] = {level, status, (unsigned long long)(globaltimer() - t0)};
 }
 
