@@ -139,6 +139,7 @@ struct gb_bfs {
     // bounded-degree graphs: a cluster per source (bfs_cluster.cu)
     uint32_t maxDegree = 0xFFFFFFFFu;  // of the graph, set when the handle's CSR is checked
     bool cOff = false;                 // a frontier of this graph outgrew the queues
+    signed char cRuns[5] = {-1, -1, -1, -1, -1};  // by log2 of a cluster's blocks: the device can run it (-1: not asked)
     bool cNbrReady = false;            // neighbour table built (dropped when the lists are re-sorted)
     gb::DevBuf<uint4> cNbr;
     gb::DevBuf<uint32_t> cSrc;
@@ -190,7 +191,8 @@ struct gb_bfs {
                            const gb_bfs_options& o, float* ms, uint32_t* levels);
     void runBatchMany(const uint32_t* src, uint32_t count, uint32_t* out, uint64_t stride,
                       const gb_bfs_options& o, float* ms, uint32_t* levels);
-    bool clusterFits(uint32_t k, const gb_bfs_options& o) const;
+    bool clusterFits(uint32_t k, const gb_bfs_options& o);
+    uint32_t clusterBlocks(uint32_t k);
     bool runCluster(const uint32_t* src, uint32_t k, uint32_t* out);
     bool runClusterMany(const uint32_t* src, uint32_t count, uint32_t* out, uint64_t stride, float* ms,
                         uint32_t* levels);

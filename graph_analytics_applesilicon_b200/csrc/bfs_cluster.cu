@@ -27,6 +27,7 @@
 
 #include "bfs.hpp"
 #include "cluster_leave.hpp"
+#include "cluster_shape.hpp"
 
 namespace cg = cooperative_groups;
 
@@ -36,13 +37,11 @@ namespace {
 // 512 threads: 256 make more passes of a level (1400 x 1400: 3.85 against 3.71
 // ms), 1024 cost more per barrier (4.37 ms).
 constexpr int kClThreads = 512;
-constexpr uint32_t kClQueue = 2048;  // queue entries per block and level
 constexpr uint32_t kClLanes = 4;     // lanes per queue entry, a neighbour slot each
 // A vertex of more than 4 neighbours keeps 3 in its slots; the fourth slot then
 // holds kClMore | (neighbours left) << kClPosBits | position of the fourth in
 // col_idx, which bounds the degree (31) and m (2^26).
 constexpr uint32_t kClMore = 0x80000000u, kClPosBits = 26, kClMaxDegree = 31;
-constexpr size_t kClSmem = 220 * 1024;  // queues and bitmap of one block
 // A wait gives up after this time and then this many polls: the timer runs on
 // while the process is preempted, the polls do not.
 constexpr unsigned long long kClWaitNs = 2000000000ull;
@@ -271,8 +270,6 @@ __global__ void nbrTableKernel(const uint32_t* __restrict__ row_ptr, const uint3
     }
 }
 
-size_t clusterSmem(uint64_t n, uint32_t nc) { return 32 * kClQueue + ((n + 31) / 32 + nc - 1) / nc * 4; }
-
 template <uint32_t NC>
 cudaLaunchConfig_t clusterConfig(uint64_t n, uint32_t k, cudaStream_t st, cudaLaunchAttribute* attr) {
     attr->id = cudaLaunchAttributeClusterDimension;
@@ -289,25 +286,39 @@ cudaLaunchConfig_t clusterConfig(uint64_t n, uint32_t k, cudaStream_t st, cudaLa
 }
 
 template <uint32_t NC>
-void launchCluster(const ClArgs& a, uint32_t k, cudaStream_t st) {
+void allowCluster() {
     GB_CUDA(cudaFuncSetAttribute(clusterBfsKernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmem));
     if (NC > 8) GB_CUDA(cudaFuncSetAttribute(clusterBfsKernel<NC>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+}
+
+template <uint32_t NC>
+void launchCluster(const ClArgs& a, uint32_t k, cudaStream_t st) {
+    allowCluster<NC>();
     cudaLaunchAttribute attr{};
     cudaLaunchConfig_t cfg = clusterConfig<NC>(a.n, k, st, &attr);
     GB_CUDA(cudaLaunchKernelEx(&cfg, clusterBfsKernel<NC>, a));
 }
 
-// Blocks per source.  More blocks make a level's passes fewer, until the
-// sources together cover the SMs (64 sources, 1400 x 1400: 7.7 ms with 2
-// blocks each, 12.2 with 4 and 13.2 with 8) or the frontier is too small to
-// need them (150 x 150, about 100 vertices a level: 0.23 ms with 1 block, 0.31
-// with 16; 700 x 700, about 600: 2.2 and 1.4 ms).  At least as many as hold
-// the bitmap; 0 when 16 do not.
-uint32_t clusterSize(uint64_t n, uint32_t k) {
-    uint32_t nc = 1;
-    while (nc < 16 && (uint64_t)k * nc * 2 <= (uint64_t)deviceSmCount() && n >= (uint64_t)nc * 2 * 16384) nc *= 2;
-    while (nc <= 16 && clusterSmem(n, nc) > kClSmem) nc *= 2;
-    return nc <= 16 ? nc : 0;
+// Whether the device can run a cluster of NC blocks of this graph.
+template <uint32_t NC>
+bool clusterRuns(uint64_t n) {
+    allowCluster<NC>();
+    cudaLaunchAttribute attr{};
+    cudaLaunchConfig_t cfg = clusterConfig<NC>(n, 1, nullptr, &attr);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, clusterBfsKernel<NC>, &cfg) == cudaSuccess) return clusters > 0;
+    cudaGetLastError();  // a size the device does not know
+    return false;
+}
+
+bool clusterRuns(uint64_t n, uint32_t nc) {
+    switch (nc) {
+        case 1: return clusterRuns<1>(n);
+        case 2: return clusterRuns<2>(n);
+        case 4: return clusterRuns<4>(n);
+        case 8: return clusterRuns<8>(n);
+        default: return clusterRuns<16>(n);
+    }
 }
 
 }  // namespace
@@ -320,9 +331,18 @@ using namespace gb;
 // 8 on average.  A graph of that shape whose frontier outgrows the queues
 // after all (a random 3-regular graph) is noticed in its first levels and
 // marked, so later calls on the handle do not try again.
-bool gb_bfs::clusterFits(uint32_t k, const gb_bfs_options& o) const {
+bool gb_bfs::clusterFits(uint32_t k, const gb_bfs_options& o) {
     return !cOff && o.force_strategy < 0 && o.grid_blocks == 0 && maxDegree <= kClMaxDegree && m <= 8 * n &&
-           m < (1ull << kClPosBits) && n < kClMore && clusterSize(n, k) != 0;
+           m < (1ull << kClPosBits) && n < kClMore && clusterBlocks(k) != 0;
+}
+
+// clusterSize for this handle, which asks the device about a size once.
+uint32_t gb_bfs::clusterBlocks(uint32_t k) {
+    return clusterSize(n, k, (uint32_t)deviceSmCount(), [&](uint32_t nc) {
+        signed char& known = cRuns[31 - __builtin_clz(nc)];
+        if (known < 0) known = clusterRuns(n, nc);
+        return known != 0;
+    });
 }
 
 // Runs k sources' traversals into out (source i's depths at out + i * n) and
@@ -342,7 +362,7 @@ bool gb_bfs::runCluster(const uint32_t* src, uint32_t k, uint32_t* out) {
     hstage.ensure(64);
     std::memcpy(hstage.p, src, k * 4);
     GB_CUDA(cudaMemcpyAsync(cSrc.get(), hstage.p, k * 4, cudaMemcpyHostToDevice, stream.s));
-    const uint32_t nc = clusterSize(n, k);
+    const uint32_t nc = clusterBlocks(k);
     const ClArgs a{cNbr.get(), colIdx.get(), out, cSrc.get(), cStat.get(), n, (uint32_t)(((n + 31) / 32 + nc - 1) / nc)};
     GB_CUDA(cudaEventRecord(ev.a, stream.s));
     GB_CUDA(cudaMemsetAsync(out, 0xFF, (uint64_t)k * n * 4, stream.s));  // every depth infinity
