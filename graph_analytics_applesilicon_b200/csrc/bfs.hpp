@@ -75,6 +75,9 @@ void widenRows(int fmt, const uint8_t* in, uint64_t pitch, uint32_t rows, uint64
 // (single persistent calls: bfs_persistent.cu).
 constexpr uint64_t kSmallDepths = 1ull << 20;
 constexpr int kEdgeStatWords = 8;
+// A spin limit under this many polls may be set for the grid's levels of a few us,
+// so only forms whose waits are that short are run with it.
+constexpr unsigned long long kSoloSpin = 1ull << 14;
 constexpr int kMaxInFlight = 16;              // traversals at once in gb_bfs::runPersistentMany
 constexpr int kManySlots = kMaxInFlight + 2;  // depth buffers it rotates (in flight + 2)
 }  // namespace gb

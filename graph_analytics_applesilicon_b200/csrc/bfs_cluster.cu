@@ -330,9 +330,10 @@ using namespace gb;
 // networks and grids, whose frontiers stay narrow: at most 31 neighbours and
 // 8 on average.  A graph of that shape whose frontier outgrows the queues
 // after all (a random 3-regular graph) is noticed in its first levels and
-// marked, so later calls on the handle do not try again.
+// marked, so later calls on the handle do not try again.  A caller's spin limit
+// under kSoloSpin asks for waits shorter than this form's: the grid forms have them.
 bool gb_bfs::clusterFits(uint32_t k, const gb_bfs_options& o) {
-    return !cOff && o.force_strategy < 0 && o.grid_blocks == 0 && maxDegree <= kClMaxDegree && m <= 8 * n &&
+    return !cOff && (o.spin_limit == 0 || o.spin_limit >= kSoloSpin) && o.force_strategy < 0 && o.grid_blocks == 0 && maxDegree <= kClMaxDegree && m <= 8 * n &&
            m < (1ull << kClPosBits) && n < kClMore && clusterBlocks(k) != 0;
 }
 

@@ -37,10 +37,9 @@ constexpr uint32_t kSoloEdges = 4;
 constexpr uint64_t kPackInKernel = 1ull << 23;  // depth arrays up to this size are packed by a single call's kernel
 constexpr unsigned kNotDone = 0xFFFFFFFFu;
 // At most so many levels at a time, which bounds the other blocks' wait (about
-// 0.3 ms, some 400 polls); a caller's spin limit under kSoloSpin polls, which may
-// be set for the grid's levels of a few us, keeps every level on the grid.
+// 0.3 ms, some 400 polls); a caller's spin limit under kSoloSpin polls keeps every
+// level on the grid.
 constexpr uint32_t kSoloLevels = 64;
-constexpr unsigned long long kSoloSpin = 1ull << 14;
 
 enum { S_LEVEL, S_BOTTOMUP, S_SCOUT, S_TOCHECK, S_UNEXPLORED, S_REACHED, S_QVALID, S_LAST, S_COUNT };
 
