@@ -1346,8 +1346,10 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
     }
     // Iteration batches as CUDA graphs (cached per variant / shape).
     const int batch = tolMode ? kGraphBatch : std::max(1, o.iters);
+    uint32_t dampingBits;
+    std::memcpy(&dampingBits, &o.damping, 4);
     auto key = std::make_tuple(v, batch, (int)o.tg, (int)(o.inplace != 0), relabel ? 1 : 0, (int)binSmall,
-                               (int)binLarge);
+                               (int)binLarge, dampingBits);
     cudaGraphExec_t exec = nullptr;
     auto it = graphs.find(key);
     if (it != graphs.end()) {
@@ -1362,6 +1364,7 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
             throw;
         }
         GB_CUDA(cudaStreamEndCapture(stream.s, &g));
+        if (graphs.size() >= kPrGraphs) invalidateGraphs();  // none is running: every run waits for its own
         GB_CUDA(cudaGraphInstantiate(&exec, g, 0));
         cudaGraphDestroy(g);
         graphs[key] = exec;

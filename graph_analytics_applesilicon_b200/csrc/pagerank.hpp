@@ -59,6 +59,8 @@ constexpr uint32_t kBlkHub = 4096;  // rows with this many in-edges are summed a
 // 24K 736 us a sweep, 32K 717, 40K 710, 48K 793, 56K 1,390; none 820).
 constexpr uint32_t kPrHotMax = 32u * 1024u;
 
+constexpr size_t kPrGraphs = 64;  // cached graphs of a handle, at most
+
 // A run of the adaptive layout: vertices [v0, vEnd), all with lists of `vecs`
 // vectors, handled by groups of 1 << lg lanes.  Lists follow one another from
 // vector e0 on; `inter`: in blocks of 32 lists with vector k of the 32 lists
@@ -144,8 +146,9 @@ struct gb_pr {
     uint32_t nRowBlocks = 0, rowsPer = 0, nParts = 0, nBlkHubs = 0;
     bool blkReady = false;
 
-    // cached CUDA graphs of iteration batches
-    std::map<std::tuple<int, int, int, int, int, int, int>, cudaGraphExec_t> graphs;
+    // cached CUDA graphs of iteration batches, by what their kernels' arguments
+    // depend on (the damping factor's bits last); at most kPrGraphs of them
+    std::map<std::tuple<int, int, int, int, int, int, int, uint32_t>, cudaGraphExec_t> graphs;
     int grid = 0;
 
     ~gb_pr();
