@@ -1153,6 +1153,18 @@ static void raiseHotLimit() {
     (void)raised;
 }
 
+// The decimal value a float option was written as (0.85f -> 0.85), as the
+// double-precision CPU reference has it: the shortest that is this float.  (Seven
+// digits for every float move more than half of them to a neighbour's value,
+// 0.99999994 to 0.9999999, which adds two thirds to 1 - d.)
+static double writtenDecimal(float x) {
+    char buf[32];
+    for (int digits = 6;; ++digits) {
+        std::snprintf(buf, sizeof buf, "%.*g", digits, (double)x);
+        if (digits == 9 || std::strtof(buf, nullptr) == x) return std::strtod(buf, nullptr);
+    }
+}
+
 // Enqueue one iteration of `variant` on the handle's stream (capturable).
 static void enqueueIteration(gb_pr& h, int v, const gb_pr_options& o, PrArgs& a, PrArgs& ag) {
     const uint32_t tg = o.tg;
@@ -1305,13 +1317,7 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
     PrArgs a = makeArgs(*this, false);
     a.damping = o.damping;
     a.invN = 1.0f / (float)n;
-    // The decimal value the float option was written as (0.85f -> 0.85), as in the
-    // double-precision CPU reference.
-    {
-        char buf[32];
-        std::snprintf(buf, sizeof buf, "%.7g", (double)o.damping);
-        a.damping64 = std::strtod(buf, nullptr);
-    }
+    a.damping64 = writtenDecimal(o.damping);
     a.base64 = (1.0 - a.damping64) / (double)n;
     a.base = (float)a.base64;
     a.dampingLo = (float)(a.damping64 - (double)o.damping);

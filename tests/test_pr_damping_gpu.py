@@ -43,3 +43,25 @@ def test_many_dampings_on_one_handle(gb):
         pr.run("gpu_pull_vector", o[i])
         assert np.array_equal(pr.ranks(), first[i]), i
     assert not np.array_equal(first[0], first[99])
+
+
+@pytest.mark.parametrize("damping", [0.85, 0.5, 0.8500001, 0.123456789, 0.9999995, 0.99999994])
+@pytest.mark.parametrize("variant", [v for v in VARIANTS if v != "gpu_pull_gs"])
+def test_the_damping_written_is_the_one_used(gb, oracle, variant, damping):
+    """Vertex 0 has no in-links and nothing dangles, so its rank is (1 - d) / n,
+    where another damping factor than the one written shows, the more the nearer
+    to 1 it is.  d: the shortest decimal of the option's float.  Tolerance: a
+    few roundings to float (6e-8 each)."""
+    n = 4097
+    u = np.arange(n, dtype=np.uint32)
+    v = np.where(u + 1 < n, u + 1, 1).astype(np.uint32)  # 0 -> 1 -> ... -> n - 1 -> 1
+    g = gb.from_edges(n, u, v, True)
+    gin = gb.transpose(g)
+    pr = gb.GpuPageRank(n, g, gin, g.degrees())
+    pr.run(variant, gb.PrOptions(iters=3, damping=damping))
+    got = pr.ranks_f64() if variant == "gpu_pull_f64" else pr.ranks().astype(np.float64)
+    decimals = [float(f"{np.float32(damping):.{k}g}") for k in range(6, 10)]
+    d = next(x for x in decimals if np.float32(x) == np.float32(damping))
+    want, _, _ = oracle.pagerank_serial(gin, g.degrees(), 3, damping=d)
+    assert abs(want[0] * n / (1.0 - d) - 1.0) < 1e-7
+    assert np.abs(got / want - 1.0).max() < 3e-7
