@@ -49,7 +49,7 @@ struct PrArgs {
     float* partF;
     double* partD;
     uint32_t n;
-    float damping, dampingLo, base, invN;
+    float invN;
     double base64, invN64, damping64;
     uint32_t lo, hi;  // GS colored: id range of the set
     // split vertices: chunk table, per-hub (first, count), tickets, partials
@@ -94,19 +94,16 @@ __device__ __forceinline__ uint32_t smemAddr(const void* p) { return (uint32_t)_
 
 __device__ __forceinline__ int ldvi(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
 
-__device__ __forceinline__ float prValue(const PrArgs& a, float s, float dang) {
-    // pr_value, src/shaders/pagerank.metal:45-48, with what the float of the damping
-    // factor leaves out (0.85: 2.4e-8) added, so the ranks are not all off the same way
-    const float x = s + dang * a.invN;
-    return fmaf(a.damping, x, fmaf(a.dampingLo, x, a.base));
-}
-
-// The same of a split list's float-float sum, in FP64 and rounded once: the hubs
-// hold most of the ranks' norm.
-__device__ __forceinline__ float prValueSplit(const PrArgs& a, float hi, float lo, const GbPrControl* c) {
-    const double dang = (double)c->dangHi + (double)c->dangLo;
-    return (float)(a.base64 + a.damping64 * ((double)hi + (double)lo + dang * a.invN64));
-}
+// pr_value, src/shaders/pagerank.metal:45-48: base + damping * (s + dangling / n).
+// What does not depend on the list is formed once per thread in FP64, and a
+// vertex's value is rounded once: in floats, every vertex with few or no
+// in-links carried the same rounding of that part.
+struct PrTerm {
+    double damping, rest;
+    __device__ __forceinline__ PrTerm(const PrArgs& a, const GbPrControl* c)
+        : damping(a.damping64), rest(a.base64 + a.damping64 * (((double)c->dangHi + (double)c->dangLo) * a.invN64)) {}
+    __device__ __forceinline__ float value(double s) const { return (float)fma(damping, s, rest); }
+};
 
 // Per-thread accumulators of one iteration.
 struct IterAcc {
@@ -475,7 +472,7 @@ __global__ void __maxnreg__(56) prAdaptiveKernel(PrArgs a, const uint4* __restri
     const GbPrControl* c = a.ctl;
     if (ldvi(&c->stopped)) return;
     const int cur = c->cur;
-    const float dang = c->dangHi + c->dangLo;
+    const PrTerm term(a, c);
     const bool withDelta = !INPLACE && c->withDelta;
     const float* contrib = INPLACE ? a.contrib[0] : a.contrib[cur];
     const float* rOld = a.r[cur];
@@ -505,7 +502,7 @@ __global__ void __maxnreg__(56) prAdaptiveKernel(PrArgs a, const uint4* __restri
         const Kahan k = gatherVecs(vecs + h.y + lane, h.y + lane < h.z ? (h.z - h.y - lane + 31) / 32 : 0u, 32, gather);
         FF f;
         if (splitSum(a, t, h.w, first, cnt, k, f) && lane == 0)
-            store(h.x, a.pos ? a.pos[h.x] : h.x, prValueSplit(a, f.hi, f.lo, c), a.outdeg[h.x], withDelta ? rOld[h.x] : 0.f);
+            store(h.x, a.pos ? a.pos[h.x] : h.x, term.value((double)f.hi + (double)f.lo), a.outdeg[h.x], withDelta ? rOld[h.x] : 0.f);
     }
     GbPrRun r{};
     uint32_t end = 0;  // first task beyond run r
@@ -530,7 +527,7 @@ __global__ void __maxnreg__(56) prAdaptiveKernel(PrArgs a, const uint4* __restri
         const uint32_t count = active && sub < r.vecs ? (r.vecs - sub + G - 1) >> r.lg : 0u;
         float s = gatherVecs(p, count, r.inter ? 32 : G, gather).sum;
         for (unsigned o = G >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-        if (lead) store(v, at, prValue(a, s, dang), od, old);
+        if (lead) store(v, at, term.value(s), od, old);
     }
     if (!INPLACE) finishBlock<0>(a, acc);
 }
@@ -546,7 +543,7 @@ __global__ void prGroupKernel(PrArgs a, uint32_t lg, uint32_t splitMin) {
     const GbPrControl* c = a.ctl;
     if (ldvi(&c->stopped)) return;
     const int cur = c->cur;
-    const float dang = c->dangHi + c->dangLo;
+    const PrTerm term(a, c);
     const bool withDelta = !INPLACE && c->withDelta;
     const float* contrib = INPLACE ? a.contrib[0] : a.contrib[cur];
     IterAcc acc;
@@ -563,7 +560,7 @@ __global__ void prGroupKernel(PrArgs a, uint32_t lg, uint32_t splitMin) {
         const Kahan k = gatherKahan<INPLACE>(a.ci, contrib, h.y, h.z, lane, 32);
         FF f;
         if (splitSum(a, (uint32_t)t, h.w, first, cnt, k, f) && lane == 0)
-            store(h.x, prValueSplit(a, f.hi, f.lo, c), a.outdeg[h.x], withDelta ? a.r[cur][h.x] : 0.f);
+            store(h.x, term.value((double)f.hi + (double)f.lo), a.outdeg[h.x], withDelta ? a.r[cur][h.x] : 0.f);
     }
     for (; t < total; t += nwarps) {
         const uint64_t v = (t - a.nChunks) * (32u >> lg) + (lane >> lg);
@@ -574,7 +571,7 @@ __global__ void prGroupKernel(PrArgs a, uint32_t lg, uint32_t splitMin) {
         const float old = lead && withDelta ? a.r[cur][v] : 0.f;
         float s = mine ? gatherGroup<INPLACE>(a.ci, contrib, b, e, sub, G) : 0.f;
         for (unsigned o = G >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-        if (lead) store((uint32_t)v, prValue(a, s, dang), od, old);
+        if (lead) store((uint32_t)v, term.value(s), od, old);
     }
     if (!INPLACE) finishBlock<0>(a, acc);
 }
@@ -585,10 +582,10 @@ __global__ void gsSetKernel(PrArgs a) {
     const GbPrControl* c = a.ctl;
     if (ldvi(&c->stopped)) return;
     const int cur = c->cur;
-    const float dang = c->dangHi + c->dangLo;
+    const PrTerm term(a, c);
     const float* contrib = a.contrib[0];
     auto store = [&](uint32_t v, float s) {
-        const float val = prValue(a, s, dang);
+        const float val = term.value(s);
         a.r[cur ^ 1][v] = val;
         const uint32_t od = a.outdeg[v];
         a.contrib[0][v] = od ? val / (float)od : 0.0f;
@@ -625,7 +622,7 @@ __global__ void gsSweepListKernel(PrArgs a, uint32_t count) {
     const GbPrControl* c = a.ctl;
     if (ldvi(&c->stopped)) return;
     const int cur = c->cur;
-    const float dang = c->dangHi + c->dangLo;
+    const PrTerm term(a, c);
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += nwarps) {
         const uint32_t v = a.list[i];
@@ -634,7 +631,7 @@ __global__ void gsSweepListKernel(PrArgs a, uint32_t count) {
         float s = gatherGroup<true>(a.ci, a.contrib[0], b, e, laneId(), 32);
         s = warpSum(s);
         if (laneId() == 0) {
-            const float val = prValue(a, s, dang);
+            const float val = term.value(s);
             a.r[cur ^ 1][v] = val;
             const uint32_t od = a.outdeg[v];
             a.contrib[0][v] = od ? val / (float)od : 0.0f;
@@ -647,9 +644,9 @@ __global__ void gsHubKernel(PrArgs a) {
     const GbPrControl* c = a.ctl;
     if (ldvi(&c->stopped)) return;
     const int cur = c->cur;
-    const float dang = c->dangHi + c->dangLo;
+    const PrTerm term(a, c);
     auto store = [&](uint32_t v, float s) {
-        const float val = prValue(a, s, dang);
+        const float val = term.value(s);
         a.r[cur ^ 1][v] = val;
         const uint32_t od = a.outdeg[v];
         a.contrib[0][v] = od ? val / (float)od : 0.0f;
@@ -755,13 +752,13 @@ __global__ void prPushFinalizeKernel(PrArgs a) {
     const GbPrControl* c = a.ctl;
     if (ldvi(&c->stopped)) return;
     const int cur = c->cur;
-    const float dang = c->dangHi + c->dangLo;
+    const PrTerm term(a, c);
     const bool withDelta = c->withDelta;
     IterAcc acc;
     for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < a.n; base += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t v = base + threadIdx.x;
         if (v < a.n) {
-            const float val = prValue(a, a.acc[v] + a.accLo[v], dang);
+            const float val = term.value((double)a.acc[v] + (double)a.accLo[v]);
             a.acc[v] = 0.0f;
             a.accLo[v] = 0.0f;
             storeJacobi(a, cur, withDelta, (uint32_t)v, val, acc);
@@ -872,7 +869,7 @@ __global__ void __launch_bounds__(kBlkThreads, 1) prBlockedKernel(PrArgs a, BlkA
     if (ldvi(&c->stopped)) return;
     const int cur = c->cur;
     const bool withDelta = c->withDelta;
-    const float dang = c->dangHi + c->dangLo;
+    const PrTerm term(a, c);
     const float* contrib = a.contrib[cur];
     const unsigned tid = threadIdx.x, warp = tid >> 5;
     if (tid == 0) {
@@ -977,7 +974,7 @@ __global__ void __launch_bounds__(kBlkThreads, 1) prBlockedKernel(PrArgs a, BlkA
             for (uint32_t i = ct; i < rows; i += kCons) {
                 const uint32_t v = r0 + i;
                 if (a.rp[v + 1] - a.rp[v] >= kBlkHub) continue;
-                storeJacobi(a, cur, withDelta, v, prValue(a, sums[i], dang), acc);
+                storeJacobi(a, cur, withDelta, v, term.value(sums[i]), acc);
             }
         }
         if (!ok && lane == 0) atomicOr(&sFailed, 1);
@@ -1016,7 +1013,7 @@ __global__ void __launch_bounds__(kBlkThreads, 1) prBlockedKernel(PrArgs a, BlkA
                 x.lo = hubLo[w];
                 t2.add(x);
             }
-            storeJacobi(a, cur, withDelta, v, prValue(a, t2.hi + t2.lo, dang), acc);
+            storeJacobi(a, cur, withDelta, v, term.value((double)t2.hi + (double)t2.lo), acc);
         }
         __syncthreads();
     }
@@ -1315,12 +1312,9 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
     c.tol = o.tol;
     c.tolRel = o.tol_rel;
     PrArgs a = makeArgs(*this, false);
-    a.damping = o.damping;
     a.invN = 1.0f / (float)n;
     a.damping64 = writtenDecimal(o.damping);
     a.base64 = (1.0 - a.damping64) / (double)n;
-    a.base = (float)a.base64;
-    a.dampingLo = (float)(a.damping64 - (double)o.damping);
     a.invN64 = 1.0 / (double)n;
     PrArgs ag = a;
     if (v == GB_PR_PULL_ADAPTIVE) {  // hub-first relabeled layout
