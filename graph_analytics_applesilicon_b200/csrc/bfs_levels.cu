@@ -8,14 +8,13 @@
 // + one atomic per warp), CAS claims on dist, shared-memory staging of the
 // scanned frontier degrees in the edge-balanced expansion, and bitmap
 // frontiers with __ballot_sync word assembly in the bottom-up step.
-#include <emmintrin.h>
-
 #include <algorithm>
 #include <atomic>
 #include <chrono>
 
 #include "bfs.hpp"
 #include "bfs_device.cuh"
+#include "host_cpu.hpp"
 
 namespace gb {
 
@@ -607,7 +606,7 @@ struct EdgeRun {
         ++h.lastLevels;
         const volatile unsigned long long* pub = h.edgePub.p;
         for (uint64_t spins = 1; pub[3] != a.seq; ++spins) {
-            _mm_pause();
+            cpuPause();
             if (spins & 1023) continue;
             const cudaError_t e = cudaStreamQuery(h.stream.s);
             if (e == cudaErrorNotReady) continue;

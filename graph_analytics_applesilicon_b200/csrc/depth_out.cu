@@ -3,12 +3,11 @@
 // A depth array is 4 bytes per vertex, but a traversal of L levels only needs
 // depths below L: when L < 15 (255, 65535) the depths travel over PCIe as 4
 // bits (1 byte, 2 bytes) per vertex, sentinel all ones for unreached, in chunks
-// whose host-side widening to uint32 (SSE2, OpenMP threads) overlaps the copy
+// whose host-side widening to uint32 (host_cpu.hpp, OpenMP threads) overlaps the copy
 // of the next chunk.  The pack kernel also checks every depth against the
 // width, so a wrong level count can only cost a plain copy, never a wrong
 // result; a caller may therefore enqueue the packing behind a traversal whose
 // level count it does not know yet (beginDepths) and widen after one wait.
-#include <emmintrin.h>
 #include <omp.h>
 
 #include <algorithm>
@@ -16,6 +15,7 @@
 
 #include "bfs.hpp"
 #include "host_copy.hpp"
+#include "host_cpu.hpp"
 
 namespace gb {
 namespace {
@@ -58,58 +58,6 @@ __global__ void packDepthsKernel(const uint32_t* d, uint64_t count, uint8_t* out
         else reinterpret_cast<uint4*>(out)[g] = make_uint4(w[0], w[1], w[2], w[3]);
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) *overflow = 1u;  // may be pinned memory
-}
-
-inline uint32_t widenOne(int fmt, const uint8_t* in, uint64_t i) {
-    if (fmt == 0) {
-        const uint32_t v = (in[i / 2] >> (4 * (i & 1))) & 15u;
-        return v == 15u ? kInf : v;
-    }
-    if (fmt == 1) return in[i] == 0xFFu ? kInf : in[i];
-    const uint32_t v = reinterpret_cast<const uint16_t*>(in)[i];
-    return v == 0xFFFFu ? kInf : v;
-}
-
-inline void store4(uint32_t* o, __m128i x) { _mm_storeu_si128(reinterpret_cast<__m128i*>(o), x); }
-
-// Sixteen bytes b (sentinel 0xFF) to sixteen uint32 (sentinel all ones): the
-// sentinel's compare mask is the high part in both unpacking steps.
-inline void widen16(__m128i b, uint32_t* o) {
-    const __m128i m = _mm_cmpeq_epi8(b, _mm_set1_epi8(-1));
-    const __m128i lo = _mm_unpacklo_epi8(b, m), hi = _mm_unpackhi_epi8(b, m);
-    const __m128i ml = _mm_unpacklo_epi8(m, m), mh = _mm_unpackhi_epi8(m, m);
-    store4(o, _mm_unpacklo_epi16(lo, ml));
-    store4(o + 4, _mm_unpackhi_epi16(lo, ml));
-    store4(o + 8, _mm_unpacklo_epi16(hi, mh));
-    store4(o + 12, _mm_unpackhi_epi16(hi, mh));
-}
-
-// Depths [lo, hi) of a packed array; lo is a multiple of 32.  Plain stores: with
-// stores that bypass the cache the 16.8 MB of R-MAT 22 take 358 us a call, so 307.
-void widenRange(int fmt, const uint8_t* in, uint64_t lo, uint64_t hi, uint32_t* out) {
-    uint64_t i = lo;
-    if (fmt == 0) {
-        const __m128i low = _mm_set1_epi8(15);
-        for (; i + 32 <= hi; i += 32) {
-            const __m128i x = _mm_loadu_si128(reinterpret_cast<const __m128i*>(in + i / 2));
-            const __m128i a = _mm_and_si128(x, low), b = _mm_and_si128(_mm_srli_epi16(x, 4), low);
-            const __m128i y0 = _mm_unpacklo_epi8(a, b), y1 = _mm_unpackhi_epi8(a, b);
-            widen16(_mm_or_si128(y0, _mm_cmpeq_epi8(y0, low)), out + i);
-            widen16(_mm_or_si128(y1, _mm_cmpeq_epi8(y1, low)), out + i + 16);
-        }
-    } else if (fmt == 1) {
-        for (; i + 16 <= hi; i += 16)
-            widen16(_mm_loadu_si128(reinterpret_cast<const __m128i*>(in + i)), out + i);
-    } else {
-        const __m128i ones = _mm_set1_epi16(-1);
-        for (; i + 8 <= hi; i += 8) {
-            const __m128i x = _mm_loadu_si128(reinterpret_cast<const __m128i*>(in + 2 * i));
-            const __m128i m = _mm_cmpeq_epi16(x, ones);
-            store4(out + i, _mm_unpacklo_epi16(x, m));
-            store4(out + i + 4, _mm_unpackhi_epi16(x, m));
-        }
-    }
-    for (; i < hi; ++i) out[i] = widenOne(fmt, in, i);
 }
 
 }  // namespace
