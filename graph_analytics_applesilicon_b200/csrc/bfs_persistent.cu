@@ -62,7 +62,8 @@ struct PArgs {
     bool fillDist;      // the kernel sets the depths to infinity (at most kSmallDepths; else a memset before the launch)
     uint8_t* packHost;  // pinned host memory for the packed depths, or null
     int packMax;        // and the widest form (packFormat) it has room for
-    unsigned* ctlHost;  // pinned: [0] levels run, [1] width of the packed depths (with packHost), [2] a wait ran out
+    unsigned* ctlHost;  // pinned: [0] levels run, [2] a wait ran out; with packHost [1] width of the packed depths,
+                        // [3] ns of the traversal (fillDist), else of the packing
     gb_level* trace;
     const float* sel;
     double* state;
@@ -182,8 +183,8 @@ struct Smem {
     unsigned long long soEdges[3];
     unsigned long long state[8];  // what block 0's levels arrived at (see soloLevels)
     // kept by thread 0, out of every thread's registers: adjacency entries and
-    // vertices not reached yet, and the time of the last level's end (block 0)
-    unsigned long long unexplored, unreached, tPrev;
+    // vertices not reached yet, and the times of the last level's end and of the start (block 0)
+    unsigned long long unexplored, unreached, tPrev, tStart;
 };
 
 // Grid barrier after which every thread of the block sees counters *c in
@@ -640,6 +641,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
     __shared__ Smem<NT> sm;
     const unsigned tid = threadIdx.x;
     const uint64_t gtid = (uint64_t)blockIdx.x * NT + tid, gthreads = (uint64_t)gridDim.x * NT;
+    if (tid == 0) sm.tStart = globaltimer();
     unsigned* bar = &a.ctl[0];
     unsigned* err = &a.ctl[1];
     const bool learned = a.selector == GB_SELECT_LEARNED && a.sel != nullptr;
@@ -977,7 +979,23 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
         bi = bi1;
         ci = ci1;
     }
-    if (a.packHost) packToHost(a, level, gtid, gthreads);
+    if (a.packHost) {
+        // The return of the depths is no part of the traversal's time.  Behind a
+        // memset the host takes the time around both and leaves out the packing,
+        // which ends when block 0's share (all are equal) has arrived: 3 us for the
+        // fence, which a call of 50 us on a small array would notice and one of 150
+        // us and more does not.
+        const uint64_t t = globaltimer();
+        packToHost(a, level, gtid, gthreads);
+        if (blockIdx.x == 0) {
+            if (!a.fillDist) {
+                __threadfence_system();
+                __syncthreads();
+            }
+            const uint64_t ns = a.fillDist ? t - sm.tStart : globaltimer() - t;
+            if (tid == 0) a.ctlHost[3] = ns <= 0xFFFFFFFFu ? (unsigned)ns : 0u;  // over 4 s the packing is nothing
+        }
+    }
     if (gtid == 0) {
         if (a.ctlHost) a.ctlHost[0] = level;
         if (a.trace && level > 0 && level - 1 < a.traceCap && lastStrat == GB_STRAT_BU)
@@ -1067,6 +1085,13 @@ void launchFor(gb_bfs& h, PArgs& a, int grid = 0, cudaStream_t st = nullptr) {
     if (!st) st = h.stream.s;
     if (h.pBlock == 256) launchPersistent<256>(a, grid, st);
     else launchPersistent<512>(a, grid, st);
+}
+
+// Device time of a traversal, `ms` by the events around it, without the packing
+// in its kernel: ns (see PArgs::ctlHost), 0 when it packed nothing.
+float traversalMs(const gb_bfs& h, float ms, unsigned ns) {
+    if (!ns) return ms;
+    return h.n <= kSmallDepths ? (float)ns * 1e-6f : std::max(ms - (float)ns * 1e-6f, 1e-6f);
 }
 
 // The state of in-flight slot `slot` (> 0) in place of slot 0's.
@@ -1164,7 +1189,7 @@ void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb
     pctlHost.ensure(4);
     volatile unsigned* done = pctlHost.p;  // the kernel's last act: levels run, width of the packed depths
     done[0] = kNotDone;
-    done[2] = 0;
+    done[2] = done[3] = 0;
     a.ctlHost = pctlHost.p;
     const bool packInKernel = out && n <= kPackInKernel;
     if (packInKernel) {
@@ -1188,7 +1213,7 @@ void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb
     } else {
         GB_CUDA(cudaStreamSynchronize(stream.s));
     }
-    lastGpuMs = ev.ms();
+    lastGpuMs = traversalMs(*this, ev.ms(), done[3]);
     if (done[0] == kNotDone || done[2]) {
         GB_CUDA(cudaMemsetAsync(pctl.get(), 0, 4 * sizeof(unsigned), stream.s));
         GB_CUDA(cudaStreamSynchronize(stream.s));
@@ -1289,7 +1314,7 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
     if (direct)
         for (uint32_t i = 0; i < count; ++i) {
             mCtlHost.p[4 * (size_t)i] = kNotDone;
-            mCtlHost.p[4 * (size_t)i + 2] = 0;
+            mCtlHost.p[4 * (size_t)i + 2] = mCtlHost.p[4 * (size_t)i + 3] = 0;
         }
     GB_CUDA(cudaMemsetAsync(mCtl.get(), 0, (size_t)count * 4 * sizeof(unsigned), stream.s));
     // the other streams start after the work queued before this call on the handle's stream
@@ -1390,11 +1415,14 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
         if (mCtlHost.p[4 * (size_t)i + 1]) throw timeout();
     for (uint32_t i = 0; i < count; ++i) {
         if (levelsOut) levelsOut[i] = mCtlHost.p[4 * (size_t)i + 2];
-        if (timed) GB_CUDA(cudaEventElapsedTime(&msOut[i], mEv[2 * i], mEv[2 * i + 1]));
+        if (timed) {
+            GB_CUDA(cudaEventElapsedTime(&msOut[i], mEv[2 * i], mEv[2 * i + 1]));
+            if (direct) msOut[i] = traversalMs(*this, msOut[i], mCtlHost.p[4 * (size_t)i + 3]);
+        }
     }
     float last = 0;
     GB_CUDA(cudaEventElapsedTime(&last, mEv[2 * (count - 1)], mEv[2 * (count - 1) + 1]));
-    lastGpuMs = last;
+    lastGpuMs = direct ? traversalMs(*this, last, mCtlHost.p[4 * (size_t)(count - 1) + 3]) : last;
     lastLevels = mCtlHost.p[4 * (size_t)(count - 1) + 2];
     const uint32_t lastBuf = (count - 1) % B;
     if (lastBuf) dist.swap(mDist[lastBuf - 1]);  // dist holds the last source's depths

@@ -267,7 +267,12 @@ int gb_bfs_run_many(gb_bfs* h, int variant, const uint32_t* sources, uint32_t co
 int gb_bfs_run_batch(gb_bfs* h, const uint32_t* sources, int k, uint32_t* out_host,
                      const gb_bfs_options* opt, gb_level* trace, size_t cap, size_t* nlev);
 /* lastGpuMs / lastLevels (src/metal/bfs_gpu.hpp:70-72): device time of the
- * last run (CUDA events on the handle's stream) and its level count. */
+ * last run and its level count.  The time is that of the traversal, whether its
+ * depths are returned or not: CUDA events on the handle's stream, or the device's
+ * own timer where other work lies between two events (gpu_edge and gpu_do: the
+ * sum over the levels, each from its first kernel's start to its last one's end;
+ * persistent runs whose kernel also returns the depths; each source of a learned
+ * gb_bfs_run_many on a road network, see gb_bfs_options.selector). */
 double gb_bfs_last_gpu_ms(const gb_bfs* h);
 uint32_t gb_bfs_last_levels(const gb_bfs* h);
 /* Device pointer of the last single-source result (n uint32), for callers that
