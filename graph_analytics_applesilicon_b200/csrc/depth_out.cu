@@ -165,7 +165,7 @@ void endDepths(gb_bfs* h, const DepthReturn& r, uint32_t levels, uint32_t* out) 
         }
         if (*h->packFlagHost.p == 0) return;
         GB_CUDA(cudaStreamSynchronize(h->stream.s));
-        GB_CUDA(cudaMemsetAsync(h->packFlag.get(), 0, 4, h->stream.s));
+        if (r.count > kSmallDepths) GB_CUDA(cudaMemsetAsync(h->packFlag.get(), 0, 4, h->stream.s));
         // the guessed width was too narrow: once more with the level count, which fits
         if (packFormat(levels) > r.fmt) {
             DepthReturn again;
