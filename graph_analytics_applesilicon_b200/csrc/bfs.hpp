@@ -114,7 +114,6 @@ struct gb_bfs {
     gb::DevBuf<unsigned> pctl;           // [0] barrier, [1] error, [2] levels, [3] flags
     gb::HostPinned<unsigned> pctlHost;
     gb::DevBuf<gb_level> ptrace;
-    gb::DevBuf<double> pstate;           // level state for resumable (profiling) runs
     int pGrid = 0, pBlock = 0, pMax = 0, pWant = 0;
     // further traversals in flight in runPersistentMany: the same per-traversal
     // state (slot 0 is the members above) and a stream each
@@ -124,7 +123,6 @@ struct gb_bfs {
         gb::DevBuf<GbPCounters> ctr;
         gb::DevBuf<unsigned long long> solo;
         gb::DevBuf<gb_level> trace;
-        gb::DevBuf<double> state;
     };
     PSlot pSlot[gb::kMaxInFlight - 1];
     std::unique_ptr<gb::Stream> pStream[gb::kMaxInFlight - 1];  // created on first use

@@ -41,8 +41,6 @@ constexpr unsigned kNotDone = 0xFFFFFFFFu;
 // level on the grid.
 constexpr uint32_t kSoloLevels = 64;
 
-enum { S_LEVEL, S_BOTTOMUP, S_SCOUT, S_TOCHECK, S_UNEXPLORED, S_REACHED, S_QVALID, S_LAST, S_COUNT };
-
 struct PArgs {
     const uint32_t* __restrict__ row_ptr;
     const uint32_t* __restrict__ col_idx;
@@ -66,14 +64,12 @@ struct PArgs {
                         // [3] ns of the traversal (fillDist), else of the packing
     gb_level* trace;
     const float* sel;
-    double* state;
     uint64_t n, m;
     uint32_t words, source, hubMin, traceCap;
     double alpha, beta;
     float selMargin;  // learned selector: log2 margin for leaving the rule's direction
     int selector, force;
     unsigned long long spinLimit;
-    uint32_t startLevel, maxLevels;
 };
 
 __device__ __forceinline__ unsigned long long ldv(const unsigned long long* p) {
@@ -465,7 +461,7 @@ __device__ __forceinline__ bool barrierWithState(const PArgs& a, Smem<NT>& sm, c
 // toCheck before this level's rule, vertices found, their degrees).  The level
 // counters are not touched: other blocks may still be reading the last level's.
 template <int NT>
-__device__ void soloLevels(const PArgs& a, Smem<NT>& sm, uint32_t level, uint32_t endLevel, uint32_t S, uint64_t scout,
+__device__ void soloLevels(const PArgs& a, Smem<NT>& sm, uint32_t level, uint32_t S, uint64_t scout,
                            uint64_t toCheck, uint32_t* front, uint32_t* next, unsigned long long* out) {
     const unsigned tid = threadIdx.x, lane = laneId();
     for (uint32_t i = tid; i < S; i += NT) front[a.qv[level & 1][i] >> 5] = 0;  // its bits are this frontier's only
@@ -543,7 +539,7 @@ __device__ void soloLevels(const PArgs& a, Smem<NT>& sm, uint32_t level, uint32_
             if (a.trace && level - 1 < a.traceCap) a.trace[level - 1].time_ms = (double)(t - sm.tPrev) * 1e-6;
             sm.tPrev = t;
         }
-        if (S == 0 || edges > kSoloEdges * NT || most >= a.hubMin || k + 1 == kSoloLevels || level >= endLevel) break;
+        if (S == 0 || edges > kSoloEdges * NT || most >= a.hubMin || k + 1 == kSoloLevels) break;
         if ((double)edges > (double)toCheck / a.alpha) break;  // bottom-up next: the grid's
         toCheck -= min(toCheck, edges);
     }
@@ -650,83 +646,61 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
     // barrier makes them visible to every warp)
     if (learned) selectorStageAsync(sm.sel, a.sel, tid, NT);
 
-    uint32_t level;
-    bool bottomUp, qValid;
-    uint64_t scout, toCheck;
-    int lastStrat;
-    if (a.startLevel == 0) {
-        // One pass writes the initial state with the source already placed
-        // (depth 0, visited, frontier bit), so a single grid barrier ends the
-        // prologue.  bm[2] needs no clearing: level 0 clears it.  The depth
-        // array is set to infinity here too, or, a large one, by a memset before
-        // the launch (faster from about 2^20 vertices on).
-        const uint32_t src = a.source;
-        const uint32_t st = a.row_ptr[src], d = a.row_ptr[src + 1] - st;
-        if (a.fillDist) {
-            uint4* d4 = reinterpret_cast<uint4*>(a.dist);  // its buffer is a multiple of 16 bytes
-            for (uint64_t i = gtid; i < (a.n + 3) / 4; i += gthreads) {
-                const uint64_t v = 4 * i;
-                d4[i] = make_uint4(v == src ? 0u : kInf, v + 1 == src ? 0u : kInf, v + 2 == src ? 0u : kInf,
-                                   v + 3 == src ? 0u : kInf);
-            }
-        } else if (gtid == 0) {
-            a.dist[src] = 0;
+    // One pass writes the initial state with the source already placed
+    // (depth 0, visited, frontier bit), so a single grid barrier ends the
+    // prologue.  bm[2] needs no clearing: level 0 clears it.  The depth
+    // array is set to infinity here too, or, a large one, by a memset before
+    // the launch (faster from about 2^20 vertices on).
+    const uint32_t src = a.source;
+    const uint32_t st = a.row_ptr[src], d = a.row_ptr[src + 1] - st;
+    if (a.fillDist) {
+        uint4* d4 = reinterpret_cast<uint4*>(a.dist);  // its buffer is a multiple of 16 bytes
+        for (uint64_t i = gtid; i < (a.n + 3) / 4; i += gthreads) {
+            const uint64_t v = 4 * i;
+            d4[i] = make_uint4(v == src ? 0u : kInf, v + 1 == src ? 0u : kInf, v + 2 == src ? 0u : kInf,
+                               v + 3 == src ? 0u : kInf);
         }
-        for (uint64_t w = gtid; w < a.words; w += gthreads) {
-            uint32_t pad = 0;
-            if (w == a.words - 1 && (a.n & 31)) pad = ~((1u << (a.n & 31)) - 1u);  // bits past n read as visited
-            const uint32_t srcBit = w == (src >> 5) ? 1u << (src & 31) : 0u;
-            // vertices of degree 0 start as visited: no edge reaches them (their
-            // depth stays infinity from the memset), and a bottom-up round then
-            // skips a bitmap word as soon as its other vertices are reached
-            a.visited[w] = pad | srcBit | (a.iso ? a.iso[w] : 0u);
-            a.bm[0][w] = srcBit;
-            a.bm[1][w] = 0;
-        }
-        if (gtid == 0) {
-            for (int s = 0; s < 3; ++s) a.ctr[s] = GbPCounters{};
-            GbPCounters& c = a.ctr[2];
-            c.found = 1;
-            c.nextEdges = d;
-            if (d >= a.hubMin) {
-                a.hv[0][0] = src;
-                a.hs[0][0] = st;
-                a.ho[0][0] = 0;
-                c.hubPack = (1ull << kHubShift) | d;
-            } else {
-                a.qv[0][0] = src;
-                a.qs[0][0] = st;
-                a.qd[0][0] = d;
-                c.qtail = 1;
-            }
-        }
-        if (learned) selectorStageWait();
-        if (!gridBarrier(bar, err, a.spinLimit)) return timedOut(a);
-        level = 0;
-        bottomUp = false;
-        qValid = true;
-        scout = d;
-        toCheck = a.m;
-        if (tid == 0) {
-            sm.unexplored = a.m - d;
-            sm.unreached = a.n - 1;
-        }
-        lastStrat = -1;
-    } else {
-        level = (uint32_t)a.state[S_LEVEL];
-        bottomUp = a.state[S_BOTTOMUP] != 0;
-        scout = (uint64_t)a.state[S_SCOUT];
-        toCheck = (uint64_t)a.state[S_TOCHECK];
-        if (tid == 0) {
-            sm.unexplored = (uint64_t)a.state[S_UNEXPLORED];
-            sm.unreached = a.n - (uint64_t)a.state[S_REACHED];
-        }
-        qValid = a.state[S_QVALID] != 0;
-        lastStrat = (int)a.state[S_LAST];
-        if (learned) selectorStageWait();
-        if (!gridBarrier(bar, err, a.spinLimit)) return timedOut(a);
+    } else if (gtid == 0) {
+        a.dist[src] = 0;
     }
-    const uint32_t endLevel = a.maxLevels ? a.startLevel + a.maxLevels : 0xFFFFFFFFu;
+    for (uint64_t w = gtid; w < a.words; w += gthreads) {
+        uint32_t pad = 0;
+        if (w == a.words - 1 && (a.n & 31)) pad = ~((1u << (a.n & 31)) - 1u);  // bits past n read as visited
+        const uint32_t srcBit = w == (src >> 5) ? 1u << (src & 31) : 0u;
+        // vertices of degree 0 start as visited: no edge reaches them (their
+        // depth stays infinity from the memset), and a bottom-up round then
+        // skips a bitmap word as soon as its other vertices are reached
+        a.visited[w] = pad | srcBit | (a.iso ? a.iso[w] : 0u);
+        a.bm[0][w] = srcBit;
+        a.bm[1][w] = 0;
+    }
+    if (gtid == 0) {
+        for (int s = 0; s < 3; ++s) a.ctr[s] = GbPCounters{};
+        GbPCounters& c = a.ctr[2];
+        c.found = 1;
+        c.nextEdges = d;
+        if (d >= a.hubMin) {
+            a.hv[0][0] = src;
+            a.hs[0][0] = st;
+            a.ho[0][0] = 0;
+            c.hubPack = (1ull << kHubShift) | d;
+        } else {
+            a.qv[0][0] = src;
+            a.qs[0][0] = st;
+            a.qd[0][0] = d;
+            c.qtail = 1;
+        }
+    }
+    if (learned) selectorStageWait();
+    if (!gridBarrier(bar, err, a.spinLimit)) return timedOut(a);
+    uint32_t level = 0;
+    bool bottomUp = false, qValid = true;
+    uint64_t scout = d, toCheck = a.m;
+    int lastStrat = -1;
+    if (tid == 0) {
+        sm.unexplored = a.m - d;
+        sm.unreached = a.n - 1;
+    }
     if (tid == 0) sm.tPrev = globaltimer();
     __syncwarp();  // warp 0 reads what thread 0 keeps
     int selLast = -1;  // last evaluated learned decision and the frontier it was made for
@@ -737,7 +711,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
     uint64_t nextSize, nextEdgesC, nextQ;
     unsigned long long nextHub;
     {
-        const GbPCounters* p0 = &a.ctr[(level + 2) % 3];
+        const GbPCounters* p0 = &a.ctr[2];
         nextSize = ldv(&p0->found);
         nextEdgesC = ldv(&p0->nextEdges);
         nextQ = ldv(&p0->qtail);
@@ -746,13 +720,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
 
     // the bitmap of the current frontier and the counters of the current level:
     // both move on by one per level that the grid runs
-    uint32_t bi = level % 3, ci = level % 3, stretch = 0;
+    uint32_t bi = 0, ci = 0, stretch = 0;
     for (;;) {
         const uint32_t ci1 = ci == 2 ? 0 : ci + 1;
         GbPCounters* prev = &a.ctr[ci1 == 2 ? 0 : ci1 + 1];
         GbPCounters* cur = &a.ctr[ci];
         const uint64_t size = nextSize, fedges = nextEdgesC;
-        if (size == 0 || level >= endLevel) break;
+        if (size == 0) break;
         const uint32_t bi1 = bi == 2 ? 0 : bi + 1, bi2 = bi1 == 2 ? 0 : bi1 + 1;
 
         // alpha/beta rule (src/cpu/bfs_cpu.cpp:247-279): always evaluated, it
@@ -774,7 +748,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
             // two places in turn: block 0 may end its next stretch before another block has read this one's
             unsigned long long* from = a.solo + 8 * (stretch++ & 1u);
             if (blockIdx.x == 0)
-                soloLevels<NT>(a, sm, level, endLevel, (uint32_t)nextQ, scout, toCheck, a.bm[bi], a.bm[bi1], from);
+                soloLevels<NT>(a, sm, level, (uint32_t)nextQ, scout, toCheck, a.bm[bi], a.bm[bi1], from);
             if (!barrierWithState<NT>(a, sm, from)) return timedOut(a);
             level = (uint32_t)sm.state[0];
             bottomUp = false;
@@ -1001,14 +975,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
         if (a.trace && level > 0 && level - 1 < a.traceCap && lastStrat == GB_STRAT_BU)
             a.trace[level - 1].edges = ldv(&a.ctr[ci == 0 ? 2 : ci - 1].examined);
         a.ctl[2] = level;
-        a.state[S_LEVEL] = level;
-        a.state[S_BOTTOMUP] = bottomUp;
-        a.state[S_SCOUT] = (double)scout;
-        a.state[S_TOCHECK] = (double)toCheck;
-        a.state[S_UNEXPLORED] = (double)sm.unexplored;
-        a.state[S_REACHED] = (double)(a.n - sm.unreached);
-        a.state[S_QVALID] = qValid;
-        a.state[S_LAST] = lastStrat;
     }
 }
 
@@ -1063,7 +1029,6 @@ PArgs makeArgs(gb_bfs& h, const gb_bfs_options& o, uint32_t src) {
     a.trace = h.ptrace.get();
     a.traceCap = kTraceCap;
     a.sel = h.selLoaded[0] ? h.selParams[0].get() : nullptr;
-    a.state = h.pstate.get();
     a.n = h.n;
     a.m = h.m;
     a.words = (uint32_t)((h.n + 31) / 32);
@@ -1075,8 +1040,6 @@ PArgs makeArgs(gb_bfs& h, const gb_bfs_options& o, uint32_t src) {
     a.selector = (int)o.selector;
     a.force = o.force_strategy;
     a.spinLimit = o.spin_limit ? o.spin_limit : (1ull << 24);
-    a.startLevel = 0;
-    a.maxLevels = 0;
     return a;
 }
 
@@ -1110,7 +1073,6 @@ void useSlot(gb_bfs& h, PArgs& a, int slot) {
     a.ctr = p.ctr.get();
     a.solo = p.solo.get();
     a.trace = p.trace.get();
-    a.state = p.state.get();
 }
 
 }  // namespace
@@ -1144,7 +1106,6 @@ void gb_bfs::ensurePersistent(const gb_bfs_options& o) {
         GB_CUDA(cudaMemsetAsync(pctl.get(), 0, 4 * sizeof(unsigned), stream.s));
     }
     ptrace.ensure(kTraceCap);
-    pstate.ensure(S_COUNT);
     for (uint32_t k = 1; k < std::max<uint32_t>(1, o.in_flight); ++k) {
         PSlot& p = pSlot[k - 1];
         for (int i = 0; i < 2; ++i) {
@@ -1157,7 +1118,6 @@ void gb_bfs::ensurePersistent(const gb_bfs_options& o) {
         p.ctr.ensure(3);
         p.solo.ensure(16);
         p.trace.ensure(kTraceCap);
-        p.state.ensure(S_COUNT);
     }
     if (pBlock != block) {
         int perSm = 0;
