@@ -19,7 +19,9 @@ the library's GPU training kernels (gb_mlp_train, Adam) and written to
 selector_single.npy beside this file, where GpuBfs users and bench.py find it.
 --seed picks the initial weights and the minibatch order (default 0); the
 shipped selector_single.npy was trained with --seed 1.
-evaluate: learned vs rule persistent BFS on held-out graphs (same depths).
+evaluate, evaluate-batch: learned vs rule on held-out graphs (same depths), both
+on the whole grid: road networks would else run a cluster per source, which
+consults neither.
 
 Every handle uses the hub-first adjacency layout (GpuBfs.hub_first), the one
 bench.py and gbench --hub-first run with; --natural keeps the caller's order.
@@ -38,6 +40,7 @@ import graph_analytics_applesilicon_b200 as G  # noqa: E402
 
 
 HUB_FIRST = "--natural" not in sys.argv
+WHOLE_GRID = 1 << 16  # grid_blocks: more than are resident, so all of them, and never the cluster form
 
 
 def handle(g):
@@ -166,7 +169,7 @@ def evaluate(params_path=None, sources=8):
         srcs = G.pick_sources(g, sources, 3)
         tt = {}
         for sel in ("rule", "learned"):
-            o = G.BfsOptions(selector=sel)
+            o = G.BfsOptions(selector=sel, grid_blocks=WHOLE_GRID)
             for s in srcs:  # warm
                 bfs.run("gpu_do_persistent", int(s), opts=o)
             ms = []
@@ -188,7 +191,7 @@ def evaluate_batch(params_path=None, batches=2):
         bfs.set_selector(p, 1)
         tt = {}
         for sel in ("rule", "learned"):
-            o = G.BfsOptions(selector=sel)
+            o = G.BfsOptions(selector=sel, grid_blocks=WHOLE_GRID)
             ms = []
             for b in range(batches):
                 srcs = G.pick_sources(g, 64, 21 + b)

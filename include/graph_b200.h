@@ -193,12 +193,25 @@ typedef struct {
     uint32_t large_min;  /* gpu_binned: degree >= large_min -> block per vertex */
     uint32_t ept;        /* gpu_edge / gpu_do top-down: edges per thread */
     double alpha, beta;  /* direction rule (cpu::bfsDO, src/cpu/bfs_cpu.cpp:227-283) */
-    uint32_t selector;   /* gb_selector, persistent variant only */
+    uint32_t selector;   /* gb_selector, persistent and batched variants.  On a graph of at most 31
+                            neighbours a vertex and 8 on average (road networks), untraced
+                            persistent runs under GB_SELECT_LEARNED and untraced batches under
+                            either selector run as a thread-block cluster per source: the same
+                            depths, by one strategy, up to 64 sources at once.  That form uses
+                            neither the selector's parameters nor alpha, beta, hub_min, block,
+                            sel_margin and in_flight, keeps 16 bytes per vertex (its neighbour
+                            table) and, in gb_bfs_run_many, a row of depths per source, and its
+                            waits end after two seconds.  grid_blocks, force_strategy or a
+                            spin_limit below 16384 keeps a call on the whole grid, where levels
+                            of up to 4 * block edges run in one block, top-down, whatever the
+                            selector. */
     int32_t force_strategy; /* >= 0: persistent kernel runs every level with it (profiling) */
     uint32_t hub_min;    /* persistent: degree at which a vertex is split across blocks */
     uint32_t block;      /* persistent / batched: threads per block (256 or 512) */
-    uint64_t spin_limit; /* grid-barrier wait bound in polls (0 = default, ~ seconds) */
-    uint32_t grid_blocks; /* persistent / batched: blocks in the grid (0 = every resident block) */
+    uint64_t spin_limit; /* grid-barrier wait bound in polls (0 = default, ~ seconds); below 16384
+                            every level runs on the whole grid, whose barriers are short */
+    uint32_t grid_blocks; /* persistent / batched: blocks in the grid, at most those resident
+                            (0 = every resident block, or a cluster per source, see selector) */
     float sel_margin;    /* learned selector: it departs from the alpha/beta rule's direction only
                             when it predicts the other direction faster by this much (log2 of
                             the time ratio); its top-down strategy choice is free.  0 = pure
