@@ -384,7 +384,10 @@ bool gb_bfs::runCluster(const uint32_t* src, uint32_t k, uint32_t* out) {
         if (cStatHost.p[i].status) cOff = true;
         levels = std::max(levels, cStatHost.p[i].levels);
     }
-    if (cOff) return false;
+    if (cOff) {  // for the handle's life
+        cNbr.release();
+        return false;
+    }
     lastGpuMs = ev.ms();
     lastLevels = levels;
     return true;
@@ -398,7 +401,10 @@ bool gb_bfs::runClusterMany(const uint32_t* src, uint32_t count, uint32_t* out, 
     bDist.ensure((uint64_t)std::min<uint32_t>(count, 64) * n + 4);
     for (uint32_t g0 = 0; g0 < count; g0 += 64) {
         const uint32_t k = std::min<uint32_t>(64, count - g0);
-        if (!runCluster(src + g0, k, bDist.get())) return false;
+        if (!runCluster(src + g0, k, bDist.get())) {
+            bDist.release();  // the grid form rotates in_flight + 2 rows; a batch takes its own again
+            return false;
+        }
         for (uint32_t j = 0; j < k; ++j) {
             if (msOut) msOut[g0 + j] = (float)((double)cStatHost.p[j].ns * 1e-6);
             if (levelsOut) levelsOut[g0 + j] = cStatHost.p[j].levels;
