@@ -135,6 +135,7 @@ struct gb_bfs {
     gb::DevBuf<uint32_t> bSrc;           // the sources
     gb::DevBuf<unsigned long long> bCtr; // level counters
     gb::DevBuf<uint2> bDefer;            // bottom-up: lists whose rest a whole block scans
+    bool bInPlanes = false;              // the last batch had its depths in bPlane
     int bGrid = 0, bBlock = 0, bMax = 0;
 
     // bounded-degree graphs: a cluster per source (bfs_cluster.cu)

@@ -825,10 +825,11 @@ void gb_bfs::ensureBatch(const gb_bfs_options& o, int k) {
     }
     bCand.ensure(n);
     bDefer.ensure(n);
-    if (k >= kPlaneSources) bPlane.ensure(kPlanes * n);
     bDist.ensure((uint64_t)k * n + 4);
     pctl.ensure(4);
     ptrace.ensure(kTraceCap);
+    bCtr.ensure(4 * sizeof(BCounters) / sizeof(unsigned long long));
+    bSrc.ensure(64);
     if (bBlock != block) {
         int perSm = 0;
         if (block == 256)
@@ -840,6 +841,8 @@ void gb_bfs::ensureBatch(const gb_bfs_options& o, int k) {
         bBlock = block;
     }
     bGrid = o.grid_blocks > 0 ? std::min<int>((int)o.grid_blocks, bMax) : bMax;
+    // last: without room for the planes every depth is stored directly
+    bInPlanes = k >= kPlaneSources && bPlane.tryEnsure(kPlanes * n);
 }
 
 // gb_bfs_run_many for the batched kernel: one launch per group of up to 64
@@ -929,8 +932,6 @@ void gb_bfs::runBatch(const uint32_t* src, int k, const gb_bfs_options& o, std::
     }
     ensureBatch(o, k);
     static_assert(sizeof(BCounters) % sizeof(unsigned long long) == 0, "whole words");
-    bCtr.ensure(4 * sizeof(BCounters) / sizeof(unsigned long long));
-    bSrc.ensure(64);
     hstage.ensure(64);
     std::memcpy(hstage.p, src, k * 4);
     GB_CUDA(cudaMemcpyAsync(bSrc.get(), hstage.p, k * 4, cudaMemcpyHostToDevice, stream.s));
@@ -952,7 +953,7 @@ void gb_bfs::runBatch(const uint32_t* src, int k, const gb_bfs_options& o, std::
     a.cq = bCand.get();
     a.dq = bDefer.get();
     a.plane = bPlane.get();
-    a.planeDepth = k >= kPlaneSources ? 1u << kPlanes : 1u;
+    a.planeDepth = bInPlanes ? 1u << kPlanes : 1u;
     a.dist = bDist.get();
     a.sources = bSrc.get();
     a.ctr = reinterpret_cast<BCounters*>(bCtr.get());

@@ -348,10 +348,10 @@ uint32_t gb_bfs::clusterBlocks(uint32_t k) {
 
 // Runs k sources' traversals into out (source i's depths at out + i * n) and
 // their level counts and times into cStatHost; false when a frontier outgrew
-// the queues (out is then not valid).
+// the queues or there is no memory for the neighbour table (out is then not valid).
 bool gb_bfs::runCluster(const uint32_t* src, uint32_t k, uint32_t* out) {
     if (!cNbrReady) {
-        cNbr.ensure(n);
+        if (!cNbr.tryEnsure(n)) return false;
         nbrTableKernel<<<(uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)deviceSmCount() * 8), 256, 0,
                          stream.s>>>(rowPtr.get(), colIdx.get(), n, cNbr.get());
         GB_LAUNCH_CHECK();
@@ -395,10 +395,10 @@ bool gb_bfs::runCluster(const uint32_t* src, uint32_t k, uint32_t* out) {
 
 // gb_bfs_run_many with the learned selector: up to 64 sources to a launch,
 // each with its own device time and level count; false (nothing valid) when a
-// frontier outgrew the queues.
+// frontier outgrew the queues or there is no memory for this form.
 bool gb_bfs::runClusterMany(const uint32_t* src, uint32_t count, uint32_t* out, uint64_t stride, float* msOut,
                             uint32_t* levelsOut) {
-    bDist.ensure((uint64_t)std::min<uint32_t>(count, 64) * n + 4);
+    if (!bDist.tryEnsure((uint64_t)std::min<uint32_t>(count, 64) * n + 4)) return false;
     for (uint32_t g0 = 0; g0 < count; g0 += 64) {
         const uint32_t k = std::min<uint32_t>(64, count - g0);
         if (!runCluster(src + g0, k, bDist.get())) {

@@ -58,6 +58,17 @@ struct DevBuf {
         GB_CUDA(cudaMalloc(&p, bytes));
         n = bytes / sizeof(T);
     }
+    // The same for a buffer there is a way without; false: no memory for it.
+    bool tryEnsure(size_t count) {
+        try {
+            ensure(count);
+        } catch (const Error& e) {
+            if (e.status != GB_ERR_OOM) throw;
+            cudaGetLastError();
+            return false;
+        }
+        return true;
+    }
     T* get() const { return p; }
     void swap(DevBuf& o) {
         std::swap(p, o.p);
