@@ -23,6 +23,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <mutex>
 
 #include "pagerank.hpp"
 
@@ -1104,6 +1105,8 @@ uint32_t gridFor(uint64_t work, uint32_t threads) {
 template <class K>
 uint32_t residentGrid(K kernel, uint64_t work, uint32_t threads) {
     static std::map<std::pair<const void*, uint32_t>, int> cache;
+    static std::mutex mu;  // handles may run in several threads
+    std::lock_guard<std::mutex> lock(mu);
     auto key = std::make_pair((const void*)kernel, threads);
     auto it = cache.find(key);
     int perSm;
@@ -1121,17 +1124,9 @@ uint32_t residentGrid(K kernel, uint64_t work, uint32_t threads) {
 
 }  // namespace
 
-// Dynamic shared memory of prBlockedKernel (the staging ring, row sums);
-// the opt-in limit is raised once per process.
-static size_t blkSmemBytes() {
-    static const size_t bytes = [] {
-        const size_t b = ((size_t)kBlkCStages * kBlkPart + kBlkRowCap) * sizeof(float) +
-                         (size_t)kBlkEStages * kBlkChunk * sizeof(uint4);
-        GB_CUDA(cudaFuncSetAttribute(prBlockedKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b));
-        return b;
-    }();
-    return bytes;
-}
+// Dynamic shared memory of prBlockedKernel: the staging ring, row sums.
+constexpr size_t kBlkSmem = ((size_t)kBlkCStages * kBlkPart + kBlkRowCap) * sizeof(float) +
+                            (size_t)kBlkEStages * kBlkChunk * sizeof(uint4);
 
 // Whether an adaptive iteration keeps the most-gathered contributions in shared
 // memory: blocks of 1,024 threads, one per SM, so it needs tasks for all of them.
@@ -1141,13 +1136,10 @@ static bool hotFits(const gb_pr& h) {
     return h.hotA && (uint64_t)h.nChunks + h.nRunTasks >= (uint64_t)deviceSmCount() * (kHotThreads / 32);
 }
 
-static void raiseHotLimit() {
-    static const bool raised = [] {
-        GB_CUDA(cudaFuncSetAttribute(prAdaptiveKernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(kPrHotMax * sizeof(float))));
-        return true;
-    }();
-    (void)raised;
+// Allows a kernel its dynamic shared memory, on the current device; before any capture.
+template <class K>
+static void allowShared(K kernel, size_t bytes) {
+    GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
 // The decimal value a float option was written as (0.85f -> 0.85), as the
@@ -1191,7 +1183,7 @@ static void enqueueIteration(gb_pr& h, int v, const gb_pr_options& o, PrArgs& a,
                   h.rowsPer, h.nParts, h.nBlkHubs, 1ull << 22};
         const uint32_t grid = (uint32_t)std::min<uint64_t>({(uint64_t)deviceSmCount(), (uint64_t)kMaxGrid,
                                                             (uint64_t)std::max(h.nRowBlocks, h.nBlkHubs)});
-        prBlockedKernel<<<std::max(grid, 1u), kBlkThreads, blkSmemBytes(), s>>>(a, b);
+        prBlockedKernel<<<std::max(grid, 1u), kBlkThreads, kBlkSmem, s>>>(a, b);
     } else if (!inplace) {
         if (v == GB_PR_PULL_SCALAR || v == GB_PR_PULL_VECTOR)
             prGroupKernel<false><<<residentGrid(prGroupKernel<false>, groupWork, tg), tg, 0, s>>>(grouped(a), sp.lg, sp.splitMin);
@@ -1276,13 +1268,13 @@ gb_pr_result gb_pr::run(int v, const gb_pr_options& o) {
     if (o.iters < 0) throw Error(GB_ERR_ARG, "iters must be >= 0");
     if (v == GB_PR_PULL_ADAPTIVE) {
         prepareAdaptive(o.small_max, o.large_min);
-        raiseHotLimit();  // before any capture
+        allowShared(prAdaptiveKernel<false, true>, kPrHotMax * sizeof(float));
     }
     if (v == GB_PR_PULL_SCALAR || v == GB_PR_PULL_VECTOR) prepareSplit(v == GB_PR_PULL_VECTOR);
     if (v == GB_PR_PULL_GS && !gsReady) prepareGS(2);
     if (v == GB_PR_PULL_BLOCKED) {
         prepareBlocked();
-        (void)blkSmemBytes();  // raise the shared-memory limit before any capture
+        allowShared(prBlockedKernel, kBlkSmem);
     }
     gb_pr_result res{};
     res.last_delta = -1;
