@@ -169,10 +169,19 @@ struct gb_bfs {
     gb::HostPinned<unsigned> mCtlHost, mFlagHost;
     std::vector<cudaEvent_t> mEv, mSlotEv;
     gb::Stream copyStream;
+    // Everything in flight ends first: pinned buffers go back to a pool that others
+    // take from, and giving them back waits for nothing.
     ~gb_bfs() {
+        drain();
         for (cudaEvent_t e : packEv) cudaEventDestroy(e);
         for (cudaEvent_t e : mEv) cudaEventDestroy(e);
         for (cudaEvent_t e : mSlotEv) cudaEventDestroy(e);
+    }
+    void drain() {
+        cudaStreamSynchronize(stream.s);
+        for (auto& s : pStream)
+            if (s) cudaStreamSynchronize(s->s);
+        cudaStreamSynchronize(copyStream.s);
     }
 
     double lastGpuMs = 0;
@@ -211,6 +220,7 @@ struct gb_bfs {
     void endLevel();  // copy stats, sync, accumulate GPU time
     void initDist(uint32_t src);
     void ensureEdgeBuffers();
+    void ensureControl();
     void ensurePersistent(const gb_bfs_options& o);
     void ensureBatch(const gb_bfs_options& o, int k);
 };

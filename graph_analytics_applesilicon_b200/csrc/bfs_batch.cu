@@ -826,7 +826,7 @@ void gb_bfs::ensureBatch(const gb_bfs_options& o, int k) {
     bCand.ensure(n);
     bDefer.ensure(n);
     bDist.ensure((uint64_t)k * n + 4);
-    pctl.ensure(4);
+    ensureControl();
     ptrace.ensure(kTraceCap);
     bCtr.ensure(4 * sizeof(BCounters) / sizeof(unsigned long long));
     bSrc.ensure(64);

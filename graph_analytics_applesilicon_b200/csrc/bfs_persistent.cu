@@ -14,11 +14,12 @@
 //   frontier queue q[2] = (vertex, adjacency start, degree) u32[n] each;
 //   hub list hub[2] = (vertex, start, exclusive offset in the hubs' edge space)
 //   for vertices of degree >= hub_min, whose edges are split across blocks;
-//   counters ctr[3] (level L writes ctr[L%3], zeroes ctr[(L+1)%3]).
+//   counters ctr[3] in turn (a level of the grid writes ctr[c], zeroes ctr[c+1]).
 // Top-down claims a vertex with atomicOr on its visited bit (an L2-resident
 // word instead of a 32-bit CAS on dist); bottom-up writes only bitmaps.
 #include <algorithm>
 #include <cstring>
+#include <exception>
 
 #include "bfs.hpp"
 #include "bfs_device.cuh"
@@ -1080,6 +1081,14 @@ void useSlot(gb_bfs& h, PArgs& a, int slot) {
 
 using namespace gb;
 
+// The control words of single and batched runs, zero when they are made: the
+// barrier word works from any value, the error word is cleared after an error.
+void gb_bfs::ensureControl() {
+    if (pctl.get()) return;
+    pctl.ensure(4);
+    GB_CUDA(cudaMemsetAsync(pctl.get(), 0, 4 * sizeof(unsigned), stream.s));
+}
+
 void gb_bfs::ensurePersistent(const gb_bfs_options& o) {
     const int block = o.block ? (int)o.block : 512;
     pWant = (int)o.grid_blocks;
@@ -1101,10 +1110,7 @@ void gb_bfs::ensurePersistent(const gb_bfs_options& o) {
     }
     pctr.ensure(3);
     psolo.ensure(16);
-    if (!pctl.get()) {  // the barrier word works from any value, the error word is cleared after an error
-        pctl.ensure(4);
-        GB_CUDA(cudaMemsetAsync(pctl.get(), 0, 4 * sizeof(unsigned), stream.s));
-    }
+    ensureControl();
     ptrace.ensure(kTraceCap);
     for (uint32_t k = 1; k < std::max<uint32_t>(1, o.in_flight); ++k) {
         PSlot& p = pSlot[k - 1];
@@ -1332,10 +1338,17 @@ void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* ou
         }
     };
     auto timeout = [&]() {
-        for (uint32_t k = 0; k < K; ++k) cudaStreamSynchronize(streams[k]);
-        cudaStreamSynchronize(cs);
         return Error(GB_ERR_TIMEOUT, "persistent BFS: grid barrier wait exceeded its spin limit");
     };
+    // a call that ends early leaves nothing in flight: the next one uses the same
+    // slots, control words and pinned buffers
+    struct Early {
+        gb_bfs& h;
+        const int before = std::uncaught_exceptions();
+        ~Early() {
+            if (std::uncaught_exceptions() > before) h.drain();
+        }
+    } early{*this};
 
     uint32_t queued = 0;
     if (!out) {
