@@ -72,7 +72,8 @@ void widenPacked(int fmt, const uint8_t* in, uint64_t count, uint32_t* out);
 void widenRows(int fmt, const uint8_t* in, uint64_t pitch, uint32_t rows, uint64_t count, uint32_t* out, uint64_t stride);
 // Depth arrays up to this size are packed straight into pinned host memory;
 // larger ones into device memory, and copied in chunks that the widening overlaps
-// (single persistent calls: bfs_persistent.cu).
+// (single persistent calls: kPackInKernel; measurements of both lines are in
+// bfs_persistent.cu).
 constexpr uint64_t kSmallDepths = 1ull << 20;
 constexpr int kEdgeStatWords = 8;
 // A spin limit under this many polls may be set for the grid's levels of a few us,

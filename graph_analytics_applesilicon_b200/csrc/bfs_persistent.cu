@@ -35,7 +35,12 @@ constexpr uint64_t kEnqueueEdges = 1ull << 18;  // top-down levels with this man
 // (soloLevels).  A level of 4 takes 5 us there against 6.5 on the grid, one of 8
 // 10 us (road 300 x 300, rule: 2.7 ms with 2 edges per thread, 1.8 with 4).
 constexpr uint32_t kSoloEdges = 4;
-constexpr uint64_t kPackInKernel = 1ull << 23;  // depth arrays up to this size are packed by a single call's kernel
+// Depth arrays up to this size are packed by a single call's kernel (packToHost).
+// Beyond, what the widening overlaps with the chunks' copies is worth as much: us a
+// call so / with a pack kernel and chunks, R-MAT: 2^18 vertices 105 / 110, 2^19 117
+// / 126, 2^20 127 / 134, 2^21 185 / 196, 2^22 365 / 374, 2^23 509-541 / 513-568, 2^24
+// 1,287-1,311 / 1,258-1,308.
+constexpr uint64_t kPackInKernel = 1ull << 23;
 constexpr unsigned kNotDone = 0xFFFFFFFFu;
 // At most so many levels at a time, which bounds the other blocks' wait (about
 // 0.3 ms, some 400 polls); a caller's spin limit under kSoloSpin polls keeps every
@@ -600,9 +605,7 @@ __device__ void soloLevels(const PArgs& a, Smem<NT>& sm, uint32_t level, uint32_
 
 // The depths packed straight into pinned host memory (at most kPackInKernel
 // vertices): the level count is known here, so the width is exact, and no
-// kernel or copy of its own follows the traversal.  Us a call against a pack
-// kernel and chunked copies, which the widening overlaps: R-MAT of 1.5M vertices
-// 192 / 217, of 2M 167 / 189, of 4.2M 270 / 291.
+// kernel or copy of its own follows the traversal.
 __device__ void packToHost(const PArgs& a, uint32_t level, uint64_t gtid, uint64_t gthreads) {
     const int fmt = level < 15 ? 0 : level < 255 ? 1 : level < 65535 ? 2 : -1;  // packFormat
     if (gtid == 0) a.ctlHost[1] = (unsigned)fmt;
@@ -742,8 +745,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persistentBfsKernel(PArgs a) {
         // then takes over what block 0 arrived at.
         if (strat != GB_STRAT_BU && a.force < 0 && qValid && fedges <= kSoloEdges * NT && (nextHub >> kHubShift) == 0 &&
             a.spinLimit >= kSoloSpin) {
-            if (gtid == 0 && a.trace && level > 0 && level - 1 < a.traceCap && lastStrat == GB_STRAT_BU)
-                a.trace[level - 1].edges = ldv(&prev->examined);
             uint32_t* third = a.bm[bi2];
             for (uint64_t w = gtid; w < a.words; w += gthreads) third[w] = 0;
             // two places in turn: block 0 may end its next stretch before another block has read this one's
@@ -1218,8 +1219,11 @@ void gb_bfs::runPersistent(uint32_t src, const gb_bfs_options& o, std::vector<gb
 // still be copied whole from its depth buffer.  Up to kSmallDepths vertices the
 // traversal packs its depths into pinned memory itself and leaves its level count
 // there (as in runPersistent): a launch and an event per source instead of a
-// dozen calls, which bound short traversals (R-MAT 18, 24 sources, 8 in flight:
-// 710 us a call, 626 so).
+// dozen calls, which bound short traversals.  From 2^21 on the kernels wait for PCIe
+// longer than those calls take.  Us for 16 sources so / with the other form, R-MAT, 1,
+// 4 and 8 in flight: 2^18 1,430 / 1,440, 487 / 529, 396 / 491; 2^19 1,611 / 1,640, 674
+// / 693, 540 / 608; 2^20 1,667 / 1,598, 841 / 872, 815 / 945; 2^21 2,407 / 2,192, 2,003 /
+// 2,068, 2,285 / 2,185; 2^22 4,754 / 4,269, 4,485 / 4,260, 5,164 / 5,075.
 void gb_bfs::runPersistentMany(const uint32_t* src, uint32_t count, uint32_t* out, uint64_t stride,
                                const gb_bfs_options& o, float* msOut, uint32_t* levelsOut) {
     validateOptions(o);

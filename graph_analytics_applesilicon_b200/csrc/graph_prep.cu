@@ -409,10 +409,14 @@ void keysToCsr(DevBuf<unsigned long long>& keys, DevBuf<unsigned long long>& tmp
         throw Error(GB_ERR_OOM, "graph prep: host allocation failed");
     }
     try {
-        // A ring of its own has to be page-locked, 2.5 ms, which a small result's
-        // slower plain copies do not cost (ms a build with plain copies / with the
-        // ring, by bytes of the result: 1.3 MB 3.2 / 6.6, 12 MB 6.6 / 9.5, 16 MB
-        // 7.4 / 10.8, 22 MB 27 / 17, 130 MB 72 / 28).
+        // A ring of its own has to be page-locked, 2.5 ms.  A plain copy costs less
+        // into memory that is mapped already, up to some 30 MB, and more into pages
+        // that it touches first.  Ms a build with plain copies / with the ring, by
+        // bytes of the result, with the results kept: 4.1 MB 6.3 / 7.9, 8.2 MB 8.1 /
+        // 8.8, 12.2 MB 10.4 / 9.1, 16.3 MB 12.1 / 9.7, 24.5 MB 16.8 / 11.2, 47.6 MB
+        // 30.5 / 18.2, 71.3 MB 45.6 / 24.2; each freed before the next: 12.2 MB 5.0 /
+        // 8.4, 16.3 MB 5.3 / 8.5, 24.5 MB 6.8 / 9.9, 47.6 MB 30.7 / 18.0, 71.3 MB 43.7 /
+        // 23.4.  The line lies where neither loses much to the other.
         if ((n + m2) * 4 < kStagedMin) {
             GB_CUDA(cudaMemcpyAsync(hrp, rp.get(), (n + 1) * 4, cudaMemcpyDeviceToHost, st));
             GB_CUDA(cudaMemcpyAsync(hci, col, (uint64_t)m2 * 4, cudaMemcpyDeviceToHost, st));

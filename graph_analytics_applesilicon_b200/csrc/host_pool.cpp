@@ -2,12 +2,12 @@
 //
 // Handles need small pinned buffers (control words, packed depths, copy rings).
 // Page-locking one costs about a millisecond whatever its size, and 14 ms for 4
-// MiB on the B200 box, more than most calls take.  Blocks are powers of two: up
-// to kSmall they are cut from slabs, larger ones are page-locked one by one and
-// kept for the next request up to kKeep bytes.  When the last block comes back
-// (the last handle is gone) everything is given back to the system.  Blocks are
-// page-locked for every context (portable) and belong to one owner at a time;
-// the owner returns a block only after the copies into it are done.
+// MiB, more than most calls take.  Blocks are powers of two, so up to twice what
+// was asked for: up to kSmall they are cut from slabs, larger ones are page-locked
+// one by one and kept for the next request up to kKeep bytes.  When the last block
+// comes back (the last handle is gone) everything is given back to the system.
+// Blocks are page-locked for every context (portable) and belong to one owner at a
+// time; the owner returns a block only after the copies into it are done.
 #include <map>
 #include <mutex>
 #include <vector>
