@@ -360,7 +360,9 @@ typedef struct {
     int32_t iters;     /* fixed mode: iterations; tol mode: cap */
     double tol;        /* > 0: stop when the L1 change < tol */
     double tol_rel;    /* > 0 (tol mode): also require max relative change < tol_rel */
-    uint32_t tg;       /* threads per block of the main kernels */
+    uint32_t tg;       /* threads per block of the main kernels (the adaptive pull of a graph whose
+                          most-gathered contributions are kept in shared memory, from 12 Mi
+                          in-edges on, takes 1024 whatever this is) */
     uint32_t small_max, large_min; /* adaptive bins (in-degree) */
     uint32_t inplace;  /* any pull variant: update contrib in place (GS-style) */
 } gb_pr_options;
