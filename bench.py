@@ -1099,8 +1099,10 @@ def headline_workload(args, world, rank, local):
         "clocks": clocks.summary(),
         "validated": valid,
         "validated_sources": (len(srcs_all) if valid else 0) if valid is not None else None,
-        "validation": ("every source's depths (from the timed e2e call) equal the reference's cpu_do "
-                       "(oracle/_ref) bit for bit" + ("; other ranks' by 128-bit digest" if world > 1 else "")),
+        "validation": ("every source's depths (from the timed e2e call) equal "
+                       + ("the reference's cpu_do (oracle/_ref)" if cpu and cpu["kind"] == "reference"
+                          else "the oracle's cpu_do (oracle/oracle.c)")
+                       + " bit for bit" + ("; other ranks' by 128-bit digest" if world > 1 else "")),
         "compare": {"plain_gpu_do_gteps": edges_per_rank_step / (plain_ms * 1e-3) / 1e9,
                     "persistent_rule_gteps": edges_per_rank_step / (rule_ms * 1e-3) / 1e9,
                     "persistent_rule_tuned": ({"block": rule_opts.block, "grid_blocks": rule_opts.grid_blocks,

@@ -16,9 +16,9 @@
 //   - a level ends with every block sending its count to the others by
 //     st.async onto their mbarriers: no fence and no cluster barrier, whose
 //     release waits for all the block's global writes (1,500-2,500 cycles).
-// Measured, road 1400 x 1400 (1,854 levels, 1,060 vertices each on average):
-// one source 12.6 -> 3.7 ms (2.0 us per level), 64 sources of one call 107
-// (batched kernel) -> 7.7 ms.
+// Measured, road 1400 x 1400 (1,854 levels, 1,060 vertices each on average),
+// device time: one source 12.6 -> 3.7 ms (2.0 us per level), 64 sources of one
+// call 107 (batched kernel) -> 7.7 ms.
 #include <cooperative_groups.h>
 
 #include <algorithm>
