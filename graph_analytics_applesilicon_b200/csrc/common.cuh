@@ -23,6 +23,7 @@ struct Error : std::runtime_error {
 
 inline void cudaCheck(cudaError_t e, const char* what, const char* file, int line) {
     if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here: the next launch's check must not find it again
         int st = (e == cudaErrorMemoryAllocation) ? GB_ERR_OOM : GB_ERR_CUDA;
         throw Error(st, std::string(what) + " failed at " + file + ":" + std::to_string(line) + ": " +
                             cudaGetErrorString(e));
@@ -64,7 +65,6 @@ struct DevBuf {
             ensure(count);
         } catch (const Error& e) {
             if (e.status != GB_ERR_OOM) throw;
-            cudaGetLastError();
             return false;
         }
         return true;
