@@ -156,10 +156,13 @@ uint32_t groupLog2(uint32_t d, uint32_t vecs, uint32_t smallMax, uint32_t largeM
 }
 
 // Chooses the contributions to keep in shared memory (h.hotA of them, 0 when they
-// are too few of the gathers to matter) and every contribution's place.
+// are too few of the gathers to matter or there is no memory for them) and every
+// contribution's place.  The contributions' buffers, which every variant uses, are
+// replaced only by larger ones that are there.
 void choosePlaces(gb_pr& h, cudaStream_t st) {
     const uint64_t n = h.n;
     h.hotA = 0;
+    for (auto& c : h.contrib) GB_CUDA(cudaMemsetAsync(c.get() + n, 0, 16, st));  // the padding's place without any
     if (h.mIn < kPrHotEntries || n + kPrHotMax + 4 >= (1ull << 32)) return;
     DevBuf<uint32_t> bins;
     std::vector<uint32_t> count(kPrHotBins);
@@ -180,11 +183,14 @@ void choosePlaces(gb_pr& h, cudaStream_t st) {
     }
     if (gathers < h.mIn / 8) return;
     const uint32_t hot = (uint32_t)((taken + 3) / 4 * 4);
-    for (auto& c : h.contrib) {
-        c.ensure(n + hot + 4);
-        GB_CUDA(cudaMemsetAsync(c.get() + n + hot, 0, 16, st));
+    DevBuf<float> larger[2];
+    for (int i = 0; i < 2; ++i)
+        if (h.contrib[i].n < n + hot + 4 && !larger[i].tryEnsure(n + hot + 4)) return;
+    if (!h.posA.tryEnsure(n)) return;
+    for (int i = 0; i < 2; ++i) {
+        if (larger[i].get()) h.contrib[i].swap(larger[i]);
+        GB_CUDA(cudaMemsetAsync(h.contrib[i].get() + n + hot, 0, 16, st));
     }
-    h.posA.ensure(n);
     GB_CUDA(cudaMemsetAsync(bins.get(), 0, 4, st));
     hotPlacesKernel<<<prepGrid(n, 256), 256, 0, st>>>(h.outdegA.get(), n, cut + 1, 0xFFFFFFFFu, hot, true, bins.get(), h.posA.get());
     GB_LAUNCH_CHECK();

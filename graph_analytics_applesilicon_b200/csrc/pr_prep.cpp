@@ -52,6 +52,7 @@ void upload(gb::DevBuf<T>& buf, const std::vector<T>& v) {
 void gb_pr::prepareGS(uint32_t pairMaxOutdeg) {
     if (gsReady && gsPairK == pairMaxOutdeg) return;
     if (!hasIn) throw Error(GB_ERR_ARG, "gpu_pull_gs needs the in-CSR");
+    gsReady = false;  // until the new layout is complete
     gsPairK = pairMaxOutdeg;
     constexpr int kRounds = 8;
     constexpr double kMinCoverage = 0.95;
