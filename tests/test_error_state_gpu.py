@@ -19,7 +19,9 @@ def test_out_of_memory_is_reported_once(gb, oracle):
         torch.cuda.empty_cache()
         held = []
         while (more := torch.cuda.mem_get_info()[0] - 64 * MB) >= 2 * MB:
-            held.append(torch.empty(min(more // (2 * MB) * 2 * MB, 16 << 30), dtype=torch.uint8, device="cuda"))
+            piece = min(more // (2 * MB) * 2 * MB, 16 << 30)
+            piece -= 1 << 30 if 0 < more - piece < 64 * MB and piece == 16 << 30 else 0  # torch rounds small pieces up
+            held.append(torch.empty(piece, dtype=torch.uint8, device="cuda"))
         with pytest.raises(gb.GraphError, match="memory"):
             gb.GpuBfs(large)
         del held

@@ -30,7 +30,9 @@ def test_a_layout_that_ran_out_of_memory(gb):
         torch.cuda.empty_cache()
         held = []
         while (more := torch.cuda.mem_get_info()[0] - leave * MB) >= 2 * MB:
-            held.append(torch.empty(min(more // (2 * MB) * 2 * MB, 16 << 30), dtype=torch.uint8, device="cuda"))
+            piece = min(more // (2 * MB) * 2 * MB, 16 << 30)
+            piece -= 1 << 30 if 0 < more - piece < 64 * MB and piece == 16 << 30 else 0  # torch rounds small pieces up
+            held.append(torch.empty(piece, dtype=torch.uint8, device="cuda"))
         try:
             pr.prepareAdaptive()
         except gb.GraphError as e:
